@@ -203,6 +203,7 @@ void Fhert_get_ntt_tables(size_t idx, int64_t* rou, uint64_t* rou_prec, int64_t*
 // ---------------------------------------------------------------------------
 
 void Alloc_poly_data(POLY poly, uint32_t degree, size_t num_q, size_t num_p) {
+  LaunchScope scope;
   Context* c              = ctx();
   poly->_ring_degree      = degree;
   poly->_num_primes       = num_q;
@@ -255,6 +256,7 @@ void Init_poly_by_size(POLY res, size_t num_q, bool is_ext) {
 }
 
 void Copy_poly(POLY res, POLY poly) {
+  LaunchScope scope;
   if (res == poly) return;
   Context* c = ctx();
   FHERT_ASSERT(res->_num_primes == poly->_num_primes && res->_num_primes_p >= poly->_num_primes_p,
@@ -274,6 +276,7 @@ int64_t* Coeffs(POLY poly, uint32_t limb, uint32_t degree) {
 }
 
 void Set_coeffs(POLY poly, uint32_t limb, uint32_t degree, int64_t* src) {
+  LaunchScope scope;
   int64_t* dst = poly->_data + (size_t)limb * degree;
   if (dst == src) return;
   Context* c = ctx_noflush();
@@ -316,6 +319,7 @@ size_t   Fhert_profile_end(char* buf, size_t cap) { return prof_end(buf, cap); }
 
 static int64_t* hw_binary(EwOp op, int64_t* res, int64_t* a, int64_t* b, int64_t s, MODULUS* m,
                           uint32_t degree) {
+  LaunchScope scope;
   Context* c = ctx_noflush();
   FHERT_ASSERT(degree == c->N, "degree mismatch");
   int prime = prime_index_of(c, m);
@@ -347,6 +351,7 @@ int64_t* Hw_modsub_scalar(int64_t* res, int64_t* a, int64_t s, MODULUS* m, uint3
   return hw_binary(EW_ADD_SCALAR, res, a, a, -s, m, degree);
 }
 int64_t* Hw_modmuladd_scalar(int64_t* res, int64_t* a, int64_t s, MODULUS* m, uint32_t degree) {
+  LaunchScope scope;
   // hal.c:109-121; no compiled program emits it, so it is launched at once
   Context* c = ctx();
   FHERT_ASSERT(degree == c->N, "degree mismatch");
@@ -354,6 +359,7 @@ int64_t* Hw_modmuladd_scalar(int64_t* res, int64_t* a, int64_t s, MODULUS* m, ui
   return res;
 }
 int64_t* Hw_rotate(int64_t* res, int64_t* val, int64_t* order, MODULUS* m, uint32_t degree) {
+  LaunchScope scope;
   Context* c = ctx_noflush();
   FHERT_ASSERT(degree == c->N, "degree mismatch");
   FHERT_ASSERT(res != val, "Hw_rotate cannot work in place");
@@ -363,11 +369,13 @@ int64_t* Hw_rotate(int64_t* res, int64_t* val, int64_t* order, MODULUS* m, uint3
   return res;
 }
 void Hw_ntt(int64_t* res, int64_t* val, size_t mod_idx, uint32_t degree) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(degree == c->N && mod_idx < c->primes.size(), "Hw_ntt: bad arguments");
   launch_ntt(ptr2(val), ptr2(res), single((int)mod_idx), false);
 }
 void Hw_intt(int64_t* res, int64_t* val, size_t mod_idx, uint32_t degree) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(degree == c->N && mod_idx < c->primes.size(), "Hw_intt: bad arguments");
   launch_ntt(ptr2(val), ptr2(res), single((int)mod_idx), true);
@@ -378,6 +386,7 @@ void Hw_intt(int64_t* res, int64_t* val, size_t mod_idx, uint32_t degree) {
 // ---------------------------------------------------------------------------
 
 POLY Conv_poly2ntt_inplace(POLY poly) {
+  LaunchScope scope;
   FHERT_ASSERT(!poly->_is_ntt, "already ntt form");
   Context* c = ctx();
   launch_ntt(ptr2(poly->_data), ptr2(poly->_data),
@@ -387,6 +396,7 @@ POLY Conv_poly2ntt_inplace(POLY poly) {
 }
 
 POLY Conv_ntt2poly_inplace(POLY poly) {
+  LaunchScope scope;
   FHERT_ASSERT(poly->_is_ntt, "already coefficient form");
   Context* c = ctx();
   launch_ntt(ptr2(poly->_data), ptr2(poly->_data),
@@ -397,6 +407,7 @@ POLY Conv_ntt2poly_inplace(POLY poly) {
 
 // rns_poly.c:637-669: Q and special limbs
 void Conv_poly2ntt(POLY res, POLY poly) {
+  LaunchScope scope;
   FHERT_ASSERT(!poly->_is_ntt, "already ntt form");
   FHERT_ASSERT(res->_ring_degree == poly->_ring_degree && res->_num_primes == poly->_num_primes &&
                    res->_num_primes_p == poly->_num_primes_p, "size not match");
@@ -408,6 +419,7 @@ void Conv_poly2ntt(POLY res, POLY poly) {
 
 // rns_poly_impl.c:202-234: Q and special limbs
 void Conv_ntt2poly(POLY res, POLY poly) {
+  LaunchScope scope;
   FHERT_ASSERT(poly->_is_ntt, "already coefficient form");
   FHERT_ASSERT(res->_ring_degree == poly->_ring_degree && res->_num_primes == poly->_num_primes &&
                    res->_num_primes_p == poly->_num_primes_p, "size not match");
@@ -418,6 +430,7 @@ void Conv_ntt2poly(POLY res, POLY poly) {
 }
 
 static POLY binary_poly(EwOp op, POLY res, POLY a, POLY b) {
+  LaunchScope scope;
   Context* c = ctx();
   // operands in coefficient form are brought to NTT form in place, as the CPU
   // runtime does: always for a product, only on a mismatch for sums
@@ -445,6 +458,7 @@ POLY Sub_poly(POLY res, POLY a, POLY b) { return binary_poly(EW_SUB, res, a, b);
 POLY Mul_poly(POLY res, POLY a, POLY b) { return binary_poly(EW_MUL, res, a, b); }
 
 POLY Modswitch(POLY res, POLY poly) {
+  LaunchScope scope;
   size_t level = poly->_num_primes;
   FHERT_ASSERT(level >= 2, "polynomial level is too small to support modswitch");
   if (res != poly) {
@@ -517,6 +531,7 @@ void fhert_rescale_polys(Context* c, int npoly, int64_t* const res[2],
 // point runs a waiting call on its own first (ctx()).
 static void pair_run(Context* c, int kind, int npoly, int64_t* const r[2],
                      const int64_t* const x[2], size_t level, int p_limb, bool is_ntt) {
+  LaunchScope scope;
   if (kind == 1) fhert_mod_down_polys(c, npoly, r, x, p_limb, nullptr, level, is_ntt);
   else fhert_rescale_polys(c, npoly, r, x, level);
 }
@@ -559,6 +574,7 @@ static void pair_submit(int kind, int64_t* res, const int64_t* src, size_t level
 }
 
 POLY Rescale(POLY res, POLY poly) {
+  LaunchScope scope;
   size_t level = poly->_num_primes;
   FHERT_ASSERT(level >= 2, "Level of rescale opnd is too small");
   FHERT_ASSERT(res->_num_primes == level && res->_data, "Rescale: primes not match");
@@ -583,6 +599,7 @@ size_t Num_decomp(POLY poly) {
 }
 
 POLY Decomp(POLY res, POLY poly, uint32_t part) {
+  LaunchScope scope;
   Context* c     = ctx();
   size_t   level = poly->_num_primes;
   size_t   start = (size_t)c->alpha * part;
@@ -689,6 +706,7 @@ static bool modup_serve(Context* c, POLY res, POLY poly, uint32_t part) {
 }
 
 POLY Decomp_modup(POLY res, POLY poly, uint32_t part) {
+  LaunchScope scope;
   Context* c     = ctx_noflush();
   size_t   level = poly->_num_primes;
   FHERT_ASSERT(res->_data && res->_num_primes == level && res->_num_primes_p == (size_t)c->K,
@@ -732,6 +750,7 @@ POLY Decomp_modup(POLY res, POLY poly, uint32_t part) {
 }
 
 POLY Mod_up(POLY res, POLY old_poly, uint32_t part) {
+  LaunchScope scope;
   // rns_poly.c:107-158: old_poly holds only the digit's limbs (from Decomp)
   Context* c     = ctx();
   size_t   level = res->_num_primes;
@@ -840,6 +859,7 @@ POLY Mod_down(POLY res, POLY poly) {
 }
 
 POLY Mod_down_rescale(POLY res, POLY poly) {
+  LaunchScope scope;
   // rns_poly.c:531-603: ModDown and Rescale in one step, computed in coefficient
   // form; like the CPU runtime it leaves `poly` in coefficient form.
   Context*       c     = ctx();
@@ -876,6 +896,7 @@ POLY Mod_down_rescale(POLY res, POLY poly) {
 }
 
 VALUE_LIST* Reduce_and_rescale_modup(POLY res, POLY poly) {
+  LaunchScope scope;
   // rns_poly_impl.c:521-620
   Context*     c     = ctx();
   const size_t level = poly->_num_primes, n = c->N;
@@ -946,6 +967,7 @@ void Chk_level(POLY res, POLY p0, POLY p1) {
 }
 
 POLY Extend(POLY res, POLY poly) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(res->_num_primes == poly->_num_primes && poly->_data, "Extend: size not match");
   FHERT_ASSERT(res->_num_alloc_primes == poly->_num_primes + (size_t)c->K,
@@ -961,6 +983,7 @@ POLY Extend(POLY res, POLY poly) {
 }
 
 POLY Dot_prod(POLY res, POLY a, POLY b, size_t parts) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(parts >= 1 && parts <= (size_t)kMaxParts, "Dot_prod: unsupported digit count");
   size_t level = a[0]._num_primes, num_p = a[0]._num_primes_p;
@@ -990,6 +1013,7 @@ POLY Dot_prod(POLY res, POLY a, POLY b, size_t parts) {
 }
 
 POLY Automorphism_transform(POLY res, POLY poly, int64_t* order) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(poly->_is_ntt, "Automorphism_transform: coefficient form is not supported");
   FHERT_ASSERT(res->_data != poly->_data, "Automorphism_transform cannot work in place");
@@ -1093,6 +1117,7 @@ static void init_ciph3_product(CIPHER3 res, CIPHER a, CIPHER b) {
 }
 
 static CIPHER add_sub_ciph(EwOp op, CIPHER res, CIPHER a, CIPHER b) {
+  LaunchScope scope;
   Context* c = ctx();
   init_like_lower(res, a, b);
   size_t level = Level(res), num_p = res->_c0_poly._num_primes_p;
@@ -1109,6 +1134,7 @@ CIPHER Add_ciph(CIPHER res, CIPHER a, CIPHER b) { return add_sub_ciph(EW_ADD, re
 CIPHER Sub_ciph(CIPHER res, CIPHER a, CIPHER b) { return add_sub_ciph(EW_SUB, res, a, b); }
 
 CIPHER3 Mul_ciph3(CIPHER3 res, CIPHER a, CIPHER b) {
+  LaunchScope scope;
   // evaluator.c:137-173: c0 = a0*b0, c1 = a0*b1 + a1*b0, c2 = a1*b1
   init_ciph3_product(res, a, b);
   size_t level = res->_c0_poly._num_primes;
@@ -1170,6 +1196,7 @@ void fhert_switch_key(Context* c, int64_t* out0, int64_t* out1, const int64_t* i
 }
 
 CIPHER Relin(CIPHER res, CIPHER3 ciph) {
+  LaunchScope scope;
   // evaluator.c:288-305
   Context* c     = ctx();
   size_t   level = ciph->_c2_poly._num_primes;
@@ -1180,6 +1207,7 @@ CIPHER Relin(CIPHER res, CIPHER3 ciph) {
 }
 
 CIPHER Mul_ciph(CIPHER res, CIPHER a, CIPHER b) {
+  LaunchScope scope;
   CIPHERTEXT3 t;
   std::memset(&t, 0, sizeof(t));
   Mul_ciph3(&t, a, b);
@@ -1191,6 +1219,7 @@ CIPHER Mul_ciph(CIPHER res, CIPHER a, CIPHER b) {
 }
 
 CIPHER Rescale_ciph(CIPHER res, CIPHER ciph) {
+  LaunchScope scope;
   // evaluator.c:344-363
   Context* c     = ctx();
   size_t   level = Level(ciph);
@@ -1211,6 +1240,7 @@ CIPHER Rescale_ciph(CIPHER res, CIPHER ciph) {
 }
 
 static CIPHER rotate_with_key(CIPHER res, CIPHER ciph, int32_t rot_idx, uint32_t k) {
+  LaunchScope scope;
   // evaluator.c:503-522: key switch c1, add c0, then permute both polynomials
   Context* c     = ctx();
   size_t   level = Level(ciph);
@@ -1231,6 +1261,7 @@ static CIPHER rotate_with_key(CIPHER res, CIPHER ciph, int32_t rot_idx, uint32_t
 // cipher.c:460-481: several rotations of one ciphertext; its digits are raised
 // once and shared by all of them
 void Rotate_batch_ciph(CIPHER res_arr, CIPHER ciph, const int32_t* rot_idx, uint32_t count) {
+  LaunchScope scope;
   if (count == 0) return;
   Context* c     = ctx();
   size_t   level = Level(ciph), words = level * c->N, ext_limbs = level + c->K;

@@ -1263,6 +1263,7 @@ extern "C" {
 
 // ckks/src/cipher.c:565-583
 CIPHER Bootstrap(CIPHER res, CIPHER ciph, uint32_t level_after_bts) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(ciph->_c0_poly._num_primes > 0, "Input cipher level is exhausted");
   uint32_t slots = ciph->_slots;
@@ -1281,6 +1282,7 @@ void Bootstrap_precom(uint32_t num_slots) { prepare_bootstrap(ctx(), num_slots);
 
 // ckks/src/cipher.c:565-579
 CIPHER Eval_bootstrap_ciph(CIPHER res, CIPHER ciph, uint32_t level_after_bts, uint32_t num_slots) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(ciph->_c0_poly._num_primes > 0, "Input cipher level is exhausted");
   ensure_precom(c, num_slots ? num_slots : ciph->_slots);
@@ -1291,6 +1293,7 @@ CIPHER Eval_bootstrap_ciph(CIPHER res, CIPHER ciph, uint32_t level_after_bts, ui
 // ckks/src/cipher.c:585-665: raise to the full modulus, CoeffsToSlots, split
 // into real and imaginary parts (the latter is kept for the next stage)
 CIPHER Eval_bootstrap_coeffs_to_slots_ciph(CIPHER res, CIPHER ciph, uint32_t num_slots) {
+  LaunchScope scope;
   Context* c = ctx();
   clear_stage_state();
   const uint32_t n = c->N, m = 2 * n;
@@ -1329,6 +1332,7 @@ CIPHER Eval_bootstrap_coeffs_to_slots_ciph(CIPHER res, CIPHER ciph, uint32_t num
 
 // ckks/src/cipher.c:667-709: the approximate modular reduction of both parts
 CIPHER Eval_bootstrap_eval_mod_ciph(CIPHER res, CIPHER ciph, uint32_t num_slots) {
+  LaunchScope scope;
   Context*       c     = ctx();
   const uint32_t slots = num_slots ? num_slots : ciph->_slots;
   ensure_precom(c, slots);
@@ -1351,6 +1355,7 @@ CIPHER Eval_bootstrap_eval_mod_ciph(CIPHER res, CIPHER ciph, uint32_t num_slots)
 
 // ckks/src/cipher.c:711-767: SlotsToCoeffs and the way back to the message's scale
 CIPHER Eval_bootstrap_slots_to_coeffs_ciph(CIPHER res, CIPHER ciph, uint32_t num_slots) {
+  LaunchScope scope;
   Context*       c     = ctx();
   const uint32_t m     = 2 * c->N;
   const uint32_t slots = num_slots ? num_slots : ciph->_slots;

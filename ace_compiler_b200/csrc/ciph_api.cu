@@ -16,6 +16,7 @@ extern "C" {
 // poly/src/rns_poly.c:39-55: cnt polynomials over one block of storage; the
 // first element owns the block (Free_polys releases it)
 POLY_ARR Alloc_polys(uint32_t cnt, uint32_t degree, size_t num_q, size_t num_p) {
+  LaunchScope scope;
   FHERT_ASSERT(cnt > 0, "Alloc_polys: zero array size specified");
   Context* c     = ctx();
   POLY_ARR res   = (POLY_ARR)std::calloc(cnt, sizeof(POLYNOMIAL));
@@ -89,6 +90,7 @@ POLY_ARR Precomp(POLY_ARR res, size_t size, POLY input) {
 
 // ckks/src/evaluator.c:98-111
 CIPHER Add_plain(CIPHER res, CIPHER ciph, PLAIN plain) {
+  LaunchScope scope;
   Context* c = ctx();
   size_t level = ciph->_c0_poly._num_primes;
   FHERT_ASSERT(plain->_poly._num_primes >= level, "plaintext level below the ciphertext's");
@@ -104,6 +106,7 @@ CIPHER Add_plain(CIPHER res, CIPHER ciph, PLAIN plain) {
 
 // ckks/src/evaluator.c:192-216
 CIPHER Mul_plain(CIPHER res, CIPHER ciph, PLAIN plain) {
+  LaunchScope scope;
   Context* c = ctx();
   size_t level = ciph->_c0_poly._num_primes, num_p = ciph->_c0_poly._num_primes_p;
   FHERT_ASSERT(plain->_poly._num_primes >= level && plain->_poly._num_primes_p == num_p,
@@ -123,6 +126,7 @@ void Modswitch_ciph(CIPHER ciph) { mod_switch(ciph); }  // evaluator.c:401-409
 
 // evaluator.c:364-378: multiply by 2^mod_size, encoded as a constant
 CIPHER Upscale_ciph(CIPHER res, CIPHER ciph, uint32_t mod_size) {
+  LaunchScope scope;
   Context* c        = ctx();
   double   up_scale = std::pow(2.0, (double)mod_size);
   size_t   level = ciph->_c0_poly._num_primes, num_p = ciph->_c0_poly._num_primes_p;
@@ -139,6 +143,7 @@ CIPHER Upscale_ciph(CIPHER res, CIPHER ciph, uint32_t mod_size) {
 
 // evaluator.c:380-399: bring the scale to `waterline` bits by a rescale
 CIPHER Downscale_ciph(CIPHER res, CIPHER ciph, uint32_t waterline) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(ciph->_c0_poly._num_primes > 1, "Downscale: multiply level is not big enough");
   uint32_t sf_bits   = (uint32_t)c->sf_bits;
@@ -154,12 +159,14 @@ CIPHER Downscale_ciph(CIPHER res, CIPHER ciph, uint32_t waterline) {
 // ckks/src/cipher.c:417-450: back to scaling degree 1, then the q_0 residues
 // lifted to mod_size primes (0 = all)
 CIPHER Raise_mod(CIPHER res, CIPHER ciph, uint32_t mod_size) {
+  LaunchScope scope;
   Context* c = ctx();
   raise_from_level0(c, res, ciph, mod_size ? mod_size : (uint32_t)c->L);
   return res;
 }
 
 CIPHER Mul_mono_ciph(CIPHER res, CIPHER ciph, uint32_t power) {  // evaluator.c:260-286
+  LaunchScope scope;
   mul_monomial(ctx(), res, ciph, power);
   return res;
 }

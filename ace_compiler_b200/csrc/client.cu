@@ -64,16 +64,16 @@ inline dim3 grid_for(uint32_t n, int limbs) {
 void launch_encode_split(int64_t* poly, const int64_t* msg, const u64* scale_pow,
                          const LimbBatch& batch) {
   Context* c = ctx();
-  encode_split_kernel<<<grid_for(c->N, batch.count), kThreads, 0, c->stream>>>(
-      (u64*)poly, msg, scale_pow, batch, c->d_mod, c->N);
+  launch(encode_split_kernel, grid_for(c->N, batch.count), kThreads, 0, c->stream,
+         (u64*)poly, msg, scale_pow, batch, c->d_mod, c->N);
   c->launches++;
   CUDA_CHECK(cudaGetLastError());
 }
 
 void launch_small_to_rns(int64_t* poly, const int64_t* vals, const LimbBatch& batch) {
   Context* c = ctx();
-  small_to_rns_kernel<<<grid_for(c->N, batch.count), kThreads, 0, c->stream>>>(
-      (u64*)poly, vals, batch, c->d_mod, c->N);
+  launch(small_to_rns_kernel, grid_for(c->N, batch.count), kThreads, 0, c->stream,
+         (u64*)poly, vals, batch, c->d_mod, c->N);
   c->launches++;
   CUDA_CHECK(cudaGetLastError());
 }

@@ -170,6 +170,7 @@ std::vector<int64_t> encode_value(Context* c, double value, uint32_t level, doub
 void encode_vector(Context* c, PLAIN plain, std::vector<cplx>& values, uint32_t sf_degree,
                    uint32_t level, uint32_t slots, uint32_t num_p, const float* reals,
                    size_t real_count) {
+  LaunchScope scope;
   ensure_fft_tables(c);
   const uint32_t n = c->N;
   if (slots == 0) slots = n / 2;
@@ -217,6 +218,7 @@ namespace {
 
 // ckks/src/encoder.c:473-575: one value on every coefficient of every limb
 void encode_scalar(Context* c, PLAIN plain, double value, uint32_t sf_degree, uint32_t level) {
+  LaunchScope scope;
   if (level == 0) level = c->L;
   const double delta = std::pow(2.0, (double)c->sf_bits), scale = std::pow(delta, sf_degree);
   init_plain(c, plain, level, scale, sf_degree);
@@ -371,6 +373,7 @@ extern "C" {
 
 // ckks/src/encryptor.c:19-89
 CIPHER Encrypt(CIPHER res, PLAIN plain) {
+  LaunchScope scope;
   Context* c = ctx();
   FHERT_ASSERT(c->pk._p0._data != nullptr, "Encrypt: no public key (keys were not generated)");
   POLY   m     = &plain->_poly;
@@ -407,6 +410,7 @@ CIPHER Encrypt(CIPHER res, PLAIN plain) {
 
 // ckks/src/decryptor.c:19-66 (two-polynomial ciphertexts)
 void Fhert_decrypt(PLAIN res, CIPHER ciph) {
+  LaunchScope scope;
   Context* c     = ctx();
   size_t   level = ciph->_c0_poly._num_primes;
   FHERT_ASSERT(c->sk_ntt._data != nullptr, "Decrypt: no secret key");
@@ -423,6 +427,7 @@ void Fhert_decrypt(PLAIN res, CIPHER ciph) {
 // ckks/src/encoder.c:657-704: out receives `count` complex values as
 // (re, im) pairs; the plaintext is left in coefficient form
 void Fhert_decode(PLAIN plain, double* out, size_t count) {
+  LaunchScope scope;
   Context* c = ctx();
   ensure_fft_tables(c);
   POLY           poly  = &plain->_poly;

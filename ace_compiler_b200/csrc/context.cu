@@ -596,6 +596,7 @@ void destroy_context() {
   }
   dev_release_all(c->stream);
   cudaStreamSynchronize(c->stream);
+  launch_release();
   cudaFree(c->d_mod);
   cudaFree(c->d_fwd);
   cudaFree(c->d_inv);
@@ -728,6 +729,7 @@ bool take_from(DevPool& pool, size_t bytes, void** ptr) {
 }  // namespace
 
 cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t stream) {
+  if (!pool_enabled()) launch_flush();
   if (!pool_enabled()) return cudaMallocAsync(ptr, bytes, stream);
   if (bytes == 0) bytes = 256;
   bytes = (bytes + 255) & ~(size_t)255;
@@ -785,7 +787,10 @@ cudaError_t dev_free(void* ptr, cudaStream_t stream) {
     return cudaSuccess;
   }
   auto it = g_pool.size_of.find(ptr);
-  if (it == g_pool.size_of.end()) return cudaFreeAsync(ptr, stream);  // not from the lists
+  if (it == g_pool.size_of.end()) {  // not from the lists
+    launch_flush();
+    return cudaFreeAsync(ptr, stream);
+  }
   if (g_private_mode && image_capturing()) {
     // the captured kernels used this block: from now on only a replay may
     g_private.size_of[ptr] = it->second;
@@ -802,6 +807,7 @@ cudaError_t dev_free(void* ptr, cudaStream_t stream) {
 }
 
 void dev_release_all(cudaStream_t stream) {
+  launch_flush();  // what was gathered may use blocks of the lists
   for (auto& kv : g_pool.free_by_size)
     for (void* p : kv.second) {
       g_pool.size_of.erase(p);

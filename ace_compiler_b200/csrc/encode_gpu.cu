@@ -149,11 +149,11 @@ void encode_message_on_device(Context* c, const std::complex<double>* values, si
   if (reals != nullptr) {
     CUDA_CHECK(dev_alloc(&d_reals, count * sizeof(float), c->stream));
     CUDA_CHECK(counted_copy(d_reals, reals, count * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    widen_floats<<<(slots + kThreads - 1) / kThreads, kThreads, 0, c->stream>>>(
-        v, d_reals, (uint32_t)count, slots);
+    launch(widen_floats, (slots + kThreads - 1) / kThreads, kThreads, 0, c->stream,
+           v, d_reals, (uint32_t)count, slots);
     c->launches++;
   } else {
-    CUDA_CHECK(cudaMemsetAsync(v, 0, (size_t)slots * sizeof(double2), c->stream));
+    CUDA_CHECK(zero_async(v, (size_t)slots * sizeof(double2), c->stream));
     // std::complex<double> is two doubles, real part first
     CUDA_CHECK(counted_copy(v, values, count * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
   }
@@ -170,13 +170,13 @@ void encode_message_on_device(Context* c, const std::complex<double>* values, si
   }
   prof_before(KID_ENCODE);
   for (int logm = lg; logm > k; logm--)
-    embed_inv_stage<<<half_blocks, kThreads, 0, c->stream>>>(v, t->roots, t->rot_group, slots, logm,
-                                                             2 * n);
-  if (gap > 1) CUDA_CHECK(cudaMemsetAsync(d_msg, 0, (size_t)n * sizeof(int64_t), c->stream));
+    launch(embed_inv_stage, half_blocks, kThreads, 0, c->stream,
+           v, t->roots, t->rot_group, slots, logm, 2 * n);
+  if (gap > 1) CUDA_CHECK(zero_async(d_msg, (size_t)n * sizeof(int64_t), c->stream));
   const uint32_t threads = std::min(1024u, std::max(32u, 1u << (k > 0 ? k - 1 : 0)));
-  embed_inv_local<<<slots >> k, threads, smem, c->stream>>>(
-      d_msg, v, t->roots, t->rot_group, slots, lg, k, 2 * n, gap,
-      std::pow(2.0, (double)c->sf_bits));
+  launch(embed_inv_local, slots >> k, threads, smem, c->stream,
+         d_msg, v, t->roots, t->rot_group, slots, lg, k, 2 * n, gap, std::pow(2.0,
+         (double)c->sf_bits));
   prof_after(KID_ENCODE, 1);
   c->launches += (lg - k) + 1;
   CUDA_CHECK(cudaGetLastError());

@@ -240,7 +240,7 @@ struct Packer {
     }
     dag.commit();
     prof_before(KID_HW_BATCH);
-    hw_batch_kernel<<<grid, kThreads, 0, c->stream>>>(l, c->d_mod, c->N);
+    launch(hw_batch_kernel, grid, kThreads, 0, c->stream, l, c->d_mod, c->N);
     prof_after(KID_HW_BATCH, used);
     c->launches++;
     c->hw_batched_limbs += used;
@@ -283,6 +283,7 @@ struct Packer {
 }  // namespace
 
 void hw_replay(Context* c) {
+  LaunchScope scope;
   HwQueue* q = c->hw_queue;
   if (q == nullptr || q->replaying) return;
   if (q->nodes.empty() && q->renamed.empty() && q->borrowed.empty()) return;

@@ -17,7 +17,7 @@ void Alloc_lpoly_data(LPOLY poly, uint32_t ring_degree) {  // lpoly/poly.h:63-69
   poly->_ring_degree = ring_degree;
   poly->_is_ntt      = false;
   CUDA_CHECK(dev_alloc(&poly->_data, (size_t)ring_degree * sizeof(int64_t), c->stream));
-  CUDA_CHECK(cudaMemsetAsync(poly->_data, 0, (size_t)ring_degree * sizeof(int64_t), c->stream));
+  CUDA_CHECK(zero_async(poly->_data, (size_t)ring_degree * sizeof(int64_t), c->stream));
 }
 
 void Init_lpoly_data(LPOLY poly, uint32_t ring_degree, int64_t* data) {  // lpoly/poly.h:72-77
@@ -49,7 +49,7 @@ void Free_lpoly(LPOLY poly) {  // lpoly/poly.h:97-101
 
 void Zero_lpoly(LPOLY poly) {  // lpoly/poly.h:104-107
   Context* c = ctx();
-  CUDA_CHECK(cudaMemsetAsync(poly->_data, 0, (size_t)poly->_ring_degree * sizeof(int64_t), c->stream));
+  CUDA_CHECK(zero_async(poly->_data, (size_t)poly->_ring_degree * sizeof(int64_t), c->stream));
 }
 
 void Copy_lpoly(LPOLY res, L_POLY poly) {  // lpoly/poly.h:110-114

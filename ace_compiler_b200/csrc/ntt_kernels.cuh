@@ -576,8 +576,8 @@ inline void launch_strided_t(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTab
     attr_done = true;
   }
   dim3 grid(kContigBlock / TC, b.count);
-  ntt_strided_kernel<INV, S1, TC><<<grid, TC << (S1 - 3), smem, stream>>>(
-      in, out, b, INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, pro);
+  launch(ntt_strided_kernel<INV, S1, TC>, grid, TC << (S1 - 3), smem, stream,
+         in, out, b, INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, pro);
 }
 
 template <bool INV, int TC>
@@ -599,14 +599,14 @@ inline void launch_contig(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables
   dim3 grid(t.n / (kContigBlock * kWarpsPerCta), b.count);
   const Twiddle* tab = INV ? t.inv : t.fwd;
   if (INV || epi.kind == 0)
-    ntt_contig_kernel<INV, 0><<<grid, kWarpsPerCta * 32, 0, stream>>>(in, out, b, tab, t.mods, t.n,
-                                                                       t.logn, epi);
+    launch(ntt_contig_kernel<INV, 0>, grid, kWarpsPerCta * 32, 0, stream,
+           in, out, b, tab, t.mods, t.n, t.logn, epi);
   else if (epi.kind == 1)
-    ntt_contig_kernel<false, 1><<<grid, kWarpsPerCta * 32, 0, stream>>>(in, out, b, tab, t.mods,
-                                                                         t.n, t.logn, epi);
+    launch(ntt_contig_kernel<false, 1>, grid, kWarpsPerCta * 32, 0, stream,
+           in, out, b, tab, t.mods, t.n, t.logn, epi);
   else
-    ntt_contig_kernel<false, 2><<<grid, kWarpsPerCta * 32, 0, stream>>>(in, out, b, tab, t.mods,
-                                                                         t.n, t.logn, epi);
+    launch(ntt_contig_kernel<false, 2>, grid, kWarpsPerCta * 32, 0, stream,
+           in, out, b, tab, t.mods, t.n, t.logn, epi);
 }
 
 template <bool INV>
@@ -614,8 +614,8 @@ inline void launch_small(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables&
                          cudaStream_t stream) {
   size_t smem    = (size_t)t.n * sizeof(u64);
   int    threads = t.n / 2 < 512 ? (t.n / 2 < 32 ? 32 : t.n / 2) : 512;
-  ntt_small_kernel<INV><<<b.count, threads, smem, stream>>>(in, out, b, INV ? t.inv : t.fwd,
-                                                             t.mods, t.inv_last, t.n, t.logn);
+  launch(ntt_small_kernel<INV>, b.count, threads, smem, stream,
+         in, out, b, INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, t.logn);
 }
 
 }  // namespace nttk

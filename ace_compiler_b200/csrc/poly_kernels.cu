@@ -445,8 +445,7 @@ void launch_elementwise(EwOp op, Ptr2 res, Ptr2 a, Ptr2 b, int64_t scalar,
   dim3 g = grid_for(c->N, 2, batch.count);
 #define EW_CASE(OP)                                                                        \
   case OP:                                                                                 \
-    ew_kernel<OP><<<g, kThreads, 0, c->stream>>>(res, a, b, (u64)scalar, batch, c->d_mod,  \
-                                                 c->N);                                    \
+    launch(ew_kernel<OP>, g, kThreads, 0, c->stream, res, a, b, (u64)scalar, batch, c->d_mod, c->N);                                    \
     break;
   switch (op) {
     EW_CASE(EW_ADD)
@@ -471,8 +470,10 @@ void launch_scalars(bool mul, Ptr2 res, Ptr2 a, const u64* per_limb, const LimbB
   dag.commit();
   prof_before(KID_ELEMENTWISE);
   dim3 g = grid_for(c->N, 2, batch.count);
-  if (mul) ew_scalars_kernel<true><<<g, kThreads, 0, c->stream>>>(res, a, sc, batch, c->d_mod, c->N);
-  else ew_scalars_kernel<false><<<g, kThreads, 0, c->stream>>>(res, a, sc, batch, c->d_mod, c->N);
+  if (mul) launch(ew_scalars_kernel<true>, g, kThreads, 0, c->stream,
+                  res, a, sc, batch, c->d_mod, c->N);
+  else launch(ew_scalars_kernel<false>, g, kThreads, 0, c->stream,
+              res, a, sc, batch, c->d_mod, c->N);
   after_launch(c, KID_ELEMENTWISE, batch.count);
 }
 
@@ -483,8 +484,8 @@ void launch_automorphism(Ptr2 res, Ptr2 val, const uint32_t* table, const LimbBa
   dag.batch(batch, c->N, &res, &val, nullptr);
   dag.commit();
   prof_before(KID_AUTOMORPHISM);
-  automorphism_kernel<<<grid_for(c->N, 2, batch.count), kThreads, 0, c->stream>>>(
-      res, val, table, batch, c->N);
+  launch(automorphism_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
+         res, val, table, batch, c->N);
   after_launch(c, KID_AUTOMORPHISM, batch.count);
 }
 
@@ -500,8 +501,8 @@ void launch_automorphism_add(Ptr2 res, Ptr2 val, const int64_t* add, const uint3
         dag.set.read(add + (size_t)batch.limb[i].b * c->N, (size_t)c->N * sizeof(int64_t));
   dag.commit();
   prof_before(KID_AUTOMORPHISM);
-  automorphism_add_kernel<<<grid_for(c->N, 2, batch.count), kThreads, 0, c->stream>>>(
-      res, val, reinterpret_cast<const u64*>(add), table, batch, c->d_mod, c->N);
+  launch(automorphism_add_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
+         res, val, reinterpret_cast<const u64*>(add), table, batch, c->d_mod, c->N);
   after_launch(c, KID_AUTOMORPHISM, batch.count);
 }
 
@@ -512,8 +513,8 @@ void launch_mul_const(Ptr2 res, Ptr2 val, const Twiddle* consts, const LimbBatch
   dag.batch(batch, c->N, &res, &val, nullptr);
   dag.commit();
   prof_before(KID_MUL_CONST);
-  mul_const_kernel<<<grid_for(c->N, 2, batch.count), kThreads, 0, c->stream>>>(
-      res, val, consts, batch, c->d_mod, c->N);
+  launch(mul_const_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
+         res, val, consts, batch, c->d_mod, c->N);
   after_launch(c, KID_MUL_CONST, batch.count);
 }
 
@@ -530,9 +531,9 @@ void launch_tensor_range(int64_t* d0, int64_t* d1, int64_t* d2, const int64_t* a
   }
   dag.commit();
   prof_before(KID_TENSOR);
-  tensor_kernel<<<grid_for(c->N, 2, count), kThreads, 0, c->stream>>>(
-      (u64*)d0, (u64*)d1, (u64*)d2, (const u64*)a0, (const u64*)a1, (const u64*)b0,
-      (const u64*)b1, c->d_mod, c->N, first_prime);
+  launch(tensor_kernel, grid_for(c->N, 2, count), kThreads, 0, c->stream,
+         (u64*)d0, (u64*)d1, (u64*)d2, (const u64*)a0, (const u64*)a1, (const u64*)b0,
+         (const u64*)b1, c->d_mod, c->N, first_prime);
   after_launch(c, KID_TENSOR, count);
 }
 
@@ -545,9 +546,9 @@ void launch_rescale_lift(Ptr2 tmp, Ptr2 last, int l, const LimbBatch& batch) {
   if (batch.count == 0) return;
   Context* c = ctx();
   prof_before(KID_RESCALE_LIFT);
-  rescale_lift_kernel<<<grid_for(c->N, 2, batch.count), kThreads, 0, c->stream>>>(
-      tmp, last, c->primes[l], c->d_ql_neg + (size_t)l * c->L, c->d_ql_mod + (size_t)l * c->L,
-      batch, c->d_mod, c->N);
+  launch(rescale_lift_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
+         tmp, last, c->primes[l], c->d_ql_neg + (size_t)l * c->L, c->d_ql_mod + (size_t)l * c->L,
+         batch, c->d_mod, c->N);
   after_launch(c, KID_RESCALE_LIFT, batch.count);
 }
 
@@ -555,19 +556,19 @@ void launch_rescale_combine(Ptr2 res, Ptr2 poly, Ptr2 tmp, int l, const LimbBatc
   if (batch.count == 0) return;
   Context* c = ctx();
   prof_before(KID_RESCALE_COMBINE);
-  rescale_combine_kernel<<<grid_for(c->N, 2, batch.count), kThreads, 0, c->stream>>>(
-      res, poly, tmp, c->d_ql_inv + (size_t)l * c->L, batch, c->d_mod, c->N);
+  launch(rescale_combine_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
+         res, poly, tmp, c->d_ql_inv + (size_t)l * c->L, batch, c->d_mod, c->N);
   after_launch(c, KID_RESCALE_COMBINE, batch.count);
 }
 
 template <int NIN>
 static void base_conv_dispatch(Context* c, const ConvArgs& args, dim3 grid, int chunk) {
   if (c->primes_below_2_60)
-    base_conv_kernel<NIN, true><<<grid, kThreads, 0, c->stream>>>(args, chunk, c->L, c->d_mod,
-                                                                  c->N);
+    launch(base_conv_kernel<NIN, true>, grid, kThreads, 0, c->stream,
+           args, chunk, c->L, c->d_mod, c->N);
   else
-    base_conv_kernel<NIN, false><<<grid, kThreads, 0, c->stream>>>(args, chunk, c->L, c->d_mod,
-                                                                   c->N);
+    launch(base_conv_kernel<NIN, false>, grid, kThreads, 0, c->stream,
+           args, chunk, c->L, c->d_mod, c->N);
 }
 
 void launch_base_conv(const ConvArgs& args) {
@@ -614,7 +615,7 @@ void launch_moddown_combine(const ModDownTail& args) {
   prof_before(KID_MODDOWN_COMBINE);
   dim3 g = grid_for(c->N, 2, args.level);
   g.z    = args.polys;
-  moddown_combine_kernel<<<g, kThreads, 0, c->stream>>>(args, c->d_p_inv, c->d_mod, c->N);
+  launch(moddown_combine_kernel, g, kThreads, 0, c->stream, args, c->d_p_inv, c->d_mod, c->N);
   after_launch(c, KID_MODDOWN_COMBINE, args.level * args.polys);
 }
 
@@ -623,9 +624,9 @@ void launch_moddown_rescale(int64_t* res, const int64_t* x, const int64_t* t, in
   Context* c    = ctx();
   const int last = level - 1;
   prof_before(KID_MODDOWN_COMBINE);
-  moddown_rescale_kernel<<<grid_for(c->N, 2, last), kThreads, 0, c->stream>>>(
-      (u64*)res, (const u64*)x, (const u64*)t, last, c->d_p_inv,
-      c->d_ql_inv + (size_t)last * c->L, c->d_mod, c->N);
+  launch(moddown_rescale_kernel, grid_for(c->N, 2, last), kThreads, 0, c->stream,
+         (u64*)res, (const u64*)x, (const u64*)t, last, c->d_p_inv,
+         c->d_ql_inv + (size_t)last * c->L, c->d_mod, c->N);
   after_launch(c, KID_MODDOWN_COMBINE, last);
 }
 
@@ -634,8 +635,8 @@ void launch_rescale_coeff(Ptr2 res, Ptr2 x, int polys, int level) {
   Context*  c    = ctx();
   const int last = level - 1;
   prof_before(KID_RESCALE_COMBINE);
-  rescale_coeff_kernel<<<grid_for(c->N, 2, polys * last), kThreads, 0, c->stream>>>(
-      res, x, last, c->d_ql_inv + (size_t)last * c->L, c->d_mod, c->N);
+  launch(rescale_coeff_kernel, grid_for(c->N, 2, polys * last), kThreads, 0, c->stream,
+         res, x, last, c->d_ql_inv + (size_t)last * c->L, c->d_mod, c->N);
   after_launch(c, KID_RESCALE_COMBINE, polys * last);
 }
 
@@ -670,8 +671,7 @@ void launch_inner_product(const InnerArgs& args) {
   bool fast = c->primes_below_2_60;
   bool two  = args.acc1 != nullptr;
 #define IP_CASE(TWO_, FAST_, U_, EXACT_)                                                       \
-  inner_product_kernel<TWO_, FAST_, U_, EXACT_><<<g, kThreads, 0, c->stream>>>(args, c->L,      \
-                                                                              c->d_mod, c->N)
+  launch(inner_product_kernel<TWO_, FAST_, U_, EXACT_>, g, kThreads, 0, c->stream, args, c->L, c->d_mod, c->N)
 #define IP_GROUPS(TWO_, FAST_)                                 \
   do {                                                         \
     if (args.parts == 1) IP_CASE(TWO_, FAST_, 1, true);        \
@@ -700,8 +700,8 @@ void launch_mod_raise(int64_t* res, const int64_t* src, const LimbBatch& batch) 
   }
   dag.commit();
   prof_before(KID_MOD_RAISE);
-  mod_raise_kernel<<<grid_for(c->N, 2, batch.count), kThreads, 0, c->stream>>>(
-      (u64*)res, (const u64*)src, c->primes[0], batch, c->d_mod, c->N);
+  launch(mod_raise_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
+         (u64*)res, (const u64*)src, c->primes[0], batch, c->d_mod, c->N);
   after_launch(c, KID_MOD_RAISE, batch.count);
 }
 

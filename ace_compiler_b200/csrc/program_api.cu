@@ -370,6 +370,7 @@ void trace_sum(const char* what, CIPHER ciph) {
 extern "C" {
 
 void Copy_ciph(CIPHER res, CIPHER ciph) {
+  LaunchScope scope;
   trace_sum("copy", ciph);
   init_from_ciph(res, ciph, ciph->_scaling_factor, ciph->_sf_degree);
   Copy_poly(&res->_c0_poly, &ciph->_c0_poly);

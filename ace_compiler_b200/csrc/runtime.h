@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/fhert_b200.h"
+#include "launch.h"
 #include "modarith.cuh"
 
 namespace fhert {
@@ -319,6 +320,7 @@ struct DagScope {
 };
 // cudaMemsetAsync of device memory to zero on the library stream, described
 inline cudaError_t zero_async(void* p, size_t bytes, cudaStream_t stream) {
+  if (launch_copy(p, nullptr, bytes, stream)) return cudaSuccess;
   DagScope dag(DAG_CLEAR);
   if (dag.live) dag.set.write(p, bytes);
   dag.commit();
@@ -341,6 +343,7 @@ void image_replay_release();  // drops a captured run (context teardown)
 // cudaStreamSynchronize that first ends a running capture
 inline cudaError_t stream_sync(cudaStream_t stream) {
   if (image_capturing()) image_capture_break("a synchronisation");
+  launch_flush();
   return cudaStreamSynchronize(stream);
 }
 
@@ -556,6 +559,8 @@ inline cudaError_t counted_copy(void* dst, const void* src, size_t bytes, cudaMe
     if (kind == cudaMemcpyHostToDevice) c->h2d_bytes += bytes;
     else if (kind == cudaMemcpyDeviceToHost) c->d2h_bytes += bytes;
   }
+  if (kind == cudaMemcpyDeviceToDevice && launch_copy(dst, src, bytes, stream)) return cudaSuccess;
+  launch_flush();
   DagScope dag(DAG_COPY);
   if (dag.live) {
     if (kind == cudaMemcpyDeviceToDevice) dag.set.read(src, bytes);
