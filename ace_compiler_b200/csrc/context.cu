@@ -6,6 +6,7 @@
 // fhe-cmplr/rtlib/ant/.
 #include <sched.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <unordered_map>
@@ -295,7 +296,13 @@ DevModulus make_dev_modulus(u64 q, uint32_t n) {
   d.mu_hi       = (u64)(mu >> 64);
   d.mu_lo       = (u64)mu;
   d.bits        = 64 - __builtin_clzll(q);
-  d.pad         = 0;
+  // double precision needs the margins derived in ntt_kernels.cuh; uncorrected
+  // integer butterflies keep up to 65q in a word
+  d.kind = n < 512 ? kNttWide
+           : q < (u64)(1.2 * (double)(1ull << 46)) ? kNttFloat
+           : q < (u64)0xFFFFFFFFFFFFFFFFull / 70   ? kNttNarrow
+                                                   : kNttWide;
+  d.q_recip = 1.0 / (double)q;
   d.bar         = (u64)(((u128)1 << (d.bits - 1 + 64)) / q);
   d.n_inv       = n ? invmod(n % q, q) : 0;
   d.n_inv_p     = n ? shoup(d.n_inv, q) : 0;
@@ -321,6 +328,51 @@ static Twiddle tw_of(u64 w, u64 q) {
   t.w  = w;
   t.wp = shoup(w, q);
   return t;
+}
+
+// One prime's twiddles (tree order: entry m + i of ntt.c:91-138) in the layout
+// the kernels read.  The last eight stages of a transform work on blocks of 256
+// words under tree node 2^S1 + blk; block blk's entries are
+//   [1 .. 15]               the nodes of its first four stages, in tree order
+//   [16 + ..]               stage 4 + l, twiddle 2^l + h of thread t, as entry j = 2^l + h:
+//                           integers [j][t], doubles [j / 2][t][j % 2]
+// so that 16 lanes read neighbouring entries; integers of the two-pass kernels
+// (ring degrees above 4096) are read by 32 lanes instead:
+//   [1 .. 31]               the nodes of the first five stages, in tree order
+//   [32 + j * 32 + lane]    stage 5 + l, twiddle h as j = 2^l - 1 + h
+static void pack_twiddles(Twiddle* out, const Twiddle* tree, const DevModulus& d, int logn) {
+  const bool    fp = d.kind == kNttFloat;
+  double*       f  = reinterpret_cast<double*>(out);
+  auto put = [&](size_t at, const Twiddle& t) {
+    if (!fp) out[at] = t;
+    else f[at] = t.w > (d.q >> 1) ? -(double)(d.q - t.w) : (double)t.w;  // centred
+  };
+  if (logn <= 8) {
+    std::copy(tree, tree + ((size_t)1 << logn), out);
+    return;
+  }
+  const size_t blocks = (size_t)1 << (logn - 8);
+  for (size_t i = 0; i < blocks; i++) put(i, tree[i]);
+  for (size_t b = 0; b < blocks; b++) {
+    const size_t base = blocks + b * 272, node = blocks + b;
+    if (!fp && logn > 12) {
+      for (int l = 0; l < 5; l++)
+        for (size_t h = 0; h < (1u << l); h++) put(base + (1u << l) + h, tree[(node << l) + h]);
+      for (int l = 0; l < 3; l++)
+        for (size_t h = 0; h < (1u << l); h++)
+          for (size_t lane = 0; lane < 32; lane++)
+            put(base + 32 + ((1u << l) - 1 + h) * 32 + lane, tree[(node << (5 + l)) + (lane << l) + h]);
+      continue;
+    }
+    for (int l = 0; l < 4; l++)
+      for (size_t h = 0; h < (1u << l); h++) {
+        const size_t j = (1u << l) + h;
+        put(base + j, tree[(node << l) + h]);
+        for (size_t t = 0; t < 16; t++)
+          put(base + 16 + (fp ? (j >> 1) * 32 + t * 2 + (j & 1) : j * 16 + t),
+              tree[(node << (4 + l)) + (t << l) + h]);
+      }
+  }
 }
 
 // ---- ModUp tables  (util/src/crt.c:459-566) --------------------------------
@@ -500,7 +552,8 @@ Context* create_context(const CKKS_PARAMS* p) {
   // twiddles (util/src/ntt.c:91-138): rou[brv(i)] = psi^i, rou_inv[brv(i)] = psi^-i
   const uint32_t          n = c->N;
   std::vector<DevModulus> dm(total);
-  std::vector<Twiddle>    fwd((size_t)total * n), inv((size_t)total * n), inv_last(total * 2);
+  const size_t            entries = table_entries((int)c->logN);
+  std::vector<Twiddle>    fwd(total * entries), inv(total * entries), inv_last(total * 2);
   c->psi.resize(total);
   c->h_fwd.resize(total);
   c->h_inv.resize(total);
@@ -510,8 +563,10 @@ Context* create_context(const CKKS_PARAMS* p) {
     u64 psi    = root_of_unity(2ull * n, qi);
     u64 psi_iv = invmod(psi, qi);
     c->psi[i]  = psi;
-    Twiddle* f = &fwd[(size_t)i * n];
-    Twiddle* v = &inv[(size_t)i * n];
+    c->h_fwd[i].resize(n);
+    c->h_inv[i].resize(n);
+    Twiddle* f = c->h_fwd[i].data();
+    Twiddle* v = c->h_inv[i].data();
     u64      pw = 1, pwi = 1;
     for (uint32_t k = 0; k < n; k++) {
       uint32_t r = bit_reverse(k, c->logN);
@@ -522,8 +577,9 @@ Context* create_context(const CKKS_PARAMS* p) {
     }
     inv_last[2 * i]     = tw_of(dm[i].n_inv, qi);
     inv_last[2 * i + 1] = tw_of(mulmod(v[1].w, dm[i].n_inv, qi), qi);
-    c->h_fwd[i].assign(f, f + n);
-    c->h_inv[i].assign(v, v + n);
+    c->ntt_float.push_back(dm[i].kind == kNttFloat);
+    pack_twiddles(&fwd[i * entries], f, dm[i], (int)c->logN);
+    pack_twiddles(&inv[i * entries], v, dm[i], (int)c->logN);
   }
   c->d_mod      = upload(dm);
   c->d_fwd      = upload(fwd);

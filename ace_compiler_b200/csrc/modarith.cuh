@@ -23,10 +23,15 @@ struct DevModulus {
   u64      mu_lo;
   u64      bar;      // floor(2^(bits-1+64) / q), single-word Barrett constant
   uint32_t bits;     // bit length of q
-  uint32_t pad;
+  uint32_t kind;     // arithmetic of its transforms, NttKind
   u64      n_inv;    // N^-1 mod q and its Shoup companion
   u64      n_inv_p;
+  double   q_recip;  // 1 / q
 };
+
+// Arithmetic of the transforms under one prime (ntt_kernels.cuh): double
+// precision, 64-bit integers without or with a range correction per butterfly.
+enum NttKind : uint32_t { kNttFloat, kNttNarrow, kNttWide };
 
 __device__ __forceinline__ u64 add_mod(u64 a, u64 b, u64 q) {
   u64 s = a + b;

@@ -1,27 +1,39 @@
 // Negacyclic NTT / inverse NTT over one or many RNS limbs: launch side.
 // The kernels and the arithmetic are in ntt_kernels.cuh.
+#include <algorithm>
+
 #include "ntt_kernels.cuh"
 
 namespace fhert {
 
 namespace {
 
-// Column tiles of the strided pass: 4 columns (128 threads at N = 2^16, 64 CTAs
-// per limb) measured fastest at every batch size from 2 to 48 limbs; ring
-// degrees below 2^14 keep 16 columns so that a CTA has at least two warps.
+// The two-pass kernels want the limbs transformed in integers first (they take
+// longest, the others fill up behind them); returns how many there are.
+int integers_first(Context* c, LimbBatch& b) {
+  auto* mid = std::stable_partition(b.limb, b.limb + b.count,
+                                    [&](const LimbRef& r) { return !c->ntt_float[r.prime]; });
+  return (int)(mid - b.limb);
+}
 
 template <bool INV>
-void launch_dir(Ptr2 in, Ptr2 out, const LimbBatch& b) {
+void launch_dir(Ptr2 in, Ptr2 out, const LimbBatch& unsorted) {
   Context*        c = ctx();
+  LimbBatch       b = unsorted;
   nttk::NttTables t{c->d_fwd, c->d_inv, c->d_inv_last, c->d_mod, c->N, (int)c->logN};
-  if (t.logn <= nttk::kSmallMaxLog) {
+  if (t.logn <= nttk::kWholeMaxLog) {  // one launch
+    DagScope dag(DAG_NTT);
+    dag.batch(b, c->N, &out, &in, nullptr);
+    dag.commit();
     prof_before(INV ? KID_INTT_SMALL : KID_NTT_SMALL);
-    nttk::launch_small<INV>(in, out, b, t, c->stream);
+    if (t.logn <= nttk::kTinyMaxLog) nttk::launch_tiny<INV>(in, out, b, t, c->stream);
+    else nttk::launch_whole<INV>(in, out, b, t, c->stream);
     prof_after(INV ? KID_INTT_SMALL : KID_NTT_SMALL, b.count);
     c->launches++;
     CUDA_CHECK(cudaGetLastError());
     return;
   }
+  const int n_int = integers_first(c, b);
   // the second pass works in place on `out`
   LimbBatch b2 = b;
   for (int i = 0; i < b2.count; i++) {
@@ -32,22 +44,19 @@ void launch_dir(Ptr2 in, Ptr2 out, const LimbBatch& b) {
   DagScope dag(DAG_NTT);
   dag.batch(b, c->N, &out, &in, nullptr);
   dag.commit();
-  const bool narrow_tiles = t.logn >= 14;
   if (!INV) {
     prof_before(KID_NTT_STRIDED);
-    if (narrow_tiles) nttk::launch_strided<false, 4>(in, out, b, t, c->stream);
-    else nttk::launch_strided<false, 16>(in, out, b, t, c->stream);
+    nttk::launch_strided<false>(in, out, b, n_int, t, c->stream);
     prof_after(KID_NTT_STRIDED, b.count);
     prof_before(KID_NTT_CONTIG);
-    nttk::launch_contig<false>(out, out, b2, t, c->stream);
+    nttk::launch_contig<false>(out, out, b2, n_int, t, c->stream);
     prof_after(KID_NTT_CONTIG, b.count);
   } else {
     prof_before(KID_INTT_CONTIG);
-    nttk::launch_contig<true>(in, out, b, t, c->stream);
+    nttk::launch_contig<true>(in, out, b, n_int, t, c->stream);
     prof_after(KID_INTT_CONTIG, b.count);
     prof_before(KID_INTT_STRIDED);
-    if (narrow_tiles) nttk::launch_strided<true, 4>(out, out, b2, t, c->stream);
-    else nttk::launch_strided<true, 16>(out, out, b2, t, c->stream);
+    nttk::launch_strided<true>(out, out, b2, n_int, t, c->stream);
     prof_after(KID_INTT_STRIDED, b.count);
   }
   c->launches += 2;
@@ -56,13 +65,13 @@ void launch_dir(Ptr2 in, Ptr2 out, const LimbBatch& b) {
 
 }  // namespace
 
-bool ntt_can_fuse() { return (int)ctx_noflush()->logN > nttk::kSmallMaxLog; }
+bool ntt_can_fuse() { return (int)ctx_noflush()->logN > nttk::kTinyMaxLog; }
 
 void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const NttFuse& f) {
   if (b.count == 0) return;
   Context*        c = ctx();
   nttk::NttTables t{c->d_fwd, c->d_inv, c->d_inv_last, c->d_mod, c->N, (int)c->logN};
-  FHERT_ASSERT(t.logn > nttk::kSmallMaxLog, "fused transform needs the two-pass kernels");
+  FHERT_ASSERT(t.logn > nttk::kTinyMaxLog, "ring degree too small for a fused transform");
   nttk::NttPro pro;
   pro.mul    = f.pro_mul;
   pro.mod    = f.pro_mod;
@@ -80,6 +89,8 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
     b2.limb[i].a   = (uint16_t)i;
     b2.limb[i].sel = (uint8_t)(b.limb[i].sel & 6);
   }
+  const int n_int = integers_first(c, b1);
+  integers_first(c, b2);
   DagScope dag(DAG_NTT_FUSED);
   if (dag.live) {
     const size_t w = (size_t)c->N * sizeof(u64);
@@ -93,13 +104,19 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
     }
   }
   dag.commit();
-  const bool narrow_tiles = t.logn >= 14;
+  if (t.logn <= nttk::kWholeMaxLog) {
+    prof_before(KID_NTT_SMALL);
+    nttk::launch_whole<false>(in, out, b, t, c->stream, pro, epi);
+    prof_after(KID_NTT_SMALL, b.count);
+    c->launches++;
+    CUDA_CHECK(cudaGetLastError());
+    return;
+  }
   prof_before(KID_NTT_STRIDED);
-  if (narrow_tiles) nttk::launch_strided<false, 4>(in, ptr2(mid), b1, t, c->stream, pro);
-  else nttk::launch_strided<false, 16>(in, ptr2(mid), b1, t, c->stream, pro);
+  nttk::launch_strided<false>(in, ptr2(mid), b1, n_int, t, c->stream, pro);
   prof_after(KID_NTT_STRIDED, b.count);
   prof_before(KID_NTT_CONTIG);
-  nttk::launch_contig<false>(ptr2(mid), out, b2, t, c->stream, epi);
+  nttk::launch_contig<false>(ptr2(mid), out, b2, n_int, t, c->stream, epi);
   prof_after(KID_NTT_CONTIG, b.count);
   c->launches += 2;
   CUDA_CHECK(cudaGetLastError());

@@ -1,37 +1,55 @@
 // Device code of the negacyclic NTT / inverse NTT (kernels and butterflies).
 //
-// Dataflow and twiddle indexing follow the CPU runtime exactly
+// Dataflow and twiddle values follow the CPU runtime exactly
 // (fhe-cmplr/rtlib/ant/util/src/ntt.c:167-241 forward, 245-330 inverse):
 // forward = Cooley-Tukey, natural order in, bit-reversed order out, stage
-// m = 1, 2, .., N/2 uses twiddle table entry m + i for butterfly group i;
-// inverse = Gentleman-Sande in the opposite order with N^-1 applied.  Residues
-// written by the last pass are canonical, which makes them equal to the CPU
-// runtime's.
+// m = 1, 2, .., N/2 uses twiddle m + i for butterfly group i; inverse =
+// Gentleman-Sande in the opposite order with N^-1 applied.  Residues written by
+// the last pass are canonical, which makes them equal to the CPU runtime's.
 //
-// What bounds these kernels is the half-rate 32-bit multiplier pipe: every
-// 32x32 multiply-add occupies it for two cycles per warp, 64-bit additions
-// and compares run on the full-rate integer pipe beside it.  The butterflies
-// are therefore written to need as few multiplies as possible:
-//   * the Shoup quotient floor(b*w'/2^64) is taken from three partial
-//     products instead of the exact four-product-and-carry sequence
+// What bounds these kernels is the multiplier of a butterfly's modular product.
+// A 32x32 -> 64 integer multiply-add keeps its pipe for four cycles per warp, a
+// low 32-bit one for two, and a Shoup product of 64-bit words needs three of
+// the former, two high halves (four cycles each) and four of the latter: 37
+// cycles per warp and butterfly with everything around it.  A double-precision
+// multiply-add takes two cycles and multiplies 53 bits exactly, so primes that
+// fit (below 1.2 * 2^46: every scaling prime of the compiled programs) are
+// transformed in floating point, 8 operations per butterfly, 17 cycles:
+//   h = b*w, l = fma(b, w, -h)       the exact product as h + l
+//   k = rint(h / p)                  with the reciprocal and the 1.5 * 2^52 trick
+//   r = fma(-k, p, h) + l            b*w - k*p, |r| < 0.8 p, every step exact
+// (registers-only loop, 12 butterflies per thread and round: 2120 against 990
+// G butterflies/s, 0.25 against 0.53 us per limb of 2^16).  The products are
+// integers below 2^97 in magnitude, so h + l is the product itself and the
+// remainder is an exact integer; the result after the last reduction is the
+// same canonical residue.  The error of k stays below 0.3 because values are
+// kept below 25p: forward values grow by less than 0.8p per stage (at most 14p
+// over 17 stages), in the inverse the sums double and are reduced once per
+// four stages.
+//
+// Wider primes keep 64-bit integers:
+//   * the Shoup quotient floor(b*w'/2^64) is taken from three partial products
 //     (it may come out up to 2 too small, the product then lies in [0, 4q));
-//   * b*w - quotient*q is one accumulation chain against -q (two wide and
-//     four low multiply-adds, no separate subtraction);
-//   * primes with enough headroom below 2^64 skip the per-butterfly range
-//     correction altogether: forward values grow by 4q per stage (at most
-//     (1 + 4 logN) q), inverse values double per stage (at most 2^(logN+1) q),
-//     and one reduction at the very end makes them canonical.  Wider primes
-//     keep a Harvey-style conditional subtraction with the range [0, 8q)
-//     forward and [0, 4q) inverse.
+//   * b*w - quotient*q is one accumulation chain against -q;
+//   * primes below 2^57.9 skip the per-butterfly range correction: forward
+//     values grow by 4q per stage, inverse sums double over the four stages of
+//     a register round and are brought back below 4q after it.  The 60-bit
+//     primes correct per butterfly (range [0, 8q) forward, [0, 4q) inverse).
 //
-// Three kernels per direction:
-//   small    N <= 4096: one CTA per limb, whole limb in shared memory.
+// A thread keeps 2^E values and does up to E stages between two exchanges:
+//   whole    512 <= N <= 4096: one CTA per limb, 16 values per thread, one launch.
 //   strided  first logN-8 stages: a CTA owns TC adjacent columns of the
-//            (N/256) x 256 view of the limb; every thread keeps 8 rows in
-//            registers and does up to three stages between exchanges.
-//   contig   last 8 stages: a warp owns one contiguous 256-word block.
+//            (N/256) x 256 view of the limb.
+//   contig   last 8 stages on contiguous 256-word blocks.
+//   tiny     N < 512: shared memory, one butterfly at a time.
+// The two-pass kernels use 16 values (two rounds of four stages, one exchange)
+// in double precision and 8 (three rounds) in integers: with 24 instructions
+// per integer butterfly, 16 values per thread measured 69 us for 48 limbs where
+// 8 take 49 (straight-line code executed once per warp, and 120 registers).  A
+// batch lists its integer limbs first; one grid covers both kinds, and CTAs of
+// both run side by side on the two multiplier pipes.
 // The inverse runs contig first, then strided.  Between the two passes the
-// values stay lazy (not canonical).
+// values stay lazy (doubles as their bit patterns).
 #pragma once
 #include "runtime.h"
 
@@ -40,9 +58,12 @@ namespace nttk {
 
 typedef unsigned int u32;
 
-constexpr int kContigLog   = 8;    // stages handled by the contiguous kernel
+constexpr int kContigLog   = 8;  // stages handled by the contiguous kernel
 constexpr int kContigBlock = 256;
-constexpr int kWarpsPerCta = 4;    // contiguous kernel: independent warps per CTA
+constexpr int kContigTable = kContigBlock + 16;  // twiddle entries per block
+constexpr int kThreads     = 128;  // two-pass kernels
+constexpr int kTinyMaxLog  = 8;  // below: no register rounds
+constexpr int kWholeMaxLog = 12;
 
 __device__ __forceinline__ u32 lo32(u64 x) { return (u32)x; }
 __device__ __forceinline__ u32 hi32(u64 x) { return (u32)(x >> 32); }
@@ -52,7 +73,10 @@ __device__ __forceinline__ u64 pack64(u32 l, u32 h) {
   return r;
 }
 
-// Per-limb constants kept in registers.
+__host__ __device__ constexpr int floor_log2(int v) { return v < 2 ? 0 : 1 + floor_log2(v >> 1); }
+
+// ---- integer arithmetic ------------------------------------------------------
+
 struct Mod {
   u64 q, nq, q2, q4;  // q, 2^64 - q, 2q, 4q
 };
@@ -99,9 +123,19 @@ __device__ __forceinline__ u64 canon_any(u64 v, const Mod m, u64 r) {
   return canon_4q(pack64(lo32(t), th), m);
 }
 
-// Work fused into a forward transform (all optional).
+__device__ __forceinline__ u64 add_canon(u64 a, u64 b, u64 q) { return csub(a + b, q); }
+
+__device__ __forceinline__ Twiddle ld_tw(const Twiddle* p) {
+  ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
+  Twiddle    t;
+  t.w  = v.x;
+  t.wp = v.y;
+  return t;
+}
+
+// ---- work fused into a forward transform (all optional) ------------------------
 //
-// Prologue of the strided pass, the lift of a rescale (rns_poly.c:351-366): the
+// Prologue of the first pass, the lift of a rescale (rns_poly.c:351-366): the
 // source limb holds residues modulo q_last in coefficient form; the value that
 // enters the transform under prime i is
 //   switch_modulus(v, q_last -> q_i) * mul[i].
@@ -110,7 +144,7 @@ struct NttPro {
   const u64*     mod = nullptr;  // [prime] q_last mod q_i
   u64            q_last = 0;
 };
-// Epilogue of the contiguous pass on the canonical transform output t:
+// Epilogue of the last pass on the canonical transform output t:
 //   kind 1 (rescale, rns_poly.c:367-383):  res = aux * mul[i] + t
 //   kind 2 (ModDown, rns_poly.c:293-304):  res = (aux - t) * mul[i] (+ add)
 // aux is limb LimbRef::b of aux.p[sel bit 1]; add uses the same limb index and
@@ -122,130 +156,396 @@ struct NttEpi {
   Ptr2           add{{nullptr, nullptr}};
 };
 
-__device__ __forceinline__ u64 add_canon(u64 a, u64 b, u64 q) { return csub(a + b, q); }
+// ---- the two arithmetics --------------------------------------------------------
+//
+// V: a value in registers, T: a twiddle.  load/store convert canonical words,
+// bits/from_bits move lazy values between the passes.
 
-// Cooley-Tukey.  WIDE: a, b in [0, 8q) -> [0, 8q).  Otherwise no correction:
-// the bound of both values grows by 4q.
-template <bool WIDE>
-__device__ __forceinline__ void ct_bfly(u64& a, u64& b, const Twiddle t, const Mod m) {
-  u64 x = WIDE ? csub(a, m.q4) : a;
-  u64 v = shoup4(b, t, m);
-  a     = x + v;
-  b     = x - v + m.q4;
-}
+struct ArithFp {
+  typedef double V;
+  typedef double T;
+  static constexpr bool kFloat = true;
+  double p, np, pinv;
+  u64    q, rq;
 
-// Gentleman-Sande.  WIDE: a, b in [0, 4q) -> [0, 4q), mq = 4q.  Otherwise no
-// correction: mq is a multiple of q not below the bound of b, the sum doubles.
-template <bool WIDE>
-__device__ __forceinline__ void gs_bfly(u64& a, u64& b, const Twiddle t, const Mod m, u64 mq) {
-  u64 s = a + b;
-  u64 d = a - b + mq;
-  a     = WIDE ? csub(s, m.q4) : s;
-  b     = shoup4(d, t, m);
-}
+  __device__ __forceinline__ explicit ArithFp(const DevModulus& d) {
+    p    = (double)d.q;
+    np   = -p;
+    pinv = d.q_recip;
+    q    = d.q;
+    rq   = d.mu_hi;
+  }
+  static constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
+  static constexpr double kWord  = 4503599627370496.0;  // 2^52
 
-__device__ __forceinline__ Twiddle ld_tw(const Twiddle* p) {
-  ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
-  Twiddle    t;
-  t.w  = v.x;
-  t.wp = v.y;
-  return t;
-}
+  static __device__ __forceinline__ V from_bits(u64 v) { return __longlong_as_double((long long)v); }
+  static __device__ __forceinline__ u64 bits(V v) { return (u64)__double_as_longlong(v); }
+  // canonical residue (below 2^52) -> value
+  static __device__ __forceinline__ V load(u64 v) {
+    return __dadd_rn(__hiloint2double((int)(hi32(v) | 0x43300000u), (int)lo32(v)), -kWord);
+  }
+  __device__ __forceinline__ double nearest(double v) const {  // rint(v / p)
+    return __dadd_rn(__fma_rn(v, pinv, kRound), -kRound);
+  }
+  // product of an integer below 25p with a twiddle, |result| < 0.8 p
+  __device__ __forceinline__ V mul(V b, T w) const {
+    double h = __dmul_rn(b, w);
+    double k = nearest(h);
+    double l = __fma_rn(b, w, -h);
+    return __dadd_rn(__fma_rn(k, np, h), l);
+  }
+  __device__ __forceinline__ V reduce(V v) const { return __fma_rn(nearest(v), np, v); }
+  // |v| < p -> canonical word
+  __device__ __forceinline__ u64 word(V v) const {
+    const long long magic = 0x4338000000000000ll;
+    long long       i     = __double_as_longlong(__dadd_rn(v, kRound)) - magic;
+    return (u64)(i + ((i >> 63) & (long long)q));
+  }
+  __device__ __forceinline__ u64 canon(V v) const { return word(reduce(v)); }
 
-// Where a round takes its twiddles from.  get<L>(jb, hp) returns the twiddle of
-// local stage L with index jb + hp inside the stage (jb is the part that
-// depends on the thread, hp the unrolled butterfly-group number).
-struct TwGlobal {
-  const Twiddle* tw;   // the prime's table
-  uint32_t       node; // (1 << s0) + blk: the transform's node in the table's tree order
-  template <int L>
-  __device__ __forceinline__ Twiddle get(uint32_t jb, int hp) const {
-    return ld_tw(tw + ((size_t)node << L) + jb + hp);
+  __device__ __forceinline__ void fwd(V& a, V& b, T w) const {
+    V r = mul(b, w), x = a;
+    a   = __dadd_rn(x, r);
+    b   = __dadd_rn(x, -r);
+  }
+  template <int K>
+  __device__ __forceinline__ void inv(V& a, V& b, T w) const {
+    V d = __dadd_rn(a, -b);
+    a   = __dadd_rn(a, b);
+    b   = mul(d, w);
+  }
+  // last inverse stage with N^-1 folded in, canonical words out
+  template <int K>
+  __device__ __forceinline__ void inv_last(V& a, V& b, T n_inv, T w_n) const {
+    V s = __dadd_rn(a, b), d = __dadd_rn(a, -b);
+    a   = from_bits(word(mul(s, n_inv)));
+    b   = from_bits(word(mul(d, w_n)));
+  }
+  // after R inverse stages value k is a sum of 2^R inputs (k = 0) or of
+  // 2^(R-1-log2 k) products: only sums of more than two need a reduction before
+  // the next round
+  template <int R, int K>
+  __device__ __forceinline__ void settle(V& v) const {
+    if (K == 0 || R - 1 - floor_log2(K) > 1) v = reduce(v);
+  }
+  template <int NT>
+  static __device__ __forceinline__ void twiddles(T (&t)[NT], const T* p) {
+    if constexpr (NT == 1) {
+      t[0] = __ldg(p);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NT; i += 2) {
+        double2 v = __ldg(reinterpret_cast<const double2*>(p + i));
+        t[i]      = v.x;
+        t[i + 1]  = v.y;
+      }
+    }
+  }
+  // stage l of a block's last four, thread g of 16
+  template <int L, int NT>
+  static __device__ __forceinline__ void twiddles16(T (&t)[NT], const T* block, int g) {
+    if constexpr (L == 0) {
+      t[0] = __ldg(block + 16 + 2 * g + 1);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NT; i += 2) {
+        double2 v = __ldg(reinterpret_cast<const double2*>(block + 16 + ((NT + i) >> 1) * 32 + 2 * g));
+        t[i]      = v.x;
+        t[i + 1]  = v.y;
+      }
+    }
+  }
+  // a constant of the integer tables, centred like the twiddles
+  __device__ __forceinline__ T constant(const Twiddle* c) const {
+    double w = load(ld_tw(c).w);
+    return w > 0.5 * p ? __dadd_rn(w, np) : w;
+  }
+
+  // the lift of a rescale; a dropped prime below 2^48 is centred in floating
+  // point (its product with w has a quotient below 2^47), a wider one goes through words
+  struct Lift {
+    bool   on, narrow;
+    u64    q_last, half, last_mod_q;
+    double w, dq_last;
+  };
+  __device__ __forceinline__ Lift make_lift(const NttPro& pro, int prime) const {
+    Lift l{};
+    l.on = pro.mul != nullptr;
+    if (l.on) {
+      l.q_last     = pro.q_last;
+      l.half       = pro.q_last >> 1;
+      l.narrow     = (pro.q_last >> 48) == 0;
+      l.last_mod_q = pro.mod[prime];
+      l.w          = constant(pro.mul + prime);
+      l.dq_last    = (double)pro.q_last;
+    }
+    return l;
+  }
+  __device__ __forceinline__ V lift(u64 v, const Lift& l) const {
+    if (l.narrow) {
+      V x = load(v);
+      if (v > l.half) x = __dadd_rn(x, -l.dq_last);
+      return mul(x, l.w);
+    }
+    const Mod m = make_mod(q);
+    u64       r = canon_any(v, m, rq);
+    if (v > l.half) r = r >= l.last_mod_q ? r - l.last_mod_q : r + q - l.last_mod_q;
+    return mul(load(r), l.w);
+  }
+  template <int EPI>
+  __device__ __forceinline__ u64 epilogue(u64 t, u64 aux, T w) const {
+    if (EPI == 1) return canon(__dadd_rn(mul(load(aux), w), load(t)));
+    return word(mul(__dadd_rn(load(aux), -load(t)), w));
   }
 };
-// Multiple of q covering the inputs of inverse stage k (1 = first stage done,
-// inputs canonical): bound of the values after k-1 uncorrected stages is
-// 2^k q for k >= 2 and q for k = 1.
-__device__ __forceinline__ u64 inv_cover(const Mod m, int k) { return k <= 1 ? m.q : m.q << k; }
 
-// One register round of R consecutive forward stages starting at local stage
-// L0 of a 2^S-point transform.  The thread holds the 8 elements
-// base | (e << LOWPOS), e = 0..7, with LOWPOS = S - L0 - R.  The twiddle of
-// local stage l for element index idx is entry idx >> (S - l) of that stage
-// (table entry (1 << (s0 + l)) + (blk << l) + (idx >> (S - l))).
-template <bool WIDE, int R, int S, int L0, typename TW, int U = 0>
-__device__ __forceinline__ void fwd_round(u64 (&x)[8], int base, const TW tws, const Mod m) {
-  if constexpr (U < R) {
-    constexpr int  bit = R - 1 - U;
-    constexpr int  l   = L0 + U;
-    // the register field starts at bit S - L0 - R, so the element offset
-    // (hp << (bit+1)) shifted there and then right by S - l is hp itself
-    const uint32_t jb  = (uint32_t)base >> (S - l);
+template <bool WIDE>
+struct ArithInt {
+  typedef u64     V;
+  typedef Twiddle T;
+  static constexpr bool kFloat = false;
+  Mod m;
+  u64 q, rq;
+
+  __device__ __forceinline__ explicit ArithInt(const DevModulus& d) {
+    m  = make_mod(d.q);
+    q  = d.q;
+    rq = d.mu_hi;
+  }
+  static __device__ __forceinline__ V from_bits(u64 v) { return v; }
+  static __device__ __forceinline__ u64 bits(V v) { return v; }
+  static __device__ __forceinline__ V load(u64 v) { return v; }
+  __device__ __forceinline__ u64 canon(V v) const {
+    return WIDE ? canon_4q(csub(v, m.q4), m) : canon_any(v, m, rq);
+  }
+  __device__ __forceinline__ void fwd(V& a, V& b, const T t) const {
+    u64 x = WIDE ? csub(a, m.q4) : a;
+    u64 v = shoup4(b, t, m);
+    a     = x + v;
+    b     = x - v + m.q4;
+  }
+  // K: stages already done in this round; without correction sums stay below 4q << K
+  template <int K>
+  __device__ __forceinline__ void inv(V& a, V& b, const T t) const {
+    u64 s = a + b;
+    u64 d = a - b + (WIDE ? m.q4 : m.q4 << K);
+    a     = WIDE ? csub(s, m.q4) : s;
+    b     = shoup4(d, t, m);
+  }
+  template <int K>
+  __device__ __forceinline__ void inv_last(V& a, V& b, const T n_inv, const T w_n) const {
+    u64 s = a + b, d = a - b + (WIDE ? m.q4 : m.q4 << K);
+    a     = canon_4q(shoup4(s, n_inv, m), m);
+    b     = canon_4q(shoup4(d, w_n, m), m);
+  }
+  // after R uncorrected inverse stages value k is below 4q << R (k = 0) or
+  // 4q << (R-1-log2 k): back below 4q
+  template <int R, int K>
+  __device__ __forceinline__ void settle(V& v) const {
+    constexpr int over = K == 0 ? R : R - 1 - floor_log2(K);
+    if (WIDE) return;
+    if (over > 3) v = csub(v, m.q4 << 3);
+    if (over > 2) v = csub(v, m.q4 << 2);
+    if (over > 1) v = csub(v, m.q4 << 1);
+    if (over > 0) v = csub(v, m.q4);
+  }
+  template <int NT>
+  static __device__ __forceinline__ void twiddles(T (&t)[NT], const T* p) {
 #pragma unroll
-    for (int hp = 0; hp < (8 >> (bit + 1)); hp++) {
-      Twiddle t = tws.template get<l>(jb, hp);
+    for (int i = 0; i < NT; i++) t[i] = ld_tw(p + i);
+  }
+  template <int L, int NT>
+  static __device__ __forceinline__ void twiddles16(T (&t)[NT], const T* block, int g) {
+#pragma unroll
+    for (int i = 0; i < NT; i++) t[i] = ld_tw(block + 16 + (NT + i) * 16 + g);
+  }
+  __device__ __forceinline__ T constant(const Twiddle* c) const { return ld_tw(c); }
+
+  struct Lift {
+    bool on;
+    u64  half, last_mod_q;
+    T    w;
+  };
+  __device__ __forceinline__ Lift make_lift(const NttPro& pro, int prime) const {
+    Lift l{};
+    l.on = pro.mul != nullptr;
+    if (l.on) {
+      l.half       = pro.q_last >> 1;
+      l.last_mod_q = pro.mod[prime];
+      l.w          = constant(pro.mul + prime);
+    }
+    return l;
+  }
+  __device__ __forceinline__ V lift(u64 v, const Lift& l) const {
+    u64 r = canon_any(v, m, rq);
+    if (v > l.half) r = r >= l.last_mod_q ? r - l.last_mod_q : r + q - l.last_mod_q;
+    return canon_4q(shoup4(r, l.w, m), m);
+  }
+  template <int EPI>
+  __device__ __forceinline__ u64 epilogue(u64 t, u64 aux, const T w) const {
+    if (EPI == 1) return add_canon(canon_4q(shoup4(aux, w, m), m), t, q);
+    return canon_4q(shoup4(aux >= t ? aux - t : aux + q - t, w, m), m);
+  }
+};
+
+// ---- register rounds --------------------------------------------------------------
+//
+// A thread holds the 2^E values of an E-bit field of the index; a round does the
+// stages of the R highest bits of the field.  Stage l of the round (bit E-1-l)
+// has 2^l groups with one twiddle each: entries node << l .. of the tree, where
+// node is the tree node of the field's subtree.
+
+template <class A>
+struct TreeTw {  // tree order
+  const typename A::T* table;
+  u32                  node;
+  template <int L, int NT>
+  __device__ __forceinline__ void get(typename A::T (&t)[NT]) const {
+    A::twiddles(t, table + ((size_t)node << L));
+  }
+};
+template <class A>
+struct Lanes16Tw {  // last four stages of a block, laid out for 16 lanes
+  const typename A::T* block;
+  int                  t;
+  template <int L, int NT>
+  __device__ __forceinline__ void get(typename A::T (&tw)[NT]) const {
+    A::template twiddles16<L>(tw, block, t);
+  }
+};
+struct Lanes32Tw {  // last three stages of a block of integers, laid out for 32 lanes
+  const Twiddle* block;
+  int            lane;
+  template <int L, int NT>
+  __device__ __forceinline__ void get(Twiddle (&tw)[NT]) const {
+#pragma unroll
+    for (int i = 0; i < NT; i++) tw[i] = ld_tw(block + 32 + ((1 << L) - 1 + i) * 32 + lane);
+  }
+};
+
+// stages [L, R) of a round
+template <class A, int E, int R, int L, class TW>
+__device__ __forceinline__ void fwd_stages(typename A::V (&x)[1 << E], const TW& tw, const A& ar) {
+  if constexpr (L < R) {
+    constexpr int bit = E - 1 - L, groups = 1 << L;
+    typename A::T t[groups];
+    tw.template get<L>(t);
+#pragma unroll
+    for (int hp = 0; hp < groups; hp++)
 #pragma unroll
       for (int lp = 0; lp < (1 << bit); lp++) {
-        int lo = (hp << (bit + 1)) | lp;
-        ct_bfly<WIDE>(x[lo], x[lo | (1 << bit)], t, m);
+        const int lo = (hp << (bit + 1)) | lp;
+        ar.fwd(x[lo], x[lo | (1 << bit)], t[hp]);
       }
-    }
-    fwd_round<WIDE, R, S, L0, TW, U + 1>(x, base, tws, m);
+    fwd_stages<A, E, R, L + 1, TW>(x, tw, ar);
   }
 }
 
-// Inverse round: same stages, processed from the highest local stage down.
-// KBASE - l is the 1-based count of the inverse stage (for the cover of the
-// uncorrected form).  When LAST is set and the round reaches local stage 0,
-// the final butterfly applies N^-1 (fin[0] = N^-1, fin[1] = rou_inv[1]*N^-1)
-// and leaves canonical values.
-template <bool WIDE, int R, int S, int L0, int KBASE, bool LAST, typename TW, int U = R - 1>
-__device__ __forceinline__ void inv_round(u64 (&x)[8], int base, const TW tws, const Mod m,
-                                          const Twiddle* fin) {
-  if constexpr (U >= 0) {
-    constexpr int bit = R - 1 - U;
-    constexpr int l   = L0 + U;
-    const u64     mq  = WIDE ? m.q4 : inv_cover(m, KBASE - l);
-    if constexpr (LAST && l == 0) {
-      Twiddle n_inv = ld_tw(fin), w_n = ld_tw(fin + 1);
+// LAST: the round that reaches the first stage of the transform
+template <class A, int E, int R, int L, bool LAST, class TW>
+__device__ __forceinline__ void inv_stages(typename A::V (&x)[1 << E], const TW& tw, const A& ar,
+                                           const Twiddle* fin) {
+  if constexpr (L >= 0) {
+    constexpr int bit = E - 1 - L, groups = 1 << L, done = R - 1 - L;
+    if constexpr (LAST && L == 0) {
+      const typename A::T n_inv = ar.constant(fin), w_n = ar.constant(fin + 1);
 #pragma unroll
-      for (int hp = 0; hp < (8 >> (bit + 1)); hp++) {
-#pragma unroll
-        for (int lp = 0; lp < (1 << bit); lp++) {
-          int lo = (hp << (bit + 1)) | lp;
-          int hi = lo | (1 << bit);
-          u64 sum = x[lo] + x[hi];
-          u64 dif = x[lo] - x[hi] + mq;
-          x[lo]   = canon_4q(shoup4(sum, n_inv, m), m);
-          x[hi]   = canon_4q(shoup4(dif, w_n, m), m);
-        }
-      }
+      for (int lp = 0; lp < (1 << bit); lp++)
+        ar.template inv_last<done>(x[lp], x[lp | (1 << bit)], n_inv, w_n);
     } else {
-      const uint32_t jb = (uint32_t)base >> (S - l);
+      typename A::T t[groups];
+      tw.template get<L>(t);
 #pragma unroll
-      for (int hp = 0; hp < (8 >> (bit + 1)); hp++) {
-        Twiddle t = tws.template get<l>(jb, hp);
+      for (int hp = 0; hp < groups; hp++)
 #pragma unroll
         for (int lp = 0; lp < (1 << bit); lp++) {
-          int lo = (hp << (bit + 1)) | lp;
-          gs_bfly<WIDE>(x[lo], x[lo | (1 << bit)], t, m, mq);
+          const int lo = (hp << (bit + 1)) | lp;
+          ar.template inv<done>(x[lo], x[lo | (1 << bit)], t[hp]);
         }
-      }
     }
-    inv_round<WIDE, R, S, L0, KBASE, LAST, TW, U - 1>(x, base, tws, m, fin);
+    inv_stages<A, E, R, L - 1, LAST, TW>(x, tw, ar, fin);
   }
 }
 
-// Bank swizzle for a 256-word block accessed with the three lane patterns of
-// the contiguous kernel (lanes over index bits {0..4}, {0,1,5,6,7}, {3..7}):
-// a permutation inside each aligned 16-word group that keeps every half-warp
-// on 16 distinct 8-byte banks.  It is linear over XOR, so for an index made of
-// disjoint bit fields swz(a | b) = swz(a) ^ swz(b): the per-element part is a
-// compile-time constant.
-__host__ __device__ constexpr int swz(int i) {
-  return i ^ (((i >> 4) & 1) << 1) ^ (((i >> 5) & 1) << 2) ^ (((i >> 6) & 1) << 3) ^ ((i >> 6) & 1);
+template <class A, int E, int R, int I = 0>
+__device__ __forceinline__ void settle_all(typename A::V (&x)[1 << E], const A& ar) {
+  if constexpr (I < (1 << E)) {
+    ar.template settle<R, (I >> (E - R))>(x[I]);
+    settle_all<A, E, R, I + 1>(x, ar);
+  }
 }
 
+// ---- contiguous 256-point blocks (global stages logN-8 .. logN-1) ---------------
+//
+// 16 lanes (16 values each): word (row r, column c) of the 16 x 16 view of the
+// block sits at column c ^ r of its row: rows and columns are then both read and
+// written without bank conflicts.
+//   by_row: thread t touches column t of every row e (coalesced order e*16 + t)
+//   by_col: thread t touches row t, columns e        (contiguous order t*16 + e)
+
+__device__ __forceinline__ int by_row(int t, int e) { return e * 16 + (t ^ e); }
+__device__ __forceinline__ int by_col(int t, int e) { return t * 16 + (e ^ t); }
+
+// x holds e*16 + t (lazy) on entry; leaves canonical words in shared memory
+template <class A>
+__device__ __forceinline__ void contig16_fwd(typename A::V (&x)[16], u64* sb, int t,
+                                             const typename A::T* table, const A& ar) {
+  fwd_stages<A, 4, 4, 0>(x, TreeTw<A>{table, 1u}, ar);
+#pragma unroll
+  for (int e = 0; e < 16; e++) sb[by_row(t, e)] = A::bits(x[e]);
+  __syncwarp();
+#pragma unroll
+  for (int e = 0; e < 16; e++) x[e] = A::from_bits(sb[by_col(t, e)]);
+  fwd_stages<A, 4, 4, 0>(x, Lanes16Tw<A>{table, t}, ar);
+#pragma unroll
+  for (int e = 0; e < 16; e++) sb[by_col(t, e)] = ar.canon(x[e]);
+  __syncwarp();
+}
+
+// canonical words in shared memory on entry; x holds e*16 + t (lazy) on exit
+template <class A>
+__device__ __forceinline__ void contig16_inv(typename A::V (&x)[16], u64* sb, int t,
+                                             const typename A::T* table, const A& ar) {
+#pragma unroll
+  for (int e = 0; e < 16; e++) x[e] = A::load(sb[by_col(t, e)]);
+  inv_stages<A, 4, 4, 3, false>(x, Lanes16Tw<A>{table, t}, ar, nullptr);
+  settle_all<A, 4, 4>(x, ar);
+#pragma unroll
+  for (int e = 0; e < 16; e++) sb[by_col(t, e)] = A::bits(x[e]);
+  __syncwarp();
+#pragma unroll
+  for (int e = 0; e < 16; e++) x[e] = A::from_bits(sb[by_row(t, e)]);
+  inv_stages<A, 4, 4, 3, false>(x, TreeTw<A>{table, 1u}, ar, nullptr);
+  settle_all<A, 4, 4>(x, ar);
+}
+
+// what becomes of transform word `v` of a limb with an epilogue
+template <class A, int EPI>
+__device__ __forceinline__ u64 finish_word(u64 v, int i, const u64* aux, const u64* add,
+                                           const typename A::T& emul, const A& ar) {
+  if (EPI != 0) {
+    v = ar.template epilogue<EPI>(v, aux[i], emul);
+    if (EPI == 2 && add != nullptr) v = add_canon(v, add[i], ar.q);
+  }
+  return v;
+}
+
+template <class A, int EPI>
+__device__ __forceinline__ void write_block16(u64* dst, const u64* sb, int t, const u64* aux,
+                                              const u64* add, const typename A::T& emul, const A& ar) {
+#pragma unroll
+  for (int e = 0; e < 16; e++)
+    dst[e * 16 + t] = finish_word<A, EPI>(sb[by_row(t, e)], e * 16 + t, aux, add, emul, ar);
+}
+
+// 32 lanes (8 values each), rounds of 2, 3 and 3 stages with the index patterns
+// e*32 + g, (b2 | e*8), g*8 + e.  The swizzle is a permutation inside each
+// aligned 16-word group that keeps every half-warp on 16 distinct 8-byte banks
+// for all three; it is linear over XOR, so with the block's shared memory
+// aligned to its size the addresses of one thread differ by constants.
+__host__ __device__ constexpr int swz(int i) {
+  return i ^ ((i >> 4) & 1) ^ (((i >> 5) & 1) << 1) ^ (((i >> 6) & 1) * 12);
+}
 __device__ __forceinline__ u64 lds64(u32 addr) {
   u64 v;
   asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
@@ -255,305 +555,396 @@ __device__ __forceinline__ void sts64(u32 addr, u64 v) {
   asm volatile("st.shared.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
 }
 
-// ---- contiguous 256-point blocks (global stages logN-8 .. logN-1) ----------
-//
-// One warp per block; the warp's 2 KiB of shared memory is aligned to its size
-// so that the swizzled byte address is (block base ^ swizzled offset).
-
-template <bool INV, bool WIDE, int EPI>
-__device__ __forceinline__ void contig_block(const u64* __restrict__ src, u64* __restrict__ dst,
-                                             u32 sbase, const TwGlobal tw, const Mod m, u64 rq,
-                                             int g, const u64* aux, const u64* add,
-                                             const Twiddle emul) {
-  u64 x[8];
-  // byte addresses inside the warp's block for the three lane patterns
-  const int b1 = g;                              // elements e*32 + g
-  const int b2 = ((g >> 2) << 5) | (g & 3);      // elements b2 | e<<2
-  const int b3 = g << 3;                         // elements g*8 + e
-  const u32 a1 = sbase ^ (u32)(swz(b1) << 3);
+template <bool INV, int EPI, class A>
+__device__ __forceinline__ void contig_int(const u64* src, u64* dst, u32 sbase, int g,
+                                           const Twiddle* table, const A& ar, const u64* aux,
+                                           const u64* add, const Twiddle* emul) {
+  u64       x[8];
+  const int b2 = ((g >> 3) << 6) | (g & 7);
+  const u32 a1 = sbase ^ (u32)(swz(g) << 3);
   const u32 a2 = sbase ^ (u32)(swz(b2) << 3);
-  const u32 a3 = sbase ^ (u32)(swz(b3) << 3);
+  const u32 a3 = sbase ^ (u32)(swz(g << 3) << 3);
+  const TreeTw<A>  first{table, 1u}, second{table, 4u + (u32)(g >> 3)};
+  const Lanes32Tw  third{table, g};
   if constexpr (!INV) {
 #pragma unroll
     for (int e = 0; e < 8; e++) x[e] = src[e * 32 + g];
-    fwd_round<WIDE, 3, kContigLog, 0>(x, b1, tw, m);
+    fwd_stages<A, 3, 2, 0>(x, first, ar);
 #pragma unroll
     for (int e = 0; e < 8; e++) sts64(a1 ^ (u32)(swz(e << 5) << 3), x[e]);
     __syncwarp();
 #pragma unroll
-    for (int e = 0; e < 8; e++) x[e] = lds64(a2 ^ (u32)(swz(e << 2) << 3));
-    fwd_round<WIDE, 3, kContigLog, 3>(x, b2, tw, m);
+    for (int e = 0; e < 8; e++) x[e] = lds64(a2 ^ (u32)(swz(e << 3) << 3));
+    fwd_stages<A, 3, 3, 0>(x, second, ar);
 #pragma unroll
-    for (int e = 0; e < 8; e++) sts64(a2 ^ (u32)(swz(e << 2) << 3), x[e]);
+    for (int e = 0; e < 8; e++) sts64(a2 ^ (u32)(swz(e << 3) << 3), x[e]);
     __syncwarp();
 #pragma unroll
     for (int e = 0; e < 8; e++) x[e] = lds64(a3 ^ (u32)(swz(e) << 3));
-    fwd_round<WIDE, 2, kContigLog, 6>(x, b3, tw, m);
+    fwd_stages<A, 3, 3, 0>(x, third, ar);
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-      u64 v = WIDE ? canon_4q(csub(x[e], m.q4), m) : canon_any(x[e], m, rq);
-      sts64(a3 ^ (u32)(swz(e) << 3), v);
-    }
+    for (int e = 0; e < 8; e++) sts64(a3 ^ (u32)(swz(e) << 3), ar.canon(x[e]));
     __syncwarp();
+    typename A::T w{};
+    if (EPI != 0) w = ar.constant(emul);
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-      u64 t = lds64(a1 ^ (u32)(swz(e << 5) << 3));
-      if (EPI == 1) {
-        t = add_canon(canon_4q(shoup4(aux[e * 32 + g], emul, m), m), t, m.q);
-      } else if (EPI == 2) {
-        u64 x = aux[e * 32 + g];
-        t     = canon_4q(shoup4(x >= t ? x - t : x + m.q - t, emul, m), m);
-        if (add != nullptr) t = add_canon(t, add[e * 32 + g], m.q);
-      }
-      dst[e * 32 + g] = t;
-    }
+    for (int e = 0; e < 8; e++)
+      dst[e * 32 + g] =
+          finish_word<A, EPI>(lds64(a1 ^ (u32)(swz(e << 5) << 3)), e * 32 + g, aux, add, w, ar);
   } else {
-    // inverse stage counts 1..8 are local stages 7..0: KBASE = 8
 #pragma unroll
     for (int e = 0; e < 8; e++) sts64(a1 ^ (u32)(swz(e << 5) << 3), src[e * 32 + g]);
     __syncwarp();
 #pragma unroll
     for (int e = 0; e < 8; e++) x[e] = lds64(a3 ^ (u32)(swz(e) << 3));
-    inv_round<WIDE, 2, kContigLog, 6, 8, false>(x, b3, tw, m, nullptr);
+    inv_stages<A, 3, 3, 2, false>(x, third, ar, nullptr);
+    settle_all<A, 3, 3>(x, ar);
 #pragma unroll
     for (int e = 0; e < 8; e++) sts64(a3 ^ (u32)(swz(e) << 3), x[e]);
     __syncwarp();
 #pragma unroll
-    for (int e = 0; e < 8; e++) x[e] = lds64(a2 ^ (u32)(swz(e << 2) << 3));
-    inv_round<WIDE, 3, kContigLog, 3, 8, false>(x, b2, tw, m, nullptr);
+    for (int e = 0; e < 8; e++) x[e] = lds64(a2 ^ (u32)(swz(e << 3) << 3));
+    inv_stages<A, 3, 3, 2, false>(x, second, ar, nullptr);
+    settle_all<A, 3, 3>(x, ar);
 #pragma unroll
-    for (int e = 0; e < 8; e++) sts64(a2 ^ (u32)(swz(e << 2) << 3), x[e]);
+    for (int e = 0; e < 8; e++) sts64(a2 ^ (u32)(swz(e << 3) << 3), x[e]);
     __syncwarp();
 #pragma unroll
     for (int e = 0; e < 8; e++) x[e] = lds64(a1 ^ (u32)(swz(e << 5) << 3));
-    inv_round<WIDE, 3, kContigLog, 0, 8, false>(x, b1, tw, m, nullptr);
+    inv_stages<A, 3, 2, 1, false>(x, first, ar, nullptr);
+    settle_all<A, 3, 2>(x, ar);
 #pragma unroll
     for (int e = 0; e < 8; e++) dst[e * 32 + g] = x[e];
   }
 }
 
-// narrow = no range correction is needed over the whole transform
-__device__ __forceinline__ bool fwd_narrow(uint32_t bits) { return bits <= 57; }
-__device__ __forceinline__ bool inv_narrow(uint32_t bits, int logn) { return bits + logn + 1 <= 64; }
+template <bool INV, int EPI>
+__device__ __forceinline__ void contig_float(const u64* src, u64* dst, u64* sb, int t,
+                                             const double* table, const ArithFp& ar, const u64* aux,
+                                             const u64* add, const Twiddle* emul) {
+  double x[16];
+  if constexpr (!INV) {
+#pragma unroll
+    for (int e = 0; e < 16; e++) x[e] = ArithFp::from_bits(src[e * 16 + t]);
+    contig16_fwd<ArithFp>(x, sb, t, table, ar);
+    double w = 0;
+    if (EPI != 0) w = ar.constant(emul);
+    write_block16<ArithFp, EPI>(dst, sb, t, aux, add, w, ar);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 16; e++) sb[by_row(t, e)] = src[e * 16 + t];
+    __syncwarp();
+    contig16_inv<ArithFp>(x, sb, t, table, ar);
+#pragma unroll
+    for (int e = 0; e < 16; e++) dst[e * 16 + t] = ArithFp::bits(x[e]);
+  }
+}
+
+// CTA -> limb of the batch and tile of the limb.  Limbs [0, n_int) of the batch
+// are transformed in integers, 2^log_int tiles each, the others in double
+// precision, 2^log_float tiles each.
+struct TileMap {
+  u32 n_int, log_int, log_float;
+};
+__device__ __forceinline__ bool locate(const TileMap& map, u32& limb, u32& tile) {
+  const u32 ints = map.n_int << map.log_int;
+  if (blockIdx.x < ints) {
+    limb = blockIdx.x >> map.log_int;
+    tile = blockIdx.x & ((1u << map.log_int) - 1);
+    return true;
+  }
+  const u32 b = blockIdx.x - ints;
+  limb = map.n_int + (b >> map.log_float);
+  tile = b & ((1u << map.log_float) - 1);
+  return false;
+}
 
 template <bool INV, int EPI>
-__global__ void __launch_bounds__(kWarpsPerCta * 32)
-ntt_contig_kernel(Ptr2 in, Ptr2 out, LimbBatch batch, const Twiddle* __restrict__ tables,
-                  const DevModulus* __restrict__ mods, uint32_t n, int logn, NttEpi epi) {
-  __shared__ __align__(2048) u64 sm[kWarpsPerCta * kContigBlock];
-  const LimbRef    lr   = batch.limb[blockIdx.y];
-  const DevModulus dm   = mods[lr.prime];
-  const Mod        m    = make_mod(dm.q);
-  const Twiddle*   tw   = tables + (size_t)lr.prime * n;
-  const int        warp = threadIdx.x >> 5;
-  const int        g    = threadIdx.x & 31;
-  const uint32_t   blk  = blockIdx.x * kWarpsPerCta + warp;  // block in limb
-  const size_t     off  = (size_t)blk * kContigBlock;
-  const u64*       src  = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + off;
-  u64*             dst  = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n + off;
-  const u32 sbase = (u32)__cvta_generic_to_shared(sm) + (u32)warp * (kContigBlock * 8);
-  const int s0    = logn - kContigLog;
-
-  const bool narrow = INV ? inv_narrow(dm.bits, logn) : fwd_narrow(dm.bits);
-  const u64* aux  = nullptr;
-  const u64* add  = nullptr;
-  Twiddle    emul{0, 0};
+__global__ void __launch_bounds__(kThreads, 6)
+ntt_contig_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, TileMap map,
+                  const Twiddle* __restrict__ tables, const DevModulus* __restrict__ mods, uint32_t n,
+                  int logn, NttEpi epi) {
+  // 16 KiB for the blocks and up to 2 KiB to align them
+  __shared__ u64 sm[kThreads / 16 * kContigBlock + kContigBlock];
+  u32              limb, tile;
+  const bool       is_int = locate(map, limb, tile);
+  const LimbRef    lr     = batch.limb[limb];
+  const DevModulus dm     = mods[lr.prime];
+  const int        s1     = logn - kContigLog;
+  const Twiddle*   tab    = tables + (size_t)lr.prime * table_entries(logn);
+  const int        per    = is_int ? 32 : 16;  // lanes per block
+  const int        slot = threadIdx.x / per, t = threadIdx.x & (per - 1);
+  const u32        blk    = tile * (kThreads / per) + slot;
+  const size_t     off    = (size_t)blk * kContigBlock;
+  const u64*       src    = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + off;
+  u64*             dst    = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n + off;
+  const u64* aux = nullptr;
+  const u64* add = nullptr;
   if (EPI != 0) {
     const size_t aoff = (size_t)lr.b * n + off;
-    aux  = ((lr.sel & 2) ? epi.aux.p[1] : epi.aux.p[0]) + aoff;
-    add  = (lr.sel & 2) ? epi.add.p[1] : epi.add.p[0];
+    aux = ((lr.sel & 2) ? epi.aux.p[1] : epi.aux.p[0]) + aoff;
+    add = (lr.sel & 2) ? epi.add.p[1] : epi.add.p[0];
     if (add != nullptr) add += aoff;
-    emul = ld_tw(epi.mul + lr.prime);
   }
-  const TwGlobal tws{tw, (1u << s0) + blk};
-  if (narrow)
-    contig_block<INV, false, EPI>(src, dst, sbase, tws, m, dm.mu_hi, g, aux, add, emul);
-  else
-    contig_block<INV, true, EPI>(src, dst, sbase, tws, m, dm.mu_hi, g, aux, add, emul);
+  const Twiddle* emul  = EPI != 0 ? epi.mul + lr.prime : nullptr;
+  const size_t   entry = ((size_t)1 << s1) + (size_t)blk * kContigTable;
+  if (is_int) {
+    const u32 sbase = (((u32)__cvta_generic_to_shared(sm) + 2047u) & ~2047u) + (u32)slot * 2048u;
+    if (dm.kind == kNttNarrow)
+      contig_int<INV, EPI>(src, dst, sbase, t, tab + entry, ArithInt<false>(dm), aux, add, emul);
+    else
+      contig_int<INV, EPI>(src, dst, sbase, t, tab + entry, ArithInt<true>(dm), aux, add, emul);
+  } else {
+    contig_float<INV, EPI>(src, dst, sm + slot * kContigBlock, t,
+                           reinterpret_cast<const double*>(tab) + entry, ArithFp(dm), aux, add, emul);
+  }
 }
 
 // ---- strided columns (global stages 0 .. logN-9) ---------------------------
 //
-// S1 = logN - 8 stages on 2^S1 rows; TC columns per CTA; threads = TC * 2^(S1-3).
-// Rounds cover local stages [l0, l0+R): forward ascending from 0 with R = 3
-// while three are left, inverse descending with the odd-sized round first.
+// S1 = logN - 8 stages on 2^S1 rows; TC columns per CTA; threads = TC * 2^(S1-E).
+// The first forward round does the odd S1 % E stages (or E), the others E each;
+// the inverse runs the same rounds backwards.
 
-// the lift of a rescale: residue modulo q_last (centred) -> residue modulo q, times w
-__device__ __forceinline__ u64 lift_value(u64 v, u64 q_last, u64 last_mod_q, const Twiddle w,
-                                          const Mod m, u64 rq) {
-  u64 r = canon_any(v, m, rq);
-  if (v > (q_last >> 1)) r = r >= last_mod_q ? r - last_mod_q : r + m.q - last_mod_q;
-  return canon_4q(shoup4(r, w, m), m);
+__host__ __device__ constexpr int first_round(int s, int e) { return s % e == 0 ? e : s % e; }
+
+// row r, column c of the tile; rows 2^E apart would meet in the same banks when
+// a tile row is shorter than 128 bytes
+template <int E, int TC>
+__device__ __forceinline__ int tile_at(int row, int c) {
+  constexpr int spread = TC < 16 ? 16 / TC - 1 : 0;
+  return ((row ^ ((row >> E) & spread)) * TC) | c;
 }
 
-struct LiftArgs {
-  bool    on;
-  u64     q_last, last_mod_q, rq;
-  Twiddle w;
-};
-
-template <bool WIDE, int S1, int TC, int L0>
-__device__ __forceinline__ void strided_fwd(u64 (&x)[8], const u64* __restrict__ src,
-                                            u64* __restrict__ dst, u64* sm, int g, int c,
-                                            const Twiddle* tw, const Mod m, const LiftArgs lift) {
-  constexpr int R      = (S1 - L0 < 3) ? (S1 - L0) : 3;
-  constexpr int LOWPOS = S1 - L0 - R;
-  const int base = ((g >> LOWPOS) << (LOWPOS + 3)) | (g & ((1 << LOWPOS) - 1));
-  if constexpr (L0 == 0) {
-#pragma unroll
-    for (int e = 0; e < 8; e++) x[e] = src[(size_t)(base | (e << LOWPOS)) << kContigLog];
-    if (lift.on) {
-#pragma unroll
-      for (int e = 0; e < 8; e++)
-        x[e] = lift_value(x[e], lift.q_last, lift.last_mod_q, lift.w, m, lift.rq);
-    }
-  } else {
+template <class A, int E, int S, int TC, int L0>
+__device__ __forceinline__ void strided_fwd(typename A::V (&x)[1 << E], u64* sm, int g, int c,
+                                            const typename A::T* table, const A& ar) {
+  constexpr int R    = L0 == 0 ? first_round(S, E) : E;
+  constexpr int LP   = L0 == 0 ? S - E : S - L0 - E;
+  const int     base = ((g >> LP) << (LP + E)) | (g & ((1 << LP) - 1));
+  if constexpr (L0 != 0) {
     __syncthreads();
 #pragma unroll
-    for (int e = 0; e < 8; e++) x[e] = sm[(base | (e << LOWPOS)) * TC + c];
+    for (int e = 0; e < (1 << E); e++) x[e] = A::from_bits(sm[tile_at<E, TC>(base | (e << LP), c)]);
   }
-  fwd_round<WIDE, R, S1, L0>(x, base, TwGlobal{tw, 1u}, m);
-  if constexpr (L0 + R < S1) {
-    __syncthreads();
+  fwd_stages<A, E, R, 0>(x, TreeTw<A>{table, (1u << L0) + ((u32)base >> (LP + E))}, ar);
+  if constexpr (L0 + R < S) {
+    if constexpr (L0 != 0) __syncthreads();
 #pragma unroll
-    for (int e = 0; e < 8; e++) sm[(base | (e << LOWPOS)) * TC + c] = x[e];
-    strided_fwd<WIDE, S1, TC, L0 + R>(x, src, dst, sm, g, c, tw, m, lift);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; e++) dst[(size_t)(base | (e << LOWPOS)) << kContigLog] = x[e];
+    for (int e = 0; e < (1 << E); e++) sm[tile_at<E, TC>(base | (e << LP), c)] = A::bits(x[e]);
+    strided_fwd<A, E, S, TC, L0 + R>(x, sm, g, c, table, ar);
   }
 }
 
-// HI = stages [0, HI) are still to do; the first call has HI = S1.
-template <bool WIDE, int S1, int TC, int HI>
-__device__ __forceinline__ void strided_inv(u64 (&x)[8], const u64* __restrict__ src,
-                                            u64* __restrict__ dst, u64* sm, int g, int c,
-                                            const Twiddle* tw, const Mod m, const Twiddle* fin) {
-  constexpr int R      = (HI % 3 == 0) ? 3 : HI % 3;
-  constexpr int L0     = HI - R;
-  constexpr int LOWPOS = S1 - L0 - R;
-  const int base = ((g >> LOWPOS) << (LOWPOS + 3)) | (g & ((1 << LOWPOS) - 1));
-  if constexpr (HI == S1) {
-#pragma unroll
-    for (int e = 0; e < 8; e++) x[e] = src[(size_t)(base | (e << LOWPOS)) << kContigLog];
-  } else {
+// HI: stages [0, HI) are still to do
+template <class A, int E, int S, int TC, int HI>
+__device__ __forceinline__ void strided_inv(typename A::V (&x)[1 << E], u64* sm, int g, int c,
+                                            const typename A::T* table, const A& ar,
+                                            const Twiddle* fin) {
+  constexpr bool LAST = HI == first_round(S, E);
+  constexpr int  R    = LAST ? HI : E;
+  constexpr int  L0   = HI - R;
+  constexpr int  LP   = LAST ? S - E : S - L0 - E;
+  const int      base = ((g >> LP) << (LP + E)) | (g & ((1 << LP) - 1));
+  if constexpr (HI != S) {
     __syncthreads();
 #pragma unroll
-    for (int e = 0; e < 8; e++) x[e] = sm[(base | (e << LOWPOS)) * TC + c];
+    for (int e = 0; e < (1 << E); e++) x[e] = A::from_bits(sm[tile_at<E, TC>(base | (e << LP), c)]);
   }
-  // inverse stage count of local stage l: 8 contiguous stages came first
-  inv_round<WIDE, R, S1, L0, kContigLog + S1, true>(x, base, TwGlobal{tw, 1u}, m, fin);
-  if constexpr (L0 > 0) {
-    __syncthreads();
+  inv_stages<A, E, R, R - 1, LAST>(x, TreeTw<A>{table, (1u << L0) + ((u32)base >> (LP + E))}, ar, fin);
+  if constexpr (!LAST) {
+    settle_all<A, E, R>(x, ar);
+    if constexpr (HI != S) __syncthreads();
 #pragma unroll
-    for (int e = 0; e < 8; e++) sm[(base | (e << LOWPOS)) * TC + c] = x[e];
-    strided_inv<WIDE, S1, TC, L0>(x, src, dst, sm, g, c, tw, m, fin);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; e++) dst[(size_t)(base | (e << LOWPOS)) << kContigLog] = x[e];
+    for (int e = 0; e < (1 << E); e++) sm[tile_at<E, TC>(base | (e << LP), c)] = A::bits(x[e]);
+    strided_inv<A, E, S, TC, L0>(x, sm, g, c, table, ar, fin);
   }
 }
 
-template <bool INV, int S1, int TC>
-__global__ void __launch_bounds__(TC << (S1 - 3))
-ntt_strided_kernel(Ptr2 in, Ptr2 out, LimbBatch batch, const Twiddle* __restrict__ tables,
-                   const DevModulus* __restrict__ mods, const Twiddle* __restrict__ inv_last,
-                   uint32_t n, NttPro pro) {
-  extern __shared__ u64 sm_dyn[];
-  constexpr int    logn = S1 + kContigLog;
-  const LimbRef    lr   = batch.limb[blockIdx.y];
-  const DevModulus dm   = mods[lr.prime];
-  const Mod        m    = make_mod(dm.q);
-  const Twiddle*   tw   = tables + (size_t)lr.prime * n;
-  const Twiddle*   fin  = inv_last + (size_t)lr.prime * 2;
-  const int        c    = threadIdx.x & (TC - 1);
-  const int        g    = threadIdx.x / TC;  // 0 .. 2^(S1-3)-1
-  const size_t     col  = (size_t)blockIdx.x * TC + c;
-  const u64*       src  = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + col;
-  u64*             dst  = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n + col;
-  u64              x[8];
-  const bool narrow = INV ? inv_narrow(dm.bits, logn) : fwd_narrow(dm.bits);
+template <class A, int E>
+__device__ __forceinline__ void load_values(typename A::V (&x)[1 << E], const u64 (&v)[1 << E],
+                                            const A& ar, const NttPro& pro, int prime) {
+  const typename A::Lift lift = ar.make_lift(pro, prime);
+  if (lift.on) {
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) x[e] = ar.lift(v[e], lift);
+  } else {
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) x[e] = A::load(v[e]);
+  }
+}
+
+template <bool INV, int E, int S1, int TC, class A>
+__device__ __forceinline__ void strided_body(const u64* src, u64* dst, u64* sm, const Twiddle* table,
+                                             const A& ar, const Twiddle* fin, const NttPro& pro,
+                                             int prime) {
+  const typename A::T* tw = reinterpret_cast<const typename A::T*>(table);
+  const int            c = threadIdx.x % TC, g = threadIdx.x / TC;
+  typename A::V        x[1 << E];
+  // the field of the first and of the last round: top E row bits, low E row bits
+  constexpr int top = S1 - E;
+  const int     at_top = g, at_low = g << E;
+  src += c;
+  dst += c;
   if constexpr (!INV) {
-    LiftArgs lift{false, 0, 0, 0, Twiddle{0, 0}};
-    if (pro.mul != nullptr) {
-      lift.on         = true;
-      lift.q_last     = pro.q_last;
-      lift.last_mod_q = pro.mod[lr.prime];
-      lift.rq         = dm.mu_hi;
-      lift.w          = ld_tw(pro.mul + lr.prime);
-    }
-    if (narrow)
-      strided_fwd<false, S1, TC, 0>(x, src, dst, sm_dyn, g, c, tw, m, lift);
-    else
-      strided_fwd<true, S1, TC, 0>(x, src, dst, sm_dyn, g, c, tw, m, lift);
+    u64 v[1 << E];
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) v[e] = src[(size_t)(at_top | (e << top)) << kContigLog];
+    load_values<A, E>(x, v, ar, pro, prime);
+    strided_fwd<A, E, S1, TC, 0>(x, sm, g, c, tw, ar);
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) dst[(size_t)(at_low | e) << kContigLog] = A::bits(x[e]);
   } else {
-    if (narrow)
-      strided_inv<false, S1, TC, S1>(x, src, dst, sm_dyn, g, c, tw, m, fin);
-    else
-      strided_inv<true, S1, TC, S1>(x, src, dst, sm_dyn, g, c, tw, m, fin);
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) x[e] = A::from_bits(src[(size_t)(at_low | e) << kContigLog]);
+    strided_inv<A, E, S1, TC, S1>(x, sm, g, c, tw, ar, fin);
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) dst[(size_t)(at_top | (e << top)) << kContigLog] = A::bits(x[e]);
   }
 }
 
-// ---- small transforms: whole limb in shared memory -------------------------
-// Always the corrected (wide) butterflies: valid for every prime below 2^61.
+// columns per CTA: kThreads threads at every ring degree
+__host__ __device__ constexpr int tile_columns(int s1, int e) { return kThreads >> (s1 - e); }
+
+template <bool INV, int S1>
+__global__ void __launch_bounds__(kThreads, 7)
+ntt_strided_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, TileMap map,
+                   const Twiddle* __restrict__ tables, const DevModulus* __restrict__ mods,
+                   const Twiddle* __restrict__ inv_last, uint32_t n, NttPro pro) {
+  constexpr int TI = tile_columns(S1, 3), TF = tile_columns(S1, 4);
+  __shared__ u64   sm[TF << S1];
+  u32              limb, tile;
+  const bool       is_int = locate(map, limb, tile);
+  const LimbRef    lr     = batch.limb[limb];
+  const DevModulus dm     = mods[lr.prime];
+  const Twiddle*   tab    = tables + (size_t)lr.prime * table_entries(S1 + kContigLog);
+  const Twiddle*   fin    = inv_last + (size_t)lr.prime * 2;
+  const size_t     col    = (size_t)tile * (is_int ? TI : TF);
+  const u64*       src    = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + col;
+  u64*             dst    = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n + col;
+  if (!is_int)
+    strided_body<INV, 4, S1, TF>(src, dst, sm, tab, ArithFp(dm), fin, pro, lr.prime);
+  else if (dm.kind == kNttNarrow)
+    strided_body<INV, 3, S1, TI>(src, dst, sm, tab, ArithInt<false>(dm), fin, pro, lr.prime);
+  else
+    strided_body<INV, 3, S1, TI>(src, dst, sm, tab, ArithInt<true>(dm), fin, pro, lr.prime);
+}
+
+// ---- whole limb in one CTA (512 <= N <= 4096) ------------------------------------
+//
+// S1 = logN - 8 stages in one register round over the top bits, then the
+// contiguous rounds; N/16 threads.
+
+template <bool INV, int EPI, int S1, class A>
+__device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, const Twiddle* table,
+                                           const DevModulus& dm, const Twiddle* fin,
+                                           const NttPro& pro, int prime, const u64* aux,
+                                           const u64* add, const Twiddle* emul) {
+  constexpr int        logn = S1 + kContigLog, top = logn - 4;
+  const A              ar(dm);
+  const typename A::T* tree = reinterpret_cast<const typename A::T*>(table);
+  const int            g = threadIdx.x, half = g >> 4, t = g & 15;
+  const typename A::T* blk   = tree + ((size_t)1 << S1) + (size_t)half * kContigTable;
+  u64*                 sb    = sm + half * kContigBlock;
+  typename A::V        x[16];
+  // word i of the limb in the swizzled view of its block
+  auto at = [](int i) { return i ^ ((i >> 4) & 15); };
+  if constexpr (!INV) {
+    u64 v[16];
+#pragma unroll
+    for (int e = 0; e < 16; e++) v[e] = src[g | (e << top)];
+    load_values<A, 4>(x, v, ar, pro, prime);
+    fwd_stages<A, 4, S1, 0>(x, TreeTw<A>{tree, 1u}, ar);
+#pragma unroll
+    for (int e = 0; e < 16; e++) sm[at(g | (e << top))] = A::bits(x[e]);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 16; e++) x[e] = A::from_bits(sb[by_row(t, e)]);
+    __syncwarp();
+    contig16_fwd<A>(x, sb, t, blk, ar);
+    typename A::T w{};
+    if (EPI != 0) w = ar.constant(emul);
+    const size_t off = (size_t)half * kContigBlock;
+    write_block16<A, EPI>(dst + off, sb, t, aux + off, add != nullptr ? add + off : nullptr, w, ar);
+  } else {
+    const size_t off = (size_t)half * kContigBlock;
+#pragma unroll
+    for (int e = 0; e < 16; e++) sb[by_row(t, e)] = src[off + e * 16 + t];
+    __syncwarp();
+    contig16_inv<A>(x, sb, t, blk, ar);
+#pragma unroll
+    for (int e = 0; e < 16; e++) sb[by_row(t, e)] = A::bits(x[e]);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 16; e++) x[e] = A::from_bits(sm[at(g | (e << top))]);
+    inv_stages<A, 4, S1, S1 - 1, true>(x, TreeTw<A>{tree, 1u}, ar, fin);
+#pragma unroll
+    for (int e = 0; e < 16; e++) dst[g | (e << top)] = A::bits(x[e]);
+  }
+}
+
+template <bool INV, int EPI, int S1>
+__global__ void __launch_bounds__(16 << S1)
+ntt_whole_kernel(Ptr2 in, Ptr2 out, LimbBatch batch, const Twiddle* __restrict__ tables,
+                 const DevModulus* __restrict__ mods, const Twiddle* __restrict__ inv_last,
+                 NttPro pro, NttEpi epi) {
+  constexpr uint32_t n = (uint32_t)kContigBlock << S1;
+  __shared__ u64 sm[n];
+  const LimbRef    lr  = batch.limb[blockIdx.x];
+  const DevModulus dm  = mods[lr.prime];
+  const Twiddle*   tab = tables + (size_t)lr.prime * table_entries(S1 + kContigLog);
+  const Twiddle*   fin = inv_last + (size_t)lr.prime * 2;
+  const u64*       src = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n;
+  u64*             dst = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n;
+  const u64* aux = nullptr;
+  const u64* add = nullptr;
+  if (EPI != 0) {
+    aux = ((lr.sel & 2) ? epi.aux.p[1] : epi.aux.p[0]) + (size_t)lr.b * n;
+    add = (lr.sel & 2) ? epi.add.p[1] : epi.add.p[0];
+    if (add != nullptr) add += (size_t)lr.b * n;
+  }
+  const Twiddle* emul = EPI != 0 ? epi.mul + lr.prime : nullptr;
+  if (dm.kind == kNttFloat)
+    whole_body<INV, EPI, S1, ArithFp>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul);
+  else if (dm.kind == kNttNarrow)
+    whole_body<INV, EPI, S1, ArithInt<false>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul);
+  else
+    whole_body<INV, EPI, S1, ArithInt<true>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul);
+}
+
+// ---- tiny transforms (N < 512): one butterfly at a time --------------------------
+// Always the corrected (wide) butterflies; twiddles in tree order.
 
 template <bool INV>
-__global__ void ntt_small_kernel(Ptr2 in, Ptr2 out, LimbBatch batch,
-                                 const Twiddle* __restrict__ tables,
-                                 const DevModulus* __restrict__ mods,
-                                 const Twiddle* __restrict__ inv_last, uint32_t n, int logn) {
-  extern __shared__ u64 sm_dyn[];
-  const LimbRef  lr  = batch.limb[blockIdx.x];
-  const Mod      m   = make_mod(mods[lr.prime].q);
-  const Twiddle* tw  = tables + (size_t)lr.prime * n;
+__global__ void ntt_tiny_kernel(Ptr2 in, Ptr2 out, LimbBatch batch,
+                                const Twiddle* __restrict__ tables,
+                                const DevModulus* __restrict__ mods,
+                                const Twiddle* __restrict__ inv_last, uint32_t n, int logn) {
+  __shared__ u64 sm[1 << kTinyMaxLog];
+  const LimbRef        lr = batch.limb[blockIdx.x];
+  const ArithInt<true> ar(mods[lr.prime]);
+  const Twiddle* tw  = tables + (size_t)lr.prime * table_entries(logn);
   const Twiddle* fin = inv_last + (size_t)lr.prime * 2;
   const u64*     src = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n;
   u64*           dst = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sm_dyn[i] = src[i];
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sm[i] = src[i];
   __syncthreads();
-  const uint32_t half = n >> 1;
-  if (!INV) {
-    for (int l = 0; l < logn; l++) {
-      int tlog = logn - 1 - l;  // t = 2^tlog
-      for (uint32_t bf = threadIdx.x; bf < half; bf += blockDim.x) {
-        uint32_t i  = bf >> tlog;
-        uint32_t j1 = ((i << (tlog + 1))) | (bf & ((1u << tlog) - 1));
-        Twiddle  t  = ld_tw(tw + (1u << l) + i);
-        u64 a = sm_dyn[j1], b = sm_dyn[j1 + (1u << tlog)];
-        ct_bfly<true>(a, b, t, m);
-        sm_dyn[j1]                 = a;
-        sm_dyn[j1 + (1u << tlog)] = b;
-      }
-      __syncthreads();
+  for (int k = 0; k < logn; k++) {
+    const int l = INV ? logn - 1 - k : k, tlog = logn - 1 - l;
+    for (uint32_t bf = threadIdx.x; bf < (n >> 1); bf += blockDim.x) {
+      const uint32_t i  = bf >> tlog;
+      const uint32_t j1 = (i << (tlog + 1)) | (bf & ((1u << tlog) - 1));
+      u64 a = sm[j1], b = sm[j1 + (1u << tlog)];
+      if (!INV) ar.fwd(a, b, ld_tw(tw + (1u << l) + i));
+      else if (l == 0) ar.inv_last<0>(a, b, ld_tw(fin), ld_tw(fin + 1));
+      else ar.inv<0>(a, b, ld_tw(tw + (1u << l) + i));
+      sm[j1]                 = a;
+      sm[j1 + (1u << tlog)] = b;
     }
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-      dst[i] = canon_4q(csub(sm_dyn[i], m.q4), m);
-  } else {
-    for (int l = logn - 1; l >= 0; l--) {
-      int tlog = logn - 1 - l;
-      for (uint32_t bf = threadIdx.x; bf < half; bf += blockDim.x) {
-        uint32_t i  = bf >> tlog;
-        uint32_t j1 = ((i << (tlog + 1))) | (bf & ((1u << tlog) - 1));
-        u64 a = sm_dyn[j1], b = sm_dyn[j1 + (1u << tlog)];
-        if (l == 0) {
-          Twiddle n_inv = ld_tw(fin), w_n = ld_tw(fin + 1);
-          u64     sum = a + b, dif = a - b + m.q4;
-          a = canon_4q(shoup4(sum, n_inv, m), m);
-          b = canon_4q(shoup4(dif, w_n, m), m);
-        } else {
-          Twiddle t = ld_tw(tw + (1u << l) + i);
-          gs_bfly<true>(a, b, t, m, m.q4);
-        }
-        sm_dyn[j1]                 = a;
-        sm_dyn[j1 + (1u << tlog)] = b;
-      }
-      __syncthreads();
-    }
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = sm_dyn[i];
+    __syncthreads();
   }
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = INV ? sm[i] : ar.canon(sm[i]);
 }
-
-constexpr int kSmallMaxLog = 12;
 
 // Tables and geometry of one transform launch.
 struct NttTables {
@@ -565,57 +956,74 @@ struct NttTables {
   int               logn;
 };
 
-template <bool INV, int S1, int TC>
-inline void launch_strided_t(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
+// n_int: how many limbs, at the front of the batch, are transformed in integers
+template <bool INV, int S1>
+inline void launch_strided_t(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
                              cudaStream_t stream, const NttPro& pro) {
-  static bool attr_done = false;
-  const size_t smem = ((size_t)TC << S1) * sizeof(u64);
-  if (!attr_done && smem > 48 * 1024) {
-    cudaFuncSetAttribute(ntt_strided_kernel<INV, S1, TC>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr_done = true;
-  }
-  dim3 grid(kContigBlock / TC, b.count);
-  launch(ntt_strided_kernel<INV, S1, TC>, grid, TC << (S1 - 3), smem, stream,
-         in, out, b, INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, pro);
+  const TileMap map{(u32)n_int, (u32)(kContigLog - floor_log2(tile_columns(S1, 3))),
+                    (u32)(kContigLog - floor_log2(tile_columns(S1, 4)))};
+  const int     ctas = (n_int << map.log_int) + ((b.count - n_int) << map.log_float);
+  launch(ntt_strided_kernel<INV, S1>, ctas, kThreads, 0, stream, in, out, b, map,
+         INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, pro);
 }
 
-template <bool INV, int TC>
-inline void launch_strided(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
+template <bool INV>
+inline void launch_strided(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
                            cudaStream_t stream, const NttPro& pro = NttPro()) {
   switch (t.logn - kContigLog) {
-    case 5: launch_strided_t<INV, 5, TC>(in, out, b, t, stream, pro); break;
-    case 6: launch_strided_t<INV, 6, TC>(in, out, b, t, stream, pro); break;
-    case 7: launch_strided_t<INV, 7, TC>(in, out, b, t, stream, pro); break;
-    case 8: launch_strided_t<INV, 8, TC>(in, out, b, t, stream, pro); break;
-    case 9: launch_strided_t<INV, 9, TC>(in, out, b, t, stream, pro); break;
+    case 5: launch_strided_t<INV, 5>(in, out, b, n_int, t, stream, pro); break;
+    case 6: launch_strided_t<INV, 6>(in, out, b, n_int, t, stream, pro); break;
+    case 7: launch_strided_t<INV, 7>(in, out, b, n_int, t, stream, pro); break;
+    case 8: launch_strided_t<INV, 8>(in, out, b, n_int, t, stream, pro); break;
+    case 9: launch_strided_t<INV, 9>(in, out, b, n_int, t, stream, pro); break;
     default: FHERT_ASSERT(false, "ring degree 2^%d has no transform kernel", t.logn);
   }
 }
 
 template <bool INV>
-inline void launch_contig(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
+inline void launch_contig(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
                           cudaStream_t stream, const NttEpi& epi = NttEpi()) {
-  dim3 grid(t.n / (kContigBlock * kWarpsPerCta), b.count);
-  const Twiddle* tab = INV ? t.inv : t.fwd;
+  const u32      blocks = (u32)(t.logn - kContigLog);
+  const TileMap  map{(u32)n_int, blocks - floor_log2(kThreads / 32), blocks - floor_log2(kThreads / 16)};
+  const int      ctas = (n_int << map.log_int) + ((b.count - n_int) << map.log_float);
+  const Twiddle* tab  = INV ? t.inv : t.fwd;
   if (INV || epi.kind == 0)
-    launch(ntt_contig_kernel<INV, 0>, grid, kWarpsPerCta * 32, 0, stream,
-           in, out, b, tab, t.mods, t.n, t.logn, epi);
+    launch(ntt_contig_kernel<INV, 0>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
+           t.logn, epi);
   else if (epi.kind == 1)
-    launch(ntt_contig_kernel<false, 1>, grid, kWarpsPerCta * 32, 0, stream,
-           in, out, b, tab, t.mods, t.n, t.logn, epi);
+    launch(ntt_contig_kernel<false, 1>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
+           t.logn, epi);
   else
-    launch(ntt_contig_kernel<false, 2>, grid, kWarpsPerCta * 32, 0, stream,
-           in, out, b, tab, t.mods, t.n, t.logn, epi);
+    launch(ntt_contig_kernel<false, 2>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
+           t.logn, epi);
+}
+
+template <bool INV, int EPI>
+inline void launch_whole_t(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
+                           cudaStream_t stream, const NttPro& pro, const NttEpi& epi) {
+  const Twiddle* tab = INV ? t.inv : t.fwd;
+  switch (t.logn - kContigLog) {
+    case 1: launch(ntt_whole_kernel<INV, EPI, 1>, b.count, 32, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
+    case 2: launch(ntt_whole_kernel<INV, EPI, 2>, b.count, 64, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
+    case 3: launch(ntt_whole_kernel<INV, EPI, 3>, b.count, 128, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
+    default: launch(ntt_whole_kernel<INV, EPI, 4>, b.count, 256, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
+  }
 }
 
 template <bool INV>
-inline void launch_small(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
-                         cudaStream_t stream) {
-  size_t smem    = (size_t)t.n * sizeof(u64);
-  int    threads = t.n / 2 < 512 ? (t.n / 2 < 32 ? 32 : t.n / 2) : 512;
-  launch(ntt_small_kernel<INV>, b.count, threads, smem, stream,
-         in, out, b, INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, t.logn);
+inline void launch_whole(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
+                         cudaStream_t stream, const NttPro& pro = NttPro(),
+                         const NttEpi& epi = NttEpi()) {
+  if (INV || epi.kind == 0) launch_whole_t<INV, 0>(in, out, b, t, stream, pro, epi);
+  else if (epi.kind == 1) launch_whole_t<false, 1>(in, out, b, t, stream, pro, epi);
+  else launch_whole_t<false, 2>(in, out, b, t, stream, pro, epi);
+}
+
+template <bool INV>
+inline void launch_tiny(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
+                        cudaStream_t stream) {
+  launch(ntt_tiny_kernel<INV>, b.count, t.n <= 64 ? 32 : t.n / 2, 0, stream, in, out, b,
+         INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, t.logn);
 }
 
 }  // namespace nttk

@@ -73,6 +73,15 @@ struct __align__(16) Twiddle {
   u64 wp;
 };
 
+// Twiddle entries per prime and direction on the device (16 bytes each; primes
+// transformed in double precision use the first half as 8-byte entries).  Ring
+// degrees of 512 and more: the 2^(logN-8) - 1 nodes of the first stages in tree
+// order, then 272 entries for each block of the last eight stages (see
+// pack_twiddles in context.cu); below, tree order.
+__host__ __device__ constexpr size_t table_entries(int logn) {
+  return logn > 8 ? ((size_t)1 << (logn - 8)) * 273 : (size_t)1 << logn;
+}
+
 struct Context {
   uint32_t N     = 0;
   uint32_t logN  = 0;
@@ -90,8 +99,9 @@ struct Context {
 
   // device tables
   DevModulus* d_mod = nullptr;   // [L+K]
-  Twiddle*    d_fwd = nullptr;   // [L+K][N], index m+i as in ntt.c:167
-  Twiddle*    d_inv = nullptr;   // [L+K][N]
+  std::vector<uint8_t> ntt_float;  // per prime: transformed in double precision
+  Twiddle*    d_fwd = nullptr;   // [L+K][table_entries(logN)]
+  Twiddle*    d_inv = nullptr;
   // last inverse stage with N^-1 folded in: (N^-1, (rou_inv[1] * N^-1))
   Twiddle*    d_inv_last = nullptr;  // [L+K][2]
 
@@ -416,9 +426,9 @@ DevModulus make_dev_modulus(u64 q, uint32_t n);
 // out.p[(sel>>2)&1]
 void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse);
 // Forward transform with the element-wise passes around it folded in (ring
-// degrees above 4096 only: ntt_can_fuse).  The strided pass reads in[a] and
-// writes limb k of `mid` (k = position in the batch), the contiguous pass reads
-// mid[k] and writes out[dst].
+// degrees of 512 and more: ntt_can_fuse).  The first pass reads in[a] and
+// writes limb k of `mid` (k = position in the batch), the last pass reads
+// mid[k] and writes out[dst]; up to 4096 both are one launch and mid is not used.
 //   prologue (pro_mul set): the source is the coefficient form of a dropped
 //     limb modulo q_last; the value transformed under prime i is
 //     switch_modulus(v, q_last -> q_i) * pro_mul[i]   (pro_mod[i] = q_last mod q_i)
