@@ -657,8 +657,6 @@ void fhert_raise_parts(Context* c, const int64_t* src, bool is_ntt, size_t level
     args.level      = (int)level;
     args.out_total  = (int)level + K;
     args.p_limb     = p_limb;
-    args.in_stride  = c->L + K;
-    args.out_stride = 1;
     for (int g = 0; g < args.groups; g++) {
       int                        part = pb + g;
       const Context::ModUpTable& t    = modup_table(c, (int)level, part);
@@ -667,7 +665,8 @@ void fhert_raise_parts(Context* c, const int64_t* src, bool is_ntt, size_t level
       cg.in          = reinterpret_cast<const u64*>(coeff);
       cg.out         = reinterpret_cast<u64*>(ext_base + (size_t)(part - part_begin) * part_stride * n);
       cg.inv         = t.d_hat_inv;
-      cg.mat         = t.d_hat_mod;
+      args.width     = t.width;
+      cg.planes      = t.d_planes;
       cg.first_limb  = start;
       cg.first_prime = start;
       cg.count       = t.digit_len;
@@ -791,15 +790,14 @@ void fhert_mod_down_polys(Context* c, int npoly, int64_t* const res[2],
   args.level      = (int)level;
   args.out_total  = (int)level;
   args.p_limb     = 0;
-  args.in_stride  = 1;
-  args.out_stride = K;
   for (int g = 0; g < npoly; g++) {
+    args.width = (K + 3) & ~3;
     ConvGroup& cg  = args.g[g];
     cg.in          = is_ntt ? reinterpret_cast<const u64*>(sc + (size_t)g * K * n)
                             : reinterpret_cast<const u64*>(ext[g] + (size_t)ext_p_limb * n);
     cg.out         = reinterpret_cast<u64*>(conv + (size_t)g * level * n);
     cg.inv         = c->d_phat_inv;
-    cg.mat         = c->d_phat_mod_q;
+    cg.planes      = c->d_phat_planes;
     cg.first_limb  = 0;
     cg.first_prime = c->L;
     cg.count       = K;
@@ -875,13 +873,12 @@ POLY Mod_down_rescale(POLY res, POLY poly) {
   args.level      = (int)level;
   args.out_total  = (int)level;
   args.p_limb     = 0;
-  args.in_stride  = 1;
-  args.out_stride = K;
+  args.width = (K + 3) & ~3;
   ConvGroup& cg   = args.g[0];
   cg.in           = reinterpret_cast<const u64*>(poly->_data + p_offset(poly) * n);
   cg.out          = reinterpret_cast<u64*>(conv);
   cg.inv          = c->d_phat_inv;
-  cg.mat          = c->d_phat_mod_q;
+  cg.planes       = c->d_phat_planes;
   cg.first_limb   = 0;
   cg.first_prime  = c->L;
   cg.count        = K;
@@ -912,13 +909,12 @@ VALUE_LIST* Reduce_and_rescale_modup(POLY res, POLY poly) {
   args.level      = (int)level;
   args.out_total  = (int)level;
   args.p_limb     = 0;
-  args.in_stride  = 1;
-  args.out_stride = K;
+  args.width = (K + 3) & ~3;
   ConvGroup& cg   = args.g[0];
   cg.in           = reinterpret_cast<const u64*>(poly->_data + p_offset(poly) * n);
   cg.out          = reinterpret_cast<u64*>(res->_data);
   cg.inv          = c->d_phat_inv;
-  cg.mat          = c->d_phat_mod_q;
+  cg.planes       = c->d_phat_planes;
   cg.first_limb   = 0;
   cg.first_prime  = c->L;
   cg.count        = K;

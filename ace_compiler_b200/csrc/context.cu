@@ -302,7 +302,9 @@ DevModulus make_dev_modulus(u64 q, uint32_t n) {
            : q < (u64)(1.2 * (double)(1ull << 46)) ? kNttFloat
            : q < (u64)0xFFFFFFFFFFFFFFFFull / 70   ? kNttNarrow
                                                    : kNttWide;
-  d.q_recip = 1.0 / (double)q;
+  d.q_recip    = 1.0 / (double)q;
+  d.conv_shift = 8 * std::max((d.bits + 7) / 8, 2u) - 16;
+  d.conv_mu    = (uint32_t)(((u128)1 << (32 + d.conv_shift)) / q);
   d.bar         = (u64)(((u128)1 << (d.bits - 1 + 64)) / q);
   d.n_inv       = n ? invmod(n % q, q) : 0;
   d.n_inv_p     = n ? shoup(d.n_inv, q) : 0;
@@ -387,9 +389,12 @@ const Context::ModUpTable& modup_table(Context* c, int level, int digit) {
   FHERT_ASSERT(start < level, "digit %d empty at level %d", digit, level);
   t.digit_len = end - start;
   t.out_count = level - t.digit_len + c->K;
-  int              total = c->L + c->K;
+  // the digits of one level share a launch: padded to the same width
+  t.width = ((level > c->alpha ? c->alpha : t.digit_len) + 3) & ~3;
   std::vector<Twiddle> hat_inv(t.digit_len);
-  std::vector<u64> hat_mod((size_t)t.digit_len * total, 0);
+  std::vector<u64>     hat_mod((size_t)t.out_count * t.digit_len), out_primes;
+  for (int m = 0; m < level + c->K; m++)
+    if (m < start || m >= end) out_primes.push_back(c->primes[m < level ? m : c->L + (m - level)]);
   for (int i = 0; i < t.digit_len; i++) {
     u64 qi  = c->primes[start + i];
     u64 hat = 1;
@@ -397,18 +402,16 @@ const Context::ModUpTable& modup_table(Context* c, int level, int digit) {
       if (k != start + i) hat = mulmod(hat, c->primes[k] % qi, qi);
     u64 inv            = invmod(hat, qi);
     hat_inv[i]         = tw_of(inv, qi);
-    for (int m = 0; m < total; m++) {
-      bool is_q = m < c->L;
-      if (is_q && (m >= level || (m >= start && m < end))) continue;
-      u64 pm = c->primes[m];
+    for (int o = 0; o < t.out_count; o++) {
+      u64 pm = out_primes[o];
       u64 h  = 1;
       for (int k = start; k < end; k++)
         if (k != start + i) h = mulmod(h, c->primes[k] % pm, pm);
-      hat_mod[(size_t)i * total + m] = h;
+      hat_mod[(size_t)o * t.digit_len + i] = h;
     }
   }
   t.d_hat_inv = upload(hat_inv);
-  t.d_hat_mod = upload(hat_mod);
+  t.d_planes  = upload(conv_planes(t.digit_len, t.width, t.out_count, hat_mod.data(), out_primes.data()));
   return c->modup.emplace(key, t).first->second;
 }
 
@@ -549,6 +552,11 @@ Context* create_context(const CKKS_PARAMS* p) {
     CUDA_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thresh));
   }
 
+  // raised by a kernel whose bounded wait ran out; read after every synchronisation
+  CUDA_CHECK(cudaHostAlloc(&c->h_error, sizeof(uint32_t), cudaHostAllocMapped));
+  *c->h_error = 0;
+  CUDA_CHECK(cudaHostGetDevicePointer(&c->d_error, c->h_error, 0));
+
   // twiddles (util/src/ntt.c:91-138): rou[brv(i)] = psi^i, rou_inv[brv(i)] = psi^-i
   const uint32_t          n = c->N;
   std::vector<DevModulus> dm(total);
@@ -627,7 +635,7 @@ Context* create_context(const CKKS_PARAMS* p) {
     }
   }
   c->d_phat_inv   = upload(phat_inv);
-  c->d_phat_mod_q = upload(phat_mod_q);
+  c->d_phat_planes = upload(conv_planes(K, (K + 3) & ~3, L, phat_mod_q.data(), c->primes.data()));
   c->d_p_inv      = upload(p_inv);
   c->d_p_mod_q    = upload(p_mod_q);
 
@@ -661,12 +669,13 @@ void destroy_context() {
   cudaFree(c->d_ql_neg);
   cudaFree(c->d_ql_mod);
   cudaFree(c->d_phat_inv);
-  cudaFree(c->d_phat_mod_q);
+  cudaFree(c->d_phat_planes);
+  cudaFreeHost(c->h_error);
   cudaFree(c->d_p_inv);
   cudaFree(c->d_p_mod_q);
   for (auto& kv : c->modup) {
     cudaFree(kv.second.d_hat_inv);
-    cudaFree(kv.second.d_hat_mod);
+    cudaFree(kv.second.d_planes);
   }
   for (auto& kv : c->auto_tables) cudaFree(kv.second);
   for (auto& kv : c->keys) {

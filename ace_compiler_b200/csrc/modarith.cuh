@@ -27,6 +27,8 @@ struct DevModulus {
   u64      n_inv;    // N^-1 mod q and its Shoup companion
   u64      n_inv_p;
   double   q_recip;  // 1 / q
+  // base conversion (base_conv.cu): 8 * bytes of q - 16, floor(2^(32 + shift) / q)
+  uint32_t conv_shift, conv_mu;
 };
 
 // Arithmetic of the transforms under one prime (ntt_kernels.cuh): double

@@ -175,81 +175,6 @@ rescale_combine_kernel(Ptr2 res, Ptr2 poly, Ptr2 tmp, const Twiddle* __restrict_
     pr[i] = add_mod(mul_shoup(pp[i], w.w, w.wp, q), pt[i], q);
 }
 
-// ---- approximate base conversion --------------------------------------------
-// One thread per coefficient; the scaled inputs y_i stay in registers (padded
-// with zeros up to NIN), the conversion matrix of the CTA's output chunk sits
-// in shared memory.  blockIdx.y selects the chunk of outputs, blockIdx.z the
-// group (digit for ModUp, polynomial for ModDown).  With FAST the sums use the
-// carry-free 32-bit-half accumulators (all primes below 2^60, NIN <= 16).
-
-constexpr int kMaxOutChunk = 18;
-
-template <int NIN, bool FAST>
-__global__ void __launch_bounds__(kThreads)
-base_conv_kernel(ConvArgs args, int chunk, int num_q, const DevModulus* __restrict__ mods,
-                 uint32_t n) {
-  // FAST keeps the matrix pre-split into 30-bit halves (x = low, y = high)
-  __shared__ uint2 sm_mat[kMaxOutChunk * NIN];
-  const ConvGroup  g         = args.g[blockIdx.z];
-  const int        out_count = args.out_total - g.skip_len;
-  const int        o_beg     = blockIdx.y * chunk;
-  if (o_beg >= out_count) return;
-  const int o_end = min(o_beg + chunk, out_count);
-  for (int t = threadIdx.x; t < (o_end - o_beg) * NIN; t += kThreads) {
-    int o = t / NIN, i = t - o * NIN;
-    int m = o_beg + o;
-    m     = m < g.skip_start ? m : m + g.skip_len;
-    int prime = m < args.level ? m : num_q + (m - args.level);
-    u64 v = i < g.count
-                ? g.mat[(size_t)i * args.in_stride + (size_t)prime * args.out_stride]
-                : 0;
-    sm_mat[t] = FAST ? make_uint2((uint32_t)v & 0x3fffffffu, (uint32_t)(v >> 30))
-                     : make_uint2((uint32_t)v, (uint32_t)(v >> 32));
-  }
-  __syncthreads();
-  const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
-  if (c >= n) return;
-  uint32_t y0[NIN], y1[NIN];  // halves of y_i: 30-bit split (FAST) or 32-bit split
-#pragma unroll
-  for (int i = 0; i < NIN; i++) {
-    u64 y = 0;
-    if (i < g.count) {
-      const Twiddle w = g.inv[i];
-      y = mul_shoup(g.in[(size_t)(g.first_limb + i) * n + c], w.w, w.wp,
-                    mods[g.first_prime + i].q);
-    }
-    y0[i] = FAST ? ((uint32_t)y & 0x3fffffffu) : (uint32_t)y;
-    y1[i] = FAST ? (uint32_t)(y >> 30) : (uint32_t)(y >> 32);
-  }
-  for (int o = o_beg; o < o_end; o++) {
-    int m     = o < g.skip_start ? o : o + g.skip_len;
-    if ((args.skip_mask >> m) & 1) continue;
-    int prime = m < args.level ? m : num_q + (m - args.level);
-    int limb  = m < args.level ? m : args.p_limb + (m - args.level);
-    const DevModulus md  = mods[prime];
-    const uint2*     row = sm_mat + (o - o_beg) * NIN;
-    u64              hi, lo;
-    if (FAST) {
-      Acc4 acc;
-      acc4_zero(acc);
-#pragma unroll
-      for (int i = 0; i < NIN; i++) {
-        const uint2 b = row[i];
-        acc4_mac_halves(acc, y0[i], y1[i], b.x, b.y);
-      }
-      acc4_fold(acc, hi, lo);
-    } else {
-      hi = lo = 0;
-#pragma unroll
-      for (int i = 0; i < NIN; i++) {
-        const uint2 b = row[i];
-        mac_128(hi, lo, ((u64)y1[i] << 32) | y0[i], ((u64)b.y << 32) | b.x);
-      }
-    }
-    g.out[(size_t)limb * n + c] = reduce_128(hi, lo, md);
-  }
-}
-
 // ---- ModDown tail (rns_poly.c:293-304), optionally adding a polynomial -------
 
 __global__ void __launch_bounds__(kThreads)
@@ -559,54 +484,6 @@ void launch_rescale_combine(Ptr2 res, Ptr2 poly, Ptr2 tmp, int l, const LimbBatc
   launch(rescale_combine_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
          res, poly, tmp, c->d_ql_inv + (size_t)l * c->L, batch, c->d_mod, c->N);
   after_launch(c, KID_RESCALE_COMBINE, batch.count);
-}
-
-template <int NIN>
-static void base_conv_dispatch(Context* c, const ConvArgs& args, dim3 grid, int chunk) {
-  if (c->primes_below_2_60)
-    launch(base_conv_kernel<NIN, true>, grid, kThreads, 0, c->stream,
-           args, chunk, c->L, c->d_mod, c->N);
-  else
-    launch(base_conv_kernel<NIN, false>, grid, kThreads, 0, c->stream,
-           args, chunk, c->L, c->d_mod, c->N);
-}
-
-void launch_base_conv(const ConvArgs& args) {
-  Context* c = ctx();
-  int max_in = 0, max_out = 0, total_out = 0;
-  for (int g = 0; g < args.groups; g++) {
-    max_in  = std::max(max_in, args.g[g].count);
-    max_out = std::max(max_out, args.out_total - args.g[g].skip_len);
-    total_out += args.out_total - args.g[g].skip_len;
-  }
-  if (max_out <= 0 || args.groups == 0) return;
-  FHERT_ASSERT(max_in <= kMaxDigit, "base conversion from %d limbs unsupported", max_in);
-  int  chunks = (max_out + kMaxOutChunk - 1) / kMaxOutChunk;
-  int  chunk  = (max_out + chunks - 1) / chunks;
-  dim3 grid((c->N + kThreads - 1) / kThreads, chunks, args.groups);
-  DagScope dag(DAG_BASE_CONV);
-  if (dag.live) {
-    const size_t w = (size_t)c->N * sizeof(u64);
-    for (int g = 0; g < args.groups; g++) {
-      const ConvGroup& cg = args.g[g];
-      dag.set.read(cg.in + (size_t)cg.first_limb * c->N, (size_t)cg.count * w);
-      for (int m = 0; m < args.out_total; m++) {
-        if (m >= cg.skip_start && m < cg.skip_start + cg.skip_len) continue;
-        if ((args.skip_mask >> m) & 1) continue;
-        int limb = m < args.level ? m : args.p_limb + (m - args.level);
-        dag.set.write(cg.out + (size_t)limb * c->N, w);
-      }
-    }
-  }
-  dag.commit();
-  prof_before(KID_BASE_CONV);
-  if (max_in <= 2) base_conv_dispatch<2>(c, args, grid, chunk);
-  else if (max_in <= 4) base_conv_dispatch<4>(c, args, grid, chunk);
-  else if (max_in <= 6) base_conv_dispatch<6>(c, args, grid, chunk);
-  else if (max_in <= 8) base_conv_dispatch<8>(c, args, grid, chunk);
-  else if (max_in <= 12) base_conv_dispatch<12>(c, args, grid, chunk);
-  else base_conv_dispatch<16>(c, args, grid, chunk);
-  after_launch(c, KID_BASE_CONV, total_out);
 }
 
 void launch_moddown_combine(const ModDownTail& args) {

@@ -114,9 +114,9 @@ struct Context {
   u64*     d_ql_mod = nullptr;
 
   // ModDown constants (crt.c:357-414): phat_inv[k] = (P/p_k)^-1 mod p_k,
-  // phat_mod_q[i*K+k] = (P/p_k) mod q_i, p_inv[i] = P^-1 mod q_i
-  Twiddle* d_phat_inv   = nullptr;
-  u64*     d_phat_mod_q = nullptr;
+  // planes of (P/p_k) mod q_i for all Q primes i (conv_planes), p_inv[i] = P^-1 mod q_i
+  Twiddle* d_phat_inv    = nullptr;
+  uint8_t* d_phat_planes = nullptr;
   Twiddle* d_p_inv      = nullptr;
   // Extend: P mod q_i
   Twiddle* d_p_mod_q = nullptr;
@@ -126,7 +126,8 @@ struct Context {
     int  digit_len = 0;          // limbs of the digit present at this level
     int  out_count = 0;          // complement limbs (other Q limbs + P)
     Twiddle* d_hat_inv = nullptr;  // [digit_len] (Qhat_j,i)^-1 mod q_i
-    u64* d_hat_mod = nullptr;    // [digit_len][L+K] indexed by prime
+    int  width     = 0;            // digit_len as the conversion kernel pads it
+    uint8_t* d_planes = nullptr;   // (Qhat_j,i mod p_m) for every complement limb m (conv_planes)
   };
   std::map<std::pair<int, int>, ModUpTable> modup;
 
@@ -180,6 +181,8 @@ struct Context {
 
   cudaStream_t stream = nullptr;
   uint64_t     launches = 0;
+  uint32_t*    h_error = nullptr;  // mapped host word: a bounded wait in a kernel ran out
+  uint32_t*    d_error = nullptr;
   // scratch polynomial storage reused by the fused operations
   int64_t* scratch      = nullptr;
   size_t   scratch_words = 0;
@@ -354,7 +357,11 @@ void image_replay_release();  // drops a captured run (context teardown)
 inline cudaError_t stream_sync(cudaStream_t stream) {
   if (image_capturing()) image_capture_break("a synchronisation");
   launch_flush();
-  return cudaStreamSynchronize(stream);
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  Context*          c = ctx_or_null();
+  FHERT_ASSERT(c == nullptr || c->h_error == nullptr || *(volatile uint32_t*)c->h_error == 0,
+               "a kernel gave up waiting for its own tensor-core product");
+  return e;
 }
 
 // ---- encode_gpu.cu ----
@@ -483,25 +490,30 @@ void launch_rescale_combine(Ptr2 res, Ptr2 poly, Ptr2 tmp, int l, const LimbBatc
 // Approximate base conversion (rns_poly.c:218-242, rns_poly_impl.c:287-339) of
 // up to kMaxParts independent groups in one launch:
 //   y_i = in[first_limb+i] * inv[i] mod p(first_prime+i)
-//   out[limb(m)] = (sum_i y_i * mat[i*in_stride + prime(m)*out_stride]) mod prime(m)
+//   out[limb(m)] = (sum_i y_i * mat[m][i]) mod prime(m)
 // for every m in [0, out_total) outside [skip_start, skip_start+skip_len), where
 // prime(m) = m < level ? m : L + m - level and limb(m) = m < level ? m : p_limb + m - level.
 constexpr int kMaxParts = 16;
+constexpr int kMaxOuts  = 96;  // outputs of one group
 struct ConvGroup {
   const u64*     in;
   u64*           out;
   const Twiddle* inv;
-  const u64*     mat;
+  const uint8_t* planes;  // conv_planes of the group's outputs, skip range left out
   int            first_limb, first_prime, count;
   int            skip_start, skip_len;
 };
 struct ConvArgs {
-  int       groups, level, out_total, p_limb, in_stride, out_stride;
+  int       groups, level, out_total, p_limb;
+  int       width;  // input limbs as padded by conv_planes, the same in all groups
   // bit m set: output m (index before the skip range is removed: Q limbs then
   // special limbs) is not computed -- it belongs to another GPU
   uint64_t  skip_mask = 0;
   ConvGroup g[kMaxParts];
 };
+// Bytes of the constants of a conversion from `inputs` limbs, mat[o * inputs + i],
+// as the matrix operand of the kernel (base_conv.cu); width: a multiple of four
+std::vector<uint8_t> conv_planes(int inputs, int width, int outputs, const u64* mat, const u64* primes);
 void launch_base_conv(const ConvArgs& args);
 
 // ModDown tail for up to two polynomials:

@@ -126,8 +126,6 @@ void Fhert_shard_mid(void* state, const int64_t* c1, const int64_t* gather_q, in
   args.level      = level;
   args.out_total  = level + K;
   args.p_limb     = level;
-  args.in_stride  = c->L + K;
-  args.out_stride = 1;
   args.skip_mask  = foreign;
   std::vector<LimbRef> raised;
   for (int part = 0; part < s->parts; part++) {
@@ -137,7 +135,8 @@ void Fhert_shard_mid(void* state, const int64_t* c1, const int64_t* gather_q, in
     cg.in          = reinterpret_cast<const u64*>(gather_q);
     cg.out         = reinterpret_cast<u64*>(s->ext + (size_t)part * ext * n);
     cg.inv         = t.d_hat_inv;
-    cg.mat         = t.d_hat_mod;
+    args.width     = t.width;
+    cg.planes      = t.d_planes;
     cg.first_limb  = start;
     cg.first_prime = start;
     cg.count       = t.digit_len;
@@ -206,15 +205,14 @@ void Fhert_shard_end2(void* state, const int64_t* add0, const int64_t* add1,
   args.level      = level;
   args.out_total  = level;
   args.p_limb     = 0;
-  args.in_stride  = 1;
-  args.out_stride = K;
   args.skip_mask  = foreign_q;
   for (int g = 0; g < 2; g++) {
+    args.width = (K + 3) & ~3;
     ConvGroup& cg  = args.g[g];
     cg.in          = reinterpret_cast<const u64*>(g ? gather_p1 : gather_p0);
     cg.out         = reinterpret_cast<u64*>(s->conv + (size_t)g * level * n);
     cg.inv         = c->d_phat_inv;
-    cg.mat         = c->d_phat_mod_q;
+    cg.planes      = c->d_phat_planes;
     cg.first_limb  = 0;
     cg.first_prime = c->L;
     cg.count       = K;

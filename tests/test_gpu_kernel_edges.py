@@ -46,3 +46,33 @@ def test_transforms_match_the_oracle(degree, bits):
         gpu.free(p)
     gpu.close()
     orc.close()
+
+
+# digits of 1 to 16 limbs (padded to 4, 8, 12, 16), a short last digit, output
+# counts on both sides of 16 and 32, rings shorter than a tile of coefficients,
+# primes of 30, 46, 48, 56 and 60 bits in and out
+@pytest.mark.parametrize("degree,primes,bits,dnum", [
+    (64, 5, (33, 30), 3), (256, 3, (60, 56), 3), (512, 9, (51, 46), 2), (1024, 17, (50, 48), 3),
+    (2048, 16, (60, 60), 1), (4096, 24, (60, 56), 3), (8192, 36, (51, 46), 3), (1024, 47, (51, 46), 3)])
+def test_base_conversions_match_the_oracle(degree, primes, bits, dnum):
+    import ace_compiler_b200 as rt
+    gpu = rt.Runtime(degree, primes, *bits, dnum)
+    orc = oracle_lib.Oracle(degree, primes, *bits, dnum)
+    assert gpu.primes == orc.primes and gpu.K == orc.K
+    rng = np.random.default_rng(primes)
+    special = gpu.primes[gpu.L:]
+    for level in sorted({1, gpu.alpha, min(gpu.alpha + 1, primes), primes - 1, primes} - {0}):
+        data = edge_limbs(rng, gpu.primes[:level], degree)
+        src, ext = gpu.new_poly(level, data=data), gpu.new_poly(level, extended=True)
+        for part in range(-(-level // gpu.alpha)):
+            gpu.lib.Decomp_modup(ext, src, part)
+            assert np.array_equal(gpu.download(ext), orc.decomp_modup(data, part)), (level, part)
+        data = edge_limbs(rng, gpu.primes[:level] + special, degree)
+        gpu.upload(ext, data)
+        down = gpu.new_poly(level)
+        gpu.lib.Mod_down(down, ext)
+        assert np.array_equal(gpu.download(down), orc.mod_down(data, level)), level
+        for p in (src, ext, down):
+            gpu.free(p)
+    gpu.close()
+    orc.close()
