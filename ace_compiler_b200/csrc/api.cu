@@ -618,12 +618,13 @@ POLY Decomp(POLY res, POLY poly, uint32_t part) {
   return res;
 }
 
-static void fhert_launch_ntt_chunked(Ptr2 in, Ptr2 out, const std::vector<LimbRef>& limbs, bool inverse) {
+static void fhert_launch_ntt_chunked(Ptr2 in, Ptr2 out, const std::vector<LimbRef>& limbs, bool inverse,
+                                     const Twiddle* last = nullptr) {
   for (size_t off = 0; off < limbs.size(); off += kMaxLimbs) {
     LimbBatch b;
     b.count = (int)std::min((size_t)kMaxLimbs, limbs.size() - off);
     std::copy(limbs.begin() + off, limbs.begin() + off + b.count, b.limb);
-    launch_ntt(in, out, b, inverse);
+    launch_ntt(in, out, b, inverse, last);
   }
 }
 
@@ -647,7 +648,8 @@ void fhert_raise_parts(Context* c, const int64_t* src, bool is_ntt, size_t level
     std::vector<LimbRef> lim;
     for (int i = first; i < last; i++)
       lim.push_back(LimbRef{(uint16_t)i, 0, (uint16_t)i, (uint8_t)i, 0});
-    fhert_launch_ntt_chunked(ptr2(src), ptr2(d), lim, true);
+    // the first factor of the conversion comes with the last inverse stage
+    fhert_launch_ntt_chunked(ptr2(src), ptr2(d), lim, true, modup_last(c, (int)level));
     coeff = d;
   }
   std::vector<LimbRef> out_limbs;
@@ -664,7 +666,7 @@ void fhert_raise_parts(Context* c, const int64_t* src, bool is_ntt, size_t level
       ConvGroup&                 cg    = args.g[g];
       cg.in          = reinterpret_cast<const u64*>(coeff);
       cg.out         = reinterpret_cast<u64*>(ext_base + (size_t)(part - part_begin) * part_stride * n);
-      cg.inv         = t.d_hat_inv;
+      cg.inv         = is_ntt ? nullptr : t.d_hat_inv;
       args.width     = t.width;
       cg.planes      = t.d_planes;
       cg.first_limb  = start;
@@ -783,7 +785,7 @@ void fhert_mod_down_polys(Context* c, int npoly, int64_t* const res[2],
       for (int k = 0; k < K; k++)
         in.limb[g * K + k] = LimbRef{(uint16_t)(ext_p_limb + k), 0, (uint16_t)(g * K + k),
                                      (uint8_t)(c->L + k), (uint8_t)g};
-    launch_ntt(ptr2(ext[0], ext[1]), ptr2(sc), in, true);
+    launch_ntt(ptr2(ext[0], ext[1]), ptr2(sc), in, true, c->d_moddown_last);
   }
   ConvArgs args;
   args.groups     = npoly;
@@ -796,7 +798,7 @@ void fhert_mod_down_polys(Context* c, int npoly, int64_t* const res[2],
     cg.in          = is_ntt ? reinterpret_cast<const u64*>(sc + (size_t)g * K * n)
                             : reinterpret_cast<const u64*>(ext[g] + (size_t)ext_p_limb * n);
     cg.out         = reinterpret_cast<u64*>(conv + (size_t)g * level * n);
-    cg.inv         = c->d_phat_inv;
+    cg.inv         = is_ntt ? nullptr : c->d_phat_inv;
     cg.planes      = c->d_phat_planes;
     cg.first_limb  = 0;
     cg.first_prime = c->L;

@@ -1,6 +1,7 @@
 // Approximate base conversion of ModUp and ModDown on the tensor cores
 // (rns_poly.c:218-242, rns_poly_impl.c:287-339 of the CPU runtime):
-//   y_i      = in_i * inv_i mod p_i            (canonical residues, up to 16 limbs)
+//   y_i      = in_i * inv_i mod p_i            (canonical residues, up to 16 limbs;
+//              no inv: the inverse transform before has multiplied already)
 //   out_m    = (sum_i y_i * mat_{i,m}) mod q_m  for up to 60 output primes m.
 //
 // Written with the bytes of y_i the sum is
@@ -37,8 +38,8 @@ using nttk::csub;
 
 constexpr int kThreads = 256;
 constexpr int kRows    = 128;  // coefficients per matrix product
-constexpr int kOuts    = 16;   // outputs per product: 128 columns
-constexpr int kColumns = 256;  // tensor memory of a CTA: two row tiles
+constexpr int kOuts    = 8;    // outputs per product: 64 columns
+constexpr int kColumns = 128;  // tensor memory of a CTA: two row tiles
 // 2 us a poll: a wait that lasts longer than any product by orders of magnitude
 constexpr uint32_t kMaxPolls = 1u << 15;
 
@@ -96,20 +97,22 @@ __device__ __forceinline__ void tmem_load32(uint32_t (&v)[32], uint32_t addr) {
 }
 
 struct OutConst {  // one output of the group
-  u64      q;
-  u64*     dst;  // its limb; nullptr = computed elsewhere
-  uint32_t mu, shift, wide, pad;
+  u64      q, nq;   // modulus, 2^64 - q
+  u64*     dst;     // its limb; nullptr = computed elsewhere (or padding)
+  uint32_t mu, shift;
 };
 
-// sum_s 2^{8s} D_s mod q.  V < 2^{8S+15} for S planes; the quotient is estimated
-// from the 32 bits of V above `shift` = 8S - 16 and mu = floor(2^{32+shift} / q):
-// it is at most 1.51 too small, one subtraction is left.
+// (sum_s 2^{8s} D_s) mod q.  V < 2^{8S+15} for S planes; the quotient is estimated
+// from the 32 bits of V above shift = 8S - 16 and mu = floor(2^{32+shift} / q): it
+// is at most 1.51 too small, one subtraction is left.  WIDE: seven or eight planes.
+template <bool WIDE>
 __device__ __forceinline__ u64 reduce_planes(const uint32_t* d, const OutConst& c) {
   const uint32_t u0 = d[0] + (d[1] << 8), u1 = d[2] + (d[3] << 8), u2 = d[4] + (d[5] << 8);
   u64            a;
   asm("mad.wide.u32 %0, %1, 65536, %2;" : "=l"(a) : "r"(u1), "l"((u64)u0));
-  uint32_t w0 = (uint32_t)a, w1, top;
-  if (c.wide) {
+  const uint32_t w0 = (uint32_t)a;
+  uint32_t       w1, top;
+  if (WIDE) {
     const uint32_t u3 = d[6] + (d[7] << 8);
     u64            b;
     asm("mad.wide.u32 %0, %1, 65536, %2;" : "=l"(b) : "r"(u3), "l"((u64)u2));
@@ -121,23 +124,34 @@ __device__ __forceinline__ u64 reduce_planes(const uint32_t* d, const OutConst& 
     top = __funnelshift_rc(w0, w1, c.shift);
   }
   const uint32_t k = __umulhi(top, c.mu);
-  const u64      nq = 0 - c.q;
   u64            r;
-  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(k), "r"((uint32_t)nq), "l"(((u64)w1 << 32) | w0));
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(k), "r"((uint32_t)c.nq), "l"(((u64)w1 << 32) | w0));
   uint32_t rh = (uint32_t)(r >> 32);
-  asm("mad.lo.u32 %0, %1, %2, %0;" : "+r"(rh) : "r"(k), "r"((uint32_t)(nq >> 32)));
-  return csub(((u64)rh << 32) | (uint32_t)r, c.q);
+  asm("mad.lo.u32 %0, %1, %2, %0;" : "+r"(rh) : "r"(k), "r"((uint32_t)(c.nq >> 32)));
+  r                 = ((u64)rh << 32) | (uint32_t)r;
+  const long long t = (long long)(r - c.q);  // r < 2q < 2^63
+  return t < 0 ? r : (u64)t;
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void finish4(const uint32_t (&d)[32], const OutConst* c, uint32_t coeff,
+                                        bool live) {
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const u64 r = reduce_planes<WIDE>(d + 8 * j, c[j]);
+    if (c[j].dst != nullptr && live) c[j].dst[coeff] = r;
+  }
 }
 
 // NIN: input limbs rounded up to a multiple of four (32 K bytes per product step)
 template <int NIN>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 4)
 base_conv_kernel(const __grid_constant__ ConvArgs args, int num_q, const DevModulus* __restrict__ mods,
                  uint32_t n, uint32_t* error) {
   constexpr int kBytes = NIN * 8;        // K bytes per row
   constexpr int kGroup = kBytes * 8;     // bytes of 8 rows: one output's planes, 8 coefficients
   extern __shared__ __align__(128) unsigned char dyn[];
-  __shared__ OutConst  outs[kMaxOuts];
+  __shared__ OutConst  outs[kMaxOuts + 4];
   __shared__ __align__(8) u64 bars[2];
   __shared__ uint32_t  tmem_slot, failed;
 
@@ -169,17 +183,19 @@ base_conv_kernel(const __grid_constant__ ConvArgs args, int num_q, const DevModu
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  for (int o = threadIdx.x; o < out_count; o += kThreads) {
-    const int  m    = o < g.skip_start ? o : o + g.skip_len;
+  for (int o = threadIdx.x; o < ((out_count + 3) & ~3); o += kThreads) {
+    const bool real = o < out_count;  // padding looks like the last output
+    const int  at   = real ? o : out_count - 1;
+    const int  m    = at < g.skip_start ? at : at + g.skip_len;
     const bool is_q = m < args.level;
     const DevModulus& md = mods[is_q ? m : num_q + (m - args.level)];
     const int  limb = is_q ? m : args.p_limb + (m - args.level);
     OutConst   c;
     c.q     = md.q;
+    c.nq    = 0 - md.q;
     c.mu    = md.conv_mu;
     c.shift = md.conv_shift;
-    c.wide  = md.conv_shift > 32;
-    c.dst   = m < 64 && ((args.skip_mask >> m) & 1) ? nullptr : g.out + (size_t)limb * n;
+    c.dst   = !real || (m < 64 && ((args.skip_mask >> m) & 1)) ? nullptr : g.out + (size_t)limb * n;
     outs[o] = c;
   }
 
@@ -190,9 +206,10 @@ base_conv_kernel(const __grid_constant__ ConvArgs args, int num_q, const DevModu
 #pragma unroll
   for (int i = 0; i < NIN; i++)
     y[i] = live && i < g.count ? g.in[(size_t)(g.first_limb + i) * n + coeff] : 0;
+  if (g.inv != nullptr) {
 #pragma unroll
-  for (int i = 0; i < NIN; i++) {
-    if (i < g.count) {
+    for (int i = 0; i < NIN; i++) {
+      if (i >= g.count) break;
       const nttk::Mod m = nttk::make_mod(mods[g.first_prime + i].q);
       y[i] = nttk::canon_4q(nttk::shoup4(y[i], nttk::ld_tw(g.inv + i), m), m);
     }
@@ -231,12 +248,19 @@ base_conv_kernel(const __grid_constant__ ConvArgs args, int num_q, const DevModu
     for (int o = 0; o < here; o += 4) {
       uint32_t d[32];
       tmem_load32(d, at + o * 8);
+      const OutConst* c = outs + o0 + o;
+      // outputs of one group are alike but for a prime or two
+      const uint32_t widest = max(max(c[0].shift, c[1].shift), max(c[2].shift, c[3].shift));
+      if (widest <= 32) {
+        finish4<false>(d, c, coeff, live);
+      } else if (min(min(c[0].shift, c[1].shift), min(c[2].shift, c[3].shift)) > 32) {
+        finish4<true>(d, c, coeff, live);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        if (o + j >= here) break;
-        const OutConst& c = outs[o0 + o + j];
-        const u64       r = reduce_planes(d + 8 * j, c);
-        if (c.dst != nullptr && live) c.dst[coeff] = r;
+        for (int j = 0; j < 4; j++) {
+          const u64 r = c[j].shift > 32 ? reduce_planes<true>(d + 8 * j, c[j]) : reduce_planes<false>(d + 8 * j, c[j]);
+          if (c[j].dst != nullptr && live) c[j].dst[coeff] = r;
+        }
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

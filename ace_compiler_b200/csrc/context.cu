@@ -402,6 +402,7 @@ const Context::ModUpTable& modup_table(Context* c, int level, int digit) {
       if (k != start + i) hat = mulmod(hat, c->primes[k] % qi, qi);
     u64 inv            = invmod(hat, qi);
     hat_inv[i]         = tw_of(inv, qi);
+    t.hat_inv.push_back(inv);
     for (int o = 0; o < t.out_count; o++) {
       u64 pm = out_primes[o];
       u64 h  = 1;
@@ -413,6 +414,24 @@ const Context::ModUpTable& modup_table(Context* c, int level, int digit) {
   t.d_hat_inv = upload(hat_inv);
   t.d_planes  = upload(conv_planes(t.digit_len, t.width, t.out_count, hat_mod.data(), out_primes.data()));
   return c->modup.emplace(key, t).first->second;
+}
+
+static void last_stage(Twiddle out[2], u64 n_inv, u64 root, u64 factor, u64 q) {
+  const u64 f = mulmod(n_inv, factor, q);
+  out[0]      = tw_of(f, q);
+  out[1]      = tw_of(mulmod(root, f, q), q);
+}
+
+const Twiddle* modup_last(Context* c, int level) {
+  auto it = c->modup_last.find(level);
+  if (it != c->modup_last.end()) return it->second;
+  std::vector<Twiddle> last(2 * (size_t)level);
+  for (int i = 0; i < level; i++) {
+    const u64 q = c->primes[i];
+    last_stage(&last[2 * i], invmod(c->N % q, q), c->h_inv[i][1].w,
+               modup_table(c, level, i / c->alpha).hat_inv[i % c->alpha], q);
+  }
+  return c->modup_last[level] = upload(last);
 }
 
 // ---- automorphism tables  (util/src/number_theory.c:206-230, NTT form) ------
@@ -616,11 +635,13 @@ Context* create_context(const CKKS_PARAMS* p) {
   // ModDown / Extend constants (crt.c:357-414)
   std::vector<Twiddle> phat_inv(K), p_inv(L), p_mod_q(L);
   std::vector<u64>     phat_mod_q((size_t)L * K);
+  std::vector<Twiddle> moddown_last(2 * (size_t)total);
   for (int k = 0; k < K; k++) {
     u64 pk = pp[k], hat = 1;
     for (int j = 0; j < K; j++)
       if (j != k) hat = mulmod(hat, pp[j] % pk, pk);
     phat_inv[k] = tw_of(invmod(hat, pk), pk);
+    last_stage(&moddown_last[2 * (L + k)], dm[L + k].n_inv, c->h_inv[L + k][1].w, phat_inv[k].w, pk);
   }
   for (int i = 0; i < L; i++) {
     u64 qi = q[i], P = 1;
@@ -636,6 +657,7 @@ Context* create_context(const CKKS_PARAMS* p) {
   }
   c->d_phat_inv   = upload(phat_inv);
   c->d_phat_planes = upload(conv_planes(K, (K + 3) & ~3, L, phat_mod_q.data(), c->primes.data()));
+  c->d_moddown_last = upload(moddown_last);
   c->d_p_inv      = upload(p_inv);
   c->d_p_mod_q    = upload(p_mod_q);
 
@@ -670,6 +692,8 @@ void destroy_context() {
   cudaFree(c->d_ql_mod);
   cudaFree(c->d_phat_inv);
   cudaFree(c->d_phat_planes);
+  cudaFree(c->d_moddown_last);
+  for (auto& kv : c->modup_last) cudaFree(kv.second);
   cudaFreeHost(c->h_error);
   cudaFree(c->d_p_inv);
   cudaFree(c->d_p_mod_q);

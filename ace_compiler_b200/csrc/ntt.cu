@@ -17,10 +17,10 @@ int integers_first(Context* c, LimbBatch& b) {
 }
 
 template <bool INV>
-void launch_dir(Ptr2 in, Ptr2 out, const LimbBatch& unsorted) {
+void launch_dir(Ptr2 in, Ptr2 out, const LimbBatch& unsorted, const Twiddle* last) {
   Context*        c = ctx();
   LimbBatch       b = unsorted;
-  nttk::NttTables t{c->d_fwd, c->d_inv, c->d_inv_last, c->d_mod, c->N, (int)c->logN};
+  nttk::NttTables t{c->d_fwd, c->d_inv, last ? last : c->d_inv_last, c->d_mod, c->N, (int)c->logN};
   if (t.logn <= nttk::kWholeMaxLog) {  // one launch
     DagScope dag(DAG_NTT);
     dag.batch(b, c->N, &out, &in, nullptr);
@@ -122,12 +122,12 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
   CUDA_CHECK(cudaGetLastError());
 }
 
-void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse) {
+void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse, const Twiddle* last) {
   if (b.count == 0) return;
   if (inverse)
-    launch_dir<true>(in, out, b);
+    launch_dir<true>(in, out, b, last);
   else
-    launch_dir<false>(in, out, b);
+    launch_dir<false>(in, out, b, nullptr);
 }
 
 }  // namespace fhert

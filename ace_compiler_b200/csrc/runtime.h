@@ -125,11 +125,17 @@ struct Context {
   struct ModUpTable {
     int  digit_len = 0;          // limbs of the digit present at this level
     int  out_count = 0;          // complement limbs (other Q limbs + P)
-    Twiddle* d_hat_inv = nullptr;  // [digit_len] (Qhat_j,i)^-1 mod q_i
+    std::vector<u64> hat_inv;      // [digit_len] (Qhat_j,i)^-1 mod q_i
+    Twiddle* d_hat_inv = nullptr;
     int  width     = 0;            // digit_len as the conversion kernel pads it
     uint8_t* d_planes = nullptr;   // (Qhat_j,i mod p_m) for every complement limb m (conv_planes)
   };
   std::map<std::pair<int, int>, ModUpTable> modup;
+  // last inverse stages with a base conversion's first factor folded in, like
+  // d_inv_last: per level, (Qhat_j,i)^-1 of the digit that limb i belongs to, and
+  // for ModDown (P/p_k)^-1 (special primes only)
+  std::map<int, Twiddle*> modup_last;
+  Twiddle*                d_moddown_last = nullptr;
 
   // automorphism index tables by automorphism index k (NTT order)
   std::map<uint32_t, uint32_t*> auto_tables;
@@ -226,6 +232,7 @@ u64  invmod(u64 a, u64 q);
 bool is_prime(u64 n);
 u64  shoup(u64 w, u64 q);
 const Context::ModUpTable& modup_table(Context* c, int level, int digit);
+const Twiddle* modup_last(Context* c, int level);
 uint32_t* auto_table(Context* c, uint32_t k);
 
 // ---- sampling.cu (host randomness, same generators as the CPU runtime) ----
@@ -431,7 +438,8 @@ DevModulus make_dev_modulus(u64 q, uint32_t n);
 // ---- kernels (launch wrappers; all queue on ctx()->stream) ----
 // limb.a selects the source limb of in.p[sel&1], limb.dst the result limb of
 // out.p[(sel>>2)&1]
-void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse);
+// (last: constants of the last inverse stage in place of d_inv_last)
+void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse, const Twiddle* last = nullptr);
 // Forward transform with the element-wise passes around it folded in (ring
 // degrees of 512 and more: ntt_can_fuse).  The first pass reads in[a] and
 // writes limb k of `mid` (k = position in the batch), the last pass reads
@@ -489,7 +497,7 @@ void launch_rescale_combine(Ptr2 res, Ptr2 poly, Ptr2 tmp, int l, const LimbBatc
 
 // Approximate base conversion (rns_poly.c:218-242, rns_poly_impl.c:287-339) of
 // up to kMaxParts independent groups in one launch:
-//   y_i = in[first_limb+i] * inv[i] mod p(first_prime+i)
+//   y_i = in[first_limb+i] * inv[i] mod p(first_prime+i)    (inv null: in holds y_i)
 //   out[limb(m)] = (sum_i y_i * mat[m][i]) mod prime(m)
 // for every m in [0, out_total) outside [skip_start, skip_start+skip_len), where
 // prime(m) = m < level ? m : L + m - level and limb(m) = m < level ? m : p_limb + m - level.
