@@ -500,6 +500,7 @@ void fhert_rescale_polys(Context* c, int npoly, int64_t* const res[2],
         bt.limb[g * l + i] = LimbRef{(uint16_t)g, (uint16_t)i, (uint16_t)i, (uint8_t)i, sel};
       }
     NttFuse f;
+    f.pro_kind = 1;
     f.pro_mul  = c->d_ql_neg + (size_t)l * c->L;
     f.pro_mod  = c->d_ql_mod + (size_t)l * c->L;
     f.q_last   = c->primes[l];

@@ -265,7 +265,8 @@ std::vector<std::vector<PLAINTEXT>> encode_stages(Context* c, Stages& coeffs, co
     size_t len = diag.size();
     Row    turned(len);
     for (size_t k = 0; k < len; k++) turned[k] = diag[(k + rot) % len];
-    encode_vector(c, dst, turned, 1, plain_level, (uint32_t)len, (uint32_t)c->K);
+    encode_vector(c, dst, MessageInput{MessageInput::kComplex, turned.data(), len}, 1, plain_level,
+                  (uint32_t)len, (uint32_t)c->K);
   };
 
   for (int s = start; s < end; s++) {

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <vector>
 
+#include "ntt_kernels.cuh"
 #include "runtime.h"
 
 namespace fhert {
@@ -19,28 +20,48 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// include/util/modular.h:278-280
-constexpr int64_t kMax64 = (int64_t)(((u64)1 << 63) - ((u64)1 << 9)) - 1;
+// only for rings too small for a transform with a fused first step
+__global__ void __launch_bounds__(kThreads)
+encode_split_kernel(u64* __restrict__ poly, const u64* __restrict__ msg, const Twiddle* __restrict__ pow,
+                    LimbBatch batch, const DevModulus* __restrict__ mods, uint32_t n) {
+  const LimbRef    lr = batch.limb[blockIdx.y];
+  const DevModulus d  = mods[lr.prime];
+  const nttk::Mod  m  = nttk::make_mod(d.q);
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+    u64 r = nttk::message_residue(msg[(size_t)lr.a * n + i], m, d.mu_hi);
+    if (pow != nullptr) r = mul_shoup(r, pow[lr.prime].w, pow[lr.prime].wp, d.q);
+    poly[(size_t)lr.dst * n + i] = r;
+  }
+}
+
+// two coefficients per thread; noise holds u, e1 and e2, `level` limbs each
+__global__ void __launch_bounds__(kThreads)
+encrypt_kernel(ulonglong2* __restrict__ c0, ulonglong2* __restrict__ c1,
+               const ulonglong2* __restrict__ noise, const ulonglong2* __restrict__ msg,
+               const ulonglong2* __restrict__ pk0, const ulonglong2* __restrict__ pk1,
+               const DevModulus* __restrict__ mods, uint32_t pairs) {
+  const uint32_t k = blockIdx.x * kThreads + threadIdx.x;
+  if (k >= pairs) return;
+  const DevModulus m   = mods[blockIdx.y];
+  const size_t     i   = (size_t)blockIdx.y * pairs + k, one = (size_t)gridDim.y * pairs;
+  const ulonglong2 u = noise[i], e1 = noise[one + i], e2 = noise[2 * one + i];
+  const ulonglong2 a = pk0[i], b = pk1[i], p = msg[i];
+  c0[i] = make_ulonglong2(add_mod(add_mod(mul_mod(a.x, u.x, m), e1.x, m.q), p.x, m.q),
+                          add_mod(add_mod(mul_mod(a.y, u.y, m), e1.y, m.q), p.y, m.q));
+  c1[i] = make_ulonglong2(add_mod(mul_mod(b.x, u.x, m), e2.x, m.q),
+                          add_mod(mul_mod(b.y, u.y, m), e2.y, m.q));
+}
 
 __global__ void __launch_bounds__(kThreads)
-encode_split_kernel(u64* __restrict__ poly, const int64_t* __restrict__ msg,
-                    const u64* __restrict__ scale_pow, LimbBatch batch,
-                    const DevModulus* __restrict__ mods, uint32_t n) {
-  const LimbRef    lr = batch.limb[blockIdx.y];
-  const DevModulus m  = mods[lr.prime];
-  const int64_t    q  = (int64_t)m.q;
-  const u64        sp = scale_pow ? scale_pow[lr.prime] : 1;
-  u64*             pr = poly + (size_t)lr.dst * n;
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-    int64_t v = msg[i];
-    // values above half of the 64-bit bound stand for negatives (crt.c:1161-1184)
-    if (v > (kMax64 >> 1)) v -= kMax64;
-    int64_t r = v % q;
-    if (r < 0) r += q;
-    u64 out = (u64)r;
-    if (scale_pow) out = mul_mod(out, sp, m);
-    pr[i] = out;
-  }
+decrypt_kernel(ulonglong2* __restrict__ res, const ulonglong2* __restrict__ c0,
+               const ulonglong2* __restrict__ c1, const ulonglong2* __restrict__ sk,
+               const DevModulus* __restrict__ mods, uint32_t pairs) {
+  const uint32_t k = blockIdx.x * kThreads + threadIdx.x;
+  if (k >= pairs) return;
+  const DevModulus m = mods[blockIdx.y];
+  const size_t     i = (size_t)blockIdx.y * pairs + k;
+  const ulonglong2 a = c0[i], b = c1[i], s = sk[i];
+  res[i] = make_ulonglong2(add_mod(a.x, mul_mod(b.x, s.x, m), m.q), add_mod(a.y, mul_mod(b.y, s.y, m), m.q));
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -61,11 +82,52 @@ inline dim3 grid_for(uint32_t n, int limbs) {
 
 }  // namespace
 
-void launch_encode_split(int64_t* poly, const int64_t* msg, const u64* scale_pow,
-                         const LimbBatch& batch) {
-  Context* c = ctx();
-  launch(encode_split_kernel, grid_for(c->N, batch.count), kThreads, 0, c->stream,
-         (u64*)poly, msg, scale_pow, batch, c->d_mod, c->N);
+void message_to_ntt(Context* c, int64_t* out, const int64_t* msg, int polys, const Twiddle* pow,
+                    const LimbBatch& one) {
+  const size_t n = c->N;
+  while (polys > 0) {
+    const int here = std::min(polys, std::max(1, kMaxLimbs / one.count));
+    LimbBatch b;
+    b.count = 0;
+    for (int g = 0; g < here; g++)
+      for (int i = 0; i < one.count; i++) {
+        const uint16_t at   = (uint16_t)b.count;
+        b.limb[b.count++] = LimbRef{(uint16_t)g, at, at, one.limb[i].prime, 0};
+      }
+    if (ntt_can_fuse()) {
+      NttFuse f;
+      f.pro_kind = 2;
+      f.pro_mul  = pow;
+      launch_ntt_fused(ptr2(msg), out, ptr2(out), b, f);
+    } else {
+      launch(encode_split_kernel, grid_for(c->N, b.count), kThreads, 0, c->stream, (u64*)out,
+             (const u64*)msg, pow, b, c->d_mod, c->N);
+      c->launches++;
+      for (int i = 0; i < b.count; i++) b.limb[i].a = b.limb[i].dst;
+      launch_ntt(ptr2(out), ptr2(out), b, false);
+    }
+    polys -= here;
+    msg += here * n;
+    out += here * one.count * n;
+  }
+}
+
+void launch_encrypt(Context* c, int64_t* c0, int64_t* c1, const int64_t* noise, const int64_t* m,
+                    size_t level) {
+  typedef ulonglong2 w2;
+  const uint32_t pairs = c->N / 2;
+  launch(encrypt_kernel, dim3((pairs + kThreads - 1) / kThreads, (unsigned)level), kThreads, 0, c->stream,
+         (w2*)c0, (w2*)c1, (const w2*)noise, (const w2*)m, (const w2*)c->pk._p0._data,
+         (const w2*)c->pk._p1._data, c->d_mod, pairs);
+  c->launches++;
+  CUDA_CHECK(cudaGetLastError());
+}
+
+void launch_decrypt(Context* c, int64_t* res, const int64_t* c0, const int64_t* c1, size_t level) {
+  typedef ulonglong2 w2;
+  const uint32_t pairs = c->N / 2;
+  launch(decrypt_kernel, dim3((pairs + kThreads - 1) / kThreads, (unsigned)level), kThreads, 0, c->stream,
+         (w2*)res, (const w2*)c0, (const w2*)c1, (const w2*)c->sk_ntt._data, c->d_mod, pairs);
   c->launches++;
   CUDA_CHECK(cudaGetLastError());
 }

@@ -73,29 +73,6 @@ void embedding_inv(Context* c, std::vector<cplx>& v) {
   for (size_t i = 0; i < len; i++) v[i] = cplx(out[i].real() / d, out[i].imag() / d);
 }
 
-// util/src/ntt.c:598-631
-void embedding(Context* c, std::vector<cplx>& v) {
-  size_t len = v.size(), m = 2ull * c->N;
-  int    lg  = 0;
-  while ((1ull << lg) < len) lg++;
-  std::vector<cplx> res(len);
-  for (size_t i = 0; i < len; i++) res[i] = v[reverse_bits((uint32_t)i, lg)];
-  for (int logm = 1; logm <= lg; logm++) {
-    size_t idx_mod = 1ull << (logm + 2), gap = m / idx_mod, num = 1ull << (logm - 1);
-    for (size_t j = 0; j < len; j += (1ull << logm)) {
-      for (size_t i = 0; i < num; i++) {
-        size_t e = j + i, o = j + i + num;
-        size_t r = (c->fft_rot_group[i] % idx_mod) * gap;
-        cplx   w = cmul(cplx(c->fft_rou_re[r], c->fft_rou_im[r]), res[o]);
-        cplx   plus = res[e] + w, minus = res[e] - w;
-        res[e] = plus;
-        res[o] = minus;
-      }
-    }
-  }
-  v.swap(res);
-}
-
 void init_plain(Context* c, PLAIN plain, size_t level, double scale, uint32_t sf_degree,
                 uint32_t slots = 0, size_t num_p = 0) {
   POLY p = &plain->_poly;
@@ -167,49 +144,28 @@ std::vector<int64_t> encode_value(Context* c, double value, uint32_t level, doub
 
 // ckks/src/encoder.c:234-325; slots = 0 means N/2, num_p = K also fills the
 // special limbs (the plaintexts of the bootstrapping linear transforms)
-void encode_vector(Context* c, PLAIN plain, std::vector<cplx>& values, uint32_t sf_degree,
-                   uint32_t level, uint32_t slots, uint32_t num_p, const float* reals,
-                   size_t real_count) {
-  LaunchScope scope;
-  ensure_fft_tables(c);
+void encode_vector(Context* c, PLAIN plain, const MessageInput& in, uint32_t sf_degree,
+                   uint32_t level, uint32_t slots, uint32_t num_p) {
+  LaunchScope    scope;
   const uint32_t n = c->N;
   if (slots == 0) slots = n / 2;
   FHERT_ASSERT(slots <= n / 2 && (slots & (slots - 1)) == 0, " slot size > N/2 ");
   FHERT_ASSERT(num_p == 0 || num_p == (uint32_t)c->K, "invalid p cnt");
-  const uint32_t gap = n / (slots * 2);
   if (level == 0) level = c->L;
   FHERT_ASSERT(level <= (uint32_t)c->L, "level should not be larger than mul_depth + 1");
-  const size_t count = reals != nullptr ? real_count : values.size();
-  FHERT_ASSERT(count <= slots, "slot size is too small");
+  FHERT_ASSERT(in.count <= slots, "slot size is too small");
   FHERT_ASSERT(sf_degree >= 1, "invalid scaling factor for encode");
   const double delta = std::pow(2.0, (double)c->sf_bits);
   init_plain(c, plain, level, std::pow(delta, (double)sf_degree), sf_degree, slots, num_p);
   int64_t* d_msg = nullptr;
-  u64*     d_pow = nullptr;
   CUDA_CHECK(dev_alloc(&d_msg, n * sizeof(int64_t), c->stream));
   // inverse embedding, scaling and rounding run on the device with the host
-  // routine's arithmetic (encode_gpu.cu)
-  encode_message_on_device(c, values.data(), count, slots, d_msg, reals);
-  std::vector<u64> powp;
-  if (sf_degree > 1) {
-    // Delta^(d-1) modulo every prime (encoder.c:297-312)
-    powp.assign(c->L + c->K, 1);
-    for (uint32_t i = 0; i < level; i++) {
-      u64 q = c->primes[i], p = (u64)(int64_t)delta % q;
-      for (uint32_t d = 2; d < sf_degree; d++) p = mulmod(p, (u64)(int64_t)delta % q, q);
-      powp[i] = p;
-    }
-    CUDA_CHECK(dev_alloc(&d_pow, powp.size() * sizeof(u64), c->stream));
-    CUDA_CHECK(counted_copy(d_pow, powp.data(), powp.size() * sizeof(u64),
-                               cudaMemcpyHostToDevice, c->stream));
-  }
-  launch_encode_split(plain->_poly._data, d_msg, d_pow, q_batch(level, num_p, c->L));
-  // powp lives on the host stack (a captured copy reads its own snapshot instead)
-  if (d_pow && !image_capturing()) CUDA_CHECK(stream_sync(c->stream));
+  // routine's arithmetic (embedding.cu)
+  encode_message_on_device(c, in, slots, d_msg);
+  message_to_ntt(c, plain->_poly._data, d_msg, 1, sf_degree > 1 ? scale_powers(c, sf_degree) : nullptr,
+                 q_batch(level, num_p, c->L));
   CUDA_CHECK(dev_free(d_msg, c->stream));
-  if (d_pow) CUDA_CHECK(dev_free(d_pow, c->stream));
-  plain->_poly._is_ntt = false;
-  Conv_poly2ntt_inplace(&plain->_poly);
+  plain->_poly._is_ntt = true;
 }
 
 }  // namespace fhert
@@ -267,9 +223,7 @@ void Encode_double(PLAIN plain, double* input, size_t len, uint32_t sc_degree, u
     encode_scalar(c, plain, *input, sc_degree, level);
     return;
   }
-  std::vector<cplx> v(len);
-  for (size_t i = 0; i < len; i++) v[i] = cplx(input[i], 0.0);
-  encode_vector(c, plain, v, sc_degree, level);
+  encode_vector(c, plain, MessageInput{MessageInput::kReals, input, len}, sc_degree, level);
 }
 
 void Encode_float(PLAIN plain, float* input, size_t len, uint32_t sc_degree, uint32_t level) {
@@ -278,14 +232,11 @@ void Encode_float(PLAIN plain, float* input, size_t len, uint32_t sc_degree, uin
     encode_scalar(c, plain, (double)*input, sc_degree, level);
     return;
   }
-  std::vector<cplx> none;  // the floats are widened to complex doubles on the device
-  encode_vector(c, plain, none, sc_degree, level, 0, 0, input, len);
+  encode_vector(c, plain, MessageInput{MessageInput::kFloats, input, len}, sc_degree, level);
 }
 
 void Encode_dcmplx(PLAIN plain, double* re_im, size_t len, uint32_t sc_degree, uint32_t level) {
-  std::vector<cplx> v(len);
-  for (size_t i = 0; i < len; i++) v[i] = cplx(re_im[2 * i], re_im[2 * i + 1]);
-  encode_vector(ctx(), plain, v, sc_degree, level);
+  encode_vector(ctx(), plain, MessageInput{MessageInput::kComplex, re_im, len}, sc_degree, level);
 }
 
 void Encode_double_mask(PLAIN plain, double cst, size_t len, uint32_t sc_degree, uint32_t level) {
@@ -303,71 +254,6 @@ void Encode_float_mask(PLAIN plain, float cst, size_t len, uint32_t sc_degree, u
 // ---------------------------------------------------------------------------
 // encrypt / decrypt / decode
 // ---------------------------------------------------------------------------
-
-namespace {
-
-// triangle sample vector as an RNS polynomial (coefficient form) at `level`
-void error_poly(Context* c, POLY e, size_t level) {
-  std::vector<int64_t> tri(c->N);
-  sample_triangle(tri.data(), c->N);
-  int64_t* d = nullptr;
-  CUDA_CHECK(dev_alloc(&d, c->N * sizeof(int64_t), c->stream));
-  CUDA_CHECK(counted_copy(d, tri.data(), c->N * sizeof(int64_t), cudaMemcpyHostToDevice,
-                             c->stream));
-  Alloc_poly_data(e, c->N, level, 0);
-  launch_small_to_rns(e->_data, d, q_batch(level));
-  CUDA_CHECK(stream_sync(c->stream));
-  CUDA_CHECK(dev_free(d, c->stream));
-  e->_is_ntt = false;
-}
-
-// little-endian multiword helpers for the CRT reconstruction of Decode
-typedef std::vector<u64> Big;
-
-void big_mul_add(Big& acc, const Big& a, u64 m) {  // acc += a * m
-  u64 carry = 0;
-  for (size_t i = 0; i < acc.size(); i++) {
-    u128 t = (u128)(i < a.size() ? a[i] : 0) * m + acc[i] + carry;
-    acc[i] = (u64)t;
-    carry  = (u64)(t >> 64);
-  }
-}
-
-int big_cmp(const Big& a, const Big& b) {
-  for (size_t i = a.size(); i-- > 0;) {
-    u64 x = a[i], y = i < b.size() ? b[i] : 0;
-    if (x != y) return x > y ? 1 : -1;
-  }
-  return 0;
-}
-
-void big_sub(Big& a, const Big& b) {  // a -= b, a >= b
-  u64 borrow = 0;
-  for (size_t i = 0; i < a.size(); i++) {
-    u64  y = i < b.size() ? b[i] : 0;
-    u128 t = (u128)a[i] - y - borrow;
-    a[i]   = (u64)t;
-    borrow = (u64)(t >> 64) & 1;
-  }
-}
-
-// magnitude -> double, truncating toward zero (the conversion the CPU runtime
-// gets from its big-integer library, encoder.c:681)
-double big_to_double(const Big& a) {
-  int top = (int)a.size() - 1;
-  while (top >= 0 && a[top] == 0) top--;
-  if (top < 0) return 0.0;
-  int  bits = top * 64 + (64 - __builtin_clzll(a[top]));
-  if (bits <= 53) return (double)a[0];
-  int  shift = bits - 53;  // keep the top 53 bits
-  int  w = shift / 64, b = shift % 64;
-  u64  lo = a[w] >> b;
-  if (b && w + 1 <= top) lo |= a[w + 1] << (64 - b);
-  lo &= (1ull << 53) - 1;
-  return std::ldexp((double)lo, shift);
-}
-
-}  // namespace
 
 extern "C" {
 
@@ -391,20 +277,17 @@ CIPHER Encrypt(CIPHER res, PLAIN plain) {
   res->_scaling_factor = plain->_scaling_factor;
   res->_sf_degree      = plain->_sf_degree;
   res->_slots          = plain->_slots;
-  POLYNOMIAL u{}, e1{}, e2{};
-  error_poly(c, &u, level);
-  error_poly(c, &e1, level);
-  error_poly(c, &e2, level);
-  POLYNOMIAL pk0 = c->pk._p0, pk1 = c->pk._p1;  // views at the ciphertext's level
-  pk0._num_primes = pk1._num_primes = level;
-  Mul_poly(&res->_c0_poly, &pk0, &u);
-  Add_poly(&res->_c0_poly, &e1, &res->_c0_poly);
-  Add_poly(&res->_c0_poly, &res->_c0_poly, m);
-  Mul_poly(&res->_c1_poly, &pk1, &u);
-  Add_poly(&res->_c1_poly, &e2, &res->_c1_poly);
-  Free_poly_data(&u);
-  Free_poly_data(&e1);
-  Free_poly_data(&e2);
+  if (!m->_is_ntt) Conv_poly2ntt_inplace(m);
+  // u, e1, e2: triangle samples (small integers), sampled and transformed together
+  int64_t *small = nullptr, *noise = nullptr;
+  CUDA_CHECK(dev_alloc(&small, 3 * (size_t)c->N * sizeof(int64_t), c->stream));
+  CUDA_CHECK(dev_alloc(&noise, 3 * level * c->N * sizeof(int64_t), c->stream));
+  sample_triangles_on_device(c, small, 3);
+  message_to_ntt(c, noise, small, 3, nullptr, q_batch(level));
+  launch_encrypt(c, res->_c0_poly._data, res->_c1_poly._data, noise, m->_data, level);
+  res->_c0_poly._is_ntt = res->_c1_poly._is_ntt = true;
+  CUDA_CHECK(dev_free(small, c->stream));
+  CUDA_CHECK(dev_free(noise, c->stream));
   return res;
 }
 
@@ -417,11 +300,11 @@ void Fhert_decrypt(PLAIN res, CIPHER ciph) {
   FHERT_ASSERT(ciph->_c0_poly._num_primes_p == 0, "Decrypt: ciph should not be extended");
   init_plain(c, res, level, ciph->_scaling_factor, ciph->_sf_degree);
   res->_slots    = ciph->_slots;
-  POLYNOMIAL sk  = c->sk_ntt, c1 = ciph->_c1_poly, c0 = ciph->_c0_poly;
-  sk._num_primes = c1._num_primes = c0._num_primes = level;
-  sk._num_primes_p = 0;
-  Mul_poly(&res->_poly, &c1, &sk);
-  Add_poly(&res->_poly, &c0, &res->_poly);
+  // a ciphertext in coefficient form is brought to NTT form in place
+  if (!ciph->_c1_poly._is_ntt) Conv_poly2ntt_inplace(&ciph->_c1_poly);
+  if (!ciph->_c0_poly._is_ntt) Conv_poly2ntt_inplace(&ciph->_c0_poly);
+  launch_decrypt(c, res->_poly._data, ciph->_c0_poly._data, ciph->_c1_poly._data, level);
+  res->_poly._is_ntt = true;
 }
 
 // ckks/src/encoder.c:657-704: out receives `count` complex values as
@@ -429,69 +312,12 @@ void Fhert_decrypt(PLAIN res, CIPHER ciph) {
 void Fhert_decode(PLAIN plain, double* out, size_t count) {
   LaunchScope scope;
   Context* c = ctx();
-  ensure_fft_tables(c);
   POLY           poly  = &plain->_poly;
-  const uint32_t n     = c->N, half = n / 2;
-  const size_t   level = poly->_num_primes;
+  const uint32_t half  = c->N / 2;
   const uint32_t slots = plain->_slots ? plain->_slots : half;
-  const uint32_t gap   = half / slots;
   FHERT_ASSERT(count <= slots, "res size larger than decode size");
   if (poly->_is_ntt) Conv_ntt2poly_inplace(poly);
-  std::vector<int64_t> host(level * n);
-  Fhert_download(poly, 0, level, host.data());
-  // Q = prod q_i, Qhat_i = Q / q_i, and (Qhat_i^-1 mod q_i)
-  size_t words = level + 1;
-  Big    big_q(words, 0);
-  big_q[0] = 1;
-  for (size_t i = 0; i < level; i++) {
-    Big t(words, 0);
-    big_mul_add(t, big_q, c->primes[i]);
-    big_q = t;
-  }
-  std::vector<Big> hat(level, Big(words, 0));
-  std::vector<u64> hat_inv(level);
-  for (size_t i = 0; i < level; i++) {
-    hat[i][0] = 1;
-    u64 qi = c->primes[i], h = 1;
-    for (size_t k = 0; k < level; k++) {
-      if (k == i) continue;
-      Big t(words, 0);
-      big_mul_add(t, hat[i], c->primes[k]);
-      hat[i] = t;
-      h      = mulmod(h, c->primes[k] % qi, qi);
-    }
-    hat_inv[i] = invmod(h, qi);
-  }
-  Big half_q = big_q;  // floor(Q / 2)
-  for (size_t i = 0; i < words; i++)
-    half_q[i] = (half_q[i] >> 1) | (i + 1 < words ? half_q[i + 1] << 63 : 0);
-  auto coeff_to_double = [&](uint32_t idx) {
-    Big acc(words + 1, 0);
-    for (size_t i = 0; i < level; i++) {
-      u64 y = mulmod((u64)host[i * n + idx], hat_inv[i], c->primes[i]);
-      big_mul_add(acc, hat[i], y);
-    }
-    while (big_cmp(acc, big_q) >= 0) big_sub(acc, big_q);
-    if (big_cmp(acc, half_q) > 0) {
-      Big neg = big_q;
-      neg.resize(words + 1, 0);
-      big_sub(neg, acc);
-      return -big_to_double(neg);
-    }
-    return big_to_double(acc);
-  };
-  std::vector<cplx> msg(slots);
-  double            factor = plain->_scaling_factor;
-  for (uint32_t i = 0; i < slots; i++) {
-    double re = coeff_to_double(i * gap) / factor;
-    double im = coeff_to_double(i * gap + half) / factor;
-    msg[i]    = cplx(re, im);
-  }
-  embedding(c, msg);
-  for (size_t i = 0; i < count; i++) {
-    out[2 * i]     = msg[i].real();
-    out[2 * i + 1] = msg[i].imag();
-  }
+  decode_on_device(c, poly->_data, (int)poly->_num_primes, slots, plain->_scaling_factor, out, count);
 }
 
 // cipher.c Get_msg: decrypt and decode, real parts; the caller frees the result

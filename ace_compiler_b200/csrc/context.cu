@@ -670,10 +670,11 @@ void destroy_context() {
   if (!c) return;
   image_replay_release();  // its blocks join the common lists, released below
   hw_release(c);
-  free_encode_tables(c);
+  free_embed_tables(c);
   free_bootstrap(c);
   free_keys(c);
   release_prng();
+  cudaFree(c->triangle_jump);
   if (c->scratch) dev_free(c->scratch, c->stream);
   c->scratch = nullptr;
   for (int64_t*& r : c->ring) {
@@ -683,6 +684,7 @@ void destroy_context() {
   dev_release_all(c->stream);
   cudaStreamSynchronize(c->stream);
   launch_release();
+  free_host_buffers(c);
   cudaFree(c->d_mod);
   cudaFree(c->d_fwd);
   cudaFree(c->d_inv);

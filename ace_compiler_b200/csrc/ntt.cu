@@ -73,6 +73,7 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
   nttk::NttTables t{c->d_fwd, c->d_inv, c->d_inv_last, c->d_mod, c->N, (int)c->logN};
   FHERT_ASSERT(t.logn > nttk::kTinyMaxLog, "ring degree too small for a fused transform");
   nttk::NttPro pro;
+  pro.kind   = f.pro_kind;
   pro.mul    = f.pro_mul;
   pro.mod    = f.pro_mod;
   pro.q_last = f.q_last;

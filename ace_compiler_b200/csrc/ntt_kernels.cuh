@@ -135,15 +135,26 @@ __device__ __forceinline__ Twiddle ld_tw(const Twiddle* p) {
 
 // ---- work fused into a forward transform (all optional) ------------------------
 //
-// Prologue of the first pass, the lift of a rescale (rns_poly.c:351-366): the
-// source limb holds residues modulo q_last in coefficient form; the value that
-// enters the transform under prime i is
-//   switch_modulus(v, q_last -> q_i) * mul[i].
+// Prologue of the first pass.
+//   kind 1, the lift of a rescale (rns_poly.c:351-366): the source limb holds
+//     residues modulo q_last in coefficient form; the value that enters the
+//     transform under prime i is switch_modulus(v, q_last -> q_i) * mul[i]
+//   kind 2, a message polynomial (crt.c:1153-1221): signed 64-bit integers,
+//     negatives also as kMax64 + v; their residues, times mul[i] when given
 struct NttPro {
-  const Twiddle* mul = nullptr;  // [prime]; nullptr = no prologue
-  const u64*     mod = nullptr;  // [prime] q_last mod q_i
+  int            kind = 0;
+  const Twiddle* mul  = nullptr;  // [prime]
+  const u64*     mod  = nullptr;  // [prime] q_last mod q_i
   u64            q_last = 0;
 };
+// a message coefficient modulo q; r = floor(2^64 / q)   (modular.h:278-280)
+__device__ __forceinline__ u64 message_residue(u64 v, const Mod m, u64 r) {
+  constexpr long long kMax64 = (long long)((1ull << 63) - (1ull << 9)) - 1;
+  long long s = (long long)v;
+  if (s > (kMax64 >> 1)) s -= kMax64;
+  const u64 t = canon_any(s < 0 ? 0 - (u64)s : (u64)s, m, r);
+  return s < 0 && t != 0 ? m.q - t : t;
+}
 // Epilogue of the last pass on the canonical transform output t:
 //   kind 1 (rescale, rns_poly.c:367-383):  res = aux * mul[i] + t
 //   kind 2 (ModDown, rns_poly.c:293-304):  res = (aux - t) * mul[i] (+ add)
@@ -264,22 +275,22 @@ struct ArithFp {
   // the lift of a rescale; a dropped prime below 2^48 is centred in floating
   // point (its product with w has a quotient below 2^47), a wider one goes through words
   struct Lift {
-    bool   on, narrow;
-    u64    q_last, half, last_mod_q;
+    bool   narrow;
+    u64    half, last_mod_q;
     double w, dq_last;
   };
   __device__ __forceinline__ Lift make_lift(const NttPro& pro, int prime) const {
     Lift l{};
-    l.on = pro.mul != nullptr;
-    if (l.on) {
-      l.q_last     = pro.q_last;
-      l.half       = pro.q_last >> 1;
-      l.narrow     = (pro.q_last >> 48) == 0;
-      l.last_mod_q = pro.mod[prime];
-      l.w          = constant(pro.mul + prime);
-      l.dq_last    = (double)pro.q_last;
-    }
+    l.half       = pro.q_last >> 1;
+    l.narrow     = (pro.q_last >> 48) == 0;
+    l.last_mod_q = pro.mod[prime];
+    l.w          = constant(pro.mul + prime);
+    l.dq_last    = (double)pro.q_last;
     return l;
+  }
+  __device__ __forceinline__ V message(u64 v, bool scaled, T w) const {
+    const V x = load(message_residue(v, make_mod(q), rq));
+    return scaled ? mul(x, w) : x;
   }
   __device__ __forceinline__ V lift(u64 v, const Lift& l) const {
     if (l.narrow) {
@@ -362,19 +373,15 @@ struct ArithInt {
   __device__ __forceinline__ T constant(const Twiddle* c) const { return ld_tw(c); }
 
   struct Lift {
-    bool on;
-    u64  half, last_mod_q;
-    T    w;
+    u64 half, last_mod_q;
+    T   w;
   };
   __device__ __forceinline__ Lift make_lift(const NttPro& pro, int prime) const {
-    Lift l{};
-    l.on = pro.mul != nullptr;
-    if (l.on) {
-      l.half       = pro.q_last >> 1;
-      l.last_mod_q = pro.mod[prime];
-      l.w          = constant(pro.mul + prime);
-    }
-    return l;
+    return Lift{pro.q_last >> 1, pro.mod[prime], constant(pro.mul + prime)};
+  }
+  __device__ __forceinline__ V message(u64 v, bool scaled, const T w) const {
+    const u64 r = message_residue(v, m, rq);
+    return scaled ? canon_4q(shoup4(r, w, m), m) : r;
   }
   __device__ __forceinline__ V lift(u64 v, const Lift& l) const {
     u64 r = canon_any(v, m, rq);
@@ -764,10 +771,15 @@ __device__ __forceinline__ void strided_inv(typename A::V (&x)[1 << E], u64* sm,
 template <class A, int E>
 __device__ __forceinline__ void load_values(typename A::V (&x)[1 << E], const u64 (&v)[1 << E],
                                             const A& ar, const NttPro& pro, int prime) {
-  const typename A::Lift lift = ar.make_lift(pro, prime);
-  if (lift.on) {
+  if (pro.kind == 1) {
+    const typename A::Lift lift = ar.make_lift(pro, prime);
 #pragma unroll
     for (int e = 0; e < (1 << E); e++) x[e] = ar.lift(v[e], lift);
+  } else if (pro.kind == 2) {
+    const bool          scaled = pro.mul != nullptr;
+    const typename A::T w      = scaled ? ar.constant(pro.mul + prime) : typename A::T{};
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) x[e] = ar.message(v[e], scaled, w);
   } else {
 #pragma unroll
     for (int e = 0; e < (1 << E); e++) x[e] = A::load(v[e]);

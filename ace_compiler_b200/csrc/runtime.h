@@ -150,8 +150,11 @@ struct Context {
   // encoder tables (util/src/ntt.c:562-590): 2N-th complex roots, powers of 5
   std::vector<double>   fft_rou_re, fft_rou_im;
   std::vector<uint32_t> fft_rot_group;
-  // device copies of the encoder's roots of unity, owned by encode_gpu.cu
-  void* encode_tables = nullptr;
+  // the encoder's and decoder's roots of unity and constants, pinned host
+  // buffers; owned by embedding.cu
+  void* embed_tables = nullptr;
+  void* host_buffers = nullptr;
+  uint32_t* triangle_jump = nullptr;  // owned by sampling.cu
   // transforms of the monomials the bootstrap multiplies by, owned by bootstrap.cu
   void* monomials = nullptr;
   // bootstrapping precomputation per slot count, owned by bootstrap.cu
@@ -241,16 +244,24 @@ void release_prng();
 void sample_uniform(int64_t* out, size_t n, u64 upper_bound);
 void sample_ternary(int64_t* out, size_t n, size_t hamming_weight);
 void sample_triangle(int64_t* out, size_t n);
+// `count` vectors of N samples each, drawn one after the other as sample_triangle does
+void sample_triangles_on_device(Context* c, int64_t* out, int count);
 
 // ---- client.cu ----
 void generate_keys(Context* c);
 void free_keys(Context* c);
 void generate_bootstrap_keys(Context* c, const std::vector<int32_t>& rotations);
 SWITCH_KEY* key_slot(Context* c, uint32_t key_id, bool create);
-// msg[N] (signed values, negatives stored as Max64 + x) -> residues per limb,
-// times scale_pow[prime] when given                       (crt.c:1153-1221)
-void launch_encode_split(int64_t* poly, const int64_t* msg, const u64* scale_pow,
-                         const LimbBatch& batch);
+// NTT form of `polys` message polynomials msg[polys][N] (signed values, negatives
+// also as Max64 + x), times pow[prime] when given, on the limbs of `one`, whose
+// limb i has to go to limb i of the result (crt.c:1153-1221)
+void message_to_ntt(Context* c, int64_t* out, const int64_t* msg, int polys, const Twiddle* pow,
+                    const LimbBatch& one);
+// c0 = pk0 u + e1 + m, c1 = pk1 u + e2 with noise = [u, e1, e2][level] (encryptor.c:19-89)
+void launch_encrypt(Context* c, int64_t* c0, int64_t* c1, const int64_t* noise, const int64_t* m,
+                    size_t level);
+// res = c0 + c1 s (decryptor.c:19-66)
+void launch_decrypt(Context* c, int64_t* res, const int64_t* c0, const int64_t* c1, size_t level);
 // small signed samples (-1, 0, 1) -> residues per limb (crt.c:1168-1172)
 void launch_small_to_rns(int64_t* poly, const int64_t* vals, const LimbBatch& batch);
 
@@ -371,20 +382,33 @@ inline cudaError_t stream_sync(cudaStream_t stream) {
   return e;
 }
 
-// ---- encode_gpu.cu ----
-// inverse embedding, scaling and rounding of `count` complex slot values (host)
-// into the message polynomial d_msg (N int64 on the device)
-// (`reals`, when given, replaces `values`: count real single-precision inputs)
-void encode_message_on_device(Context* c, const std::complex<double>* values, size_t count,
-                              uint32_t slots, int64_t* d_msg, const float* reals = nullptr);
-void free_encode_tables(Context* c);
+// ---- embedding.cu ----
+// slot values of a message on the host
+struct MessageInput {
+  enum Kind { kComplex, kReals, kFloats } kind;  // re/im pairs of doubles, doubles, floats
+  const void* data;
+  size_t      count;
+};
+// inverse embedding, scaling and rounding of the slot values into the message
+// polynomial d_msg (N int64 on the device; negatives as Max64 + x)
+void encode_message_on_device(Context* c, const MessageInput& in, uint32_t slots, int64_t* d_msg);
+// the first `count` slots (re/im pairs) of a polynomial in coefficient form, divided by `factor`
+void decode_on_device(Context* c, const int64_t* poly, int level, uint32_t slots, double factor,
+                      double* out, size_t count);
+// Delta^(degree-1) modulo every prime (kept on the device)
+const Twiddle* scale_powers(Context* c, uint32_t degree);
+void free_embed_tables(Context* c);
+// host data of the caller to the device, through pinned buffers; `dst` is a
+// whole block of dev_alloc (rounded up to 16 bytes)
+void  upload_staged(Context* c, void* dst, const void* src, size_t bytes);
+void* pinned_output(Context* c, size_t bytes);  // mapped host memory for a result
+void  free_host_buffers(Context* c);
 
 // ---- client_api.cu ----
 // encode at sf_degree and level; slots = 0 means N/2, num_p = K also fills
 // the special limbs (stored right behind the level Q limbs)
-void encode_vector(Context* c, PLAIN plain, std::vector<std::complex<double>>& values,
-                   uint32_t sf_degree, uint32_t level, uint32_t slots = 0, uint32_t num_p = 0,
-                   const float* reals = nullptr, size_t real_count = 0);
+void encode_vector(Context* c, PLAIN plain, const MessageInput& in, uint32_t sf_degree,
+                   uint32_t level, uint32_t slots = 0, uint32_t num_p = 0);
 // residues of one real value at the given scale on level Q limbs then num_p
 // special limbs
 std::vector<int64_t> encode_value(Context* c, double value, uint32_t level, double scale,
@@ -444,13 +468,16 @@ void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse, const Twidd
 // degrees of 512 and more: ntt_can_fuse).  The first pass reads in[a] and
 // writes limb k of `mid` (k = position in the batch), the last pass reads
 // mid[k] and writes out[dst]; up to 4096 both are one launch and mid is not used.
-//   prologue (pro_mul set): the source is the coefficient form of a dropped
-//     limb modulo q_last; the value transformed under prime i is
-//     switch_modulus(v, q_last -> q_i) * pro_mul[i]   (pro_mod[i] = q_last mod q_i)
+//   prologue: kind 1  the source is the coefficient form of a dropped limb modulo
+//             q_last; the value transformed under prime i is
+//             switch_modulus(v, q_last -> q_i) * pro_mul[i]   (pro_mod[i] = q_last mod q_i)
+//             kind 2  the source is a message of signed integers; its residues
+//             (times pro_mul[i] when given) are transformed
 //   epilogue: kind 1  out = aux[b] * epi_mul[i] + t      (rescale)
 //             kind 2  out = (aux[b] - t) * epi_mul[i] (+ add[b])   (ModDown)
 //     aux / add use base p[sel bit 1]
 struct NttFuse {
+  int            pro_kind = 0;
   const Twiddle* pro_mul = nullptr;
   const u64*     pro_mod = nullptr;
   u64            q_last  = 0;

@@ -312,6 +312,7 @@ void Fhert_shard_rescale_end(const int64_t* c0, const int64_t* c1, size_t level,
     }
   if (ntt_can_fuse()) {
     NttFuse f;
+    f.pro_kind = 1;
     f.pro_mul  = c->d_ql_neg + (size_t)l * c->L;
     f.pro_mod  = c->d_ql_mod + (size_t)l * c->L;
     f.q_last   = c->primes[l];
