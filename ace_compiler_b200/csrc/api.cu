@@ -773,7 +773,8 @@ POLY Mod_up(POLY res, POLY old_poly, uint32_t part) {
 // add[g] when given.  ext[g] has its special limbs at limb index ext_p_limb.
 void fhert_mod_down_polys(Context* c, int npoly, int64_t* const res[2],
                            const int64_t* const ext[2], int ext_p_limb,
-                           const int64_t* const add[2], size_t level, bool is_ntt) {
+                           const int64_t* const add[2], size_t level, bool is_ntt,
+                           const uint32_t* perm) {
   const uint32_t n = c->N;
   const int      K = c->K;
   FHERT_ASSERT(npoly * (int)level <= kMaxLimbs && npoly * K <= kMaxLimbs, "ModDown batch too large");
@@ -819,7 +820,8 @@ void fhert_mod_down_polys(Context* c, int npoly, int64_t* const res[2],
             LimbRef{(uint16_t)(g * level + i), (uint16_t)i, (uint16_t)i, (uint8_t)i, sel};
       }
     NttFuse f;
-    f.epi_kind = 2;
+    f.epi_kind = perm != nullptr ? 3 : 2;
+    f.perm     = perm;
     f.epi_mul  = c->d_p_inv;
     f.aux      = ptr2(ext[0], npoly > 1 ? ext[1] : nullptr);
     if (add) f.add = ptr2(add[0], npoly > 1 ? add[1] : nullptr);
@@ -1152,7 +1154,8 @@ CIPHER3 Mul_ciph3(CIPHER3 res, CIPHER a, CIPHER b) {
 // (parts extended polynomials of level + K limbs each).
 void fhert_switch_key_raised(Context* c, int64_t* out0, int64_t* out1, const int64_t* in,
                              const int64_t* digits, int parts, size_t level, SW_KEY swk,
-                             const int64_t* add0, const int64_t* add1) {
+                             const int64_t* add0, const int64_t* add1,
+                             const uint32_t* perm = nullptr) {
   const uint32_t n         = c->N;
   const size_t   ext_limbs = level + c->K;
   int64_t*       acc0      = nullptr;
@@ -1178,19 +1181,20 @@ void fhert_switch_key_raised(Context* c, int64_t* out0, int64_t* out1, const int
   int64_t*       r[2] = {out0, out1};
   const int64_t* x[2] = {acc0, acc1};
   const int64_t* a[2] = {add0, add1};
-  fhert_mod_down_polys(c, 2, r, x, (int)level, a, level, true);
+  fhert_mod_down_polys(c, 2, r, x, (int)level, a, level, true, perm);
   CUDA_CHECK(dev_free(acc0, c->stream));
 }
 
 void fhert_switch_key(Context* c, int64_t* out0, int64_t* out1, const int64_t* in, size_t level,
-                      SW_KEY swk, const int64_t* add0, const int64_t* add1) {
+                      SW_KEY swk, const int64_t* add0, const int64_t* add1,
+                      const uint32_t* perm = nullptr) {
   const int parts = (int)std::min<size_t>((level + c->alpha - 1) / c->alpha, c->dnum);
   FHERT_ASSERT(parts <= kMaxParts, "too many digits");
   const size_t ext_limbs = level + c->K;
   int64_t*     digits    = nullptr;
   CUDA_CHECK(dev_alloc(&digits, (size_t)parts * ext_limbs * c->N * sizeof(int64_t), c->stream));
   fhert_raise_parts(c, in, true, level, 0, parts, digits, ext_limbs, (int)level);
-  fhert_switch_key_raised(c, out0, out1, in, digits, parts, level, swk, add0, add1);
+  fhert_switch_key_raised(c, out0, out1, in, digits, parts, level, swk, add0, add1, perm);
   CUDA_CHECK(dev_free(digits, c->stream));
 }
 
@@ -1245,11 +1249,17 @@ static CIPHER rotate_with_key(CIPHER res, CIPHER ciph, int32_t rot_idx, uint32_t
   size_t   level = Level(ciph);
   size_t   words = level * c->N;
   int64_t* t     = nullptr;
+  if (res != ciph)
+    init_ciph(res, c->N, level, 0, ciph->_scaling_factor, ciph->_sf_degree, ciph->_slots);
+  if (ntt_can_fuse() && res->_c0_poly._data != ciph->_c0_poly._data) {
+    // permuted by the last pass of the key switch
+    fhert_switch_key(c, res->_c0_poly._data, res->_c1_poly._data, ciph->_c1_poly._data, level,
+                     Swk(true, rot_idx), ciph->_c0_poly._data, nullptr, auto_table(c, k));
+    return res;
+  }
   CUDA_CHECK(dev_alloc(&t, 2 * words * sizeof(int64_t), c->stream));
   fhert_switch_key(c, t, t + words, ciph->_c1_poly._data, level, Swk(true, rot_idx),
              ciph->_c0_poly._data, nullptr);
-  if (res != ciph)
-    init_ciph(res, c->N, level, 0, ciph->_scaling_factor, ciph->_sf_degree, ciph->_slots);
   LimbBatch one = poly_batch(c, &res->_c0_poly, &res->_c0_poly, nullptr, level, 0);
   launch_automorphism(ptr2(res->_c0_poly._data, res->_c1_poly._data), ptr2(t, t + words),
                       auto_table(c, k), both_polys(one));

@@ -82,6 +82,7 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
   epi.mul  = f.epi_mul;
   epi.aux  = f.aux;
   epi.add  = f.add;
+  epi.perm = f.perm;
   // strided pass: in[a] -> mid[k]; contiguous pass: mid[k] -> out[dst] with the epilogue
   LimbBatch b1 = b, b2 = b;
   for (int i = 0; i < b.count; i++) {

@@ -158,9 +158,16 @@ __device__ __forceinline__ u64 message_residue(u64 v, const Mod m, u64 r) {
 // Epilogue of the last pass on the canonical transform output t:
 //   kind 1 (rescale, rns_poly.c:367-383):  res = aux * mul[i] + t
 //   kind 2 (ModDown, rns_poly.c:293-304):  res = (aux - t) * mul[i] (+ add)
+//   kind 3:  kind 2, the result then permuted, res[i] = value[perm[i]] for an
+//            automorphism in NTT order.  The high bits of perm[i] depend on the
+//            high bits of i alone, so blocks of 256 go to blocks of 256: a CTA
+//            transforms the source blocks of its destination blocks, permutes in
+//            shared memory and still writes in order (a gather of its own cost
+//            23 us for 72 limbs at N = 2^16).
 // aux is limb LimbRef::b of aux.p[sel bit 1]; add uses the same limb index and
 // selector, a null base means no addend.
 struct NttEpi {
+  const uint32_t* perm = nullptr;
   int            kind = 0;
   const Twiddle* mul  = nullptr;  // [prime]
   Ptr2           aux{{nullptr, nullptr}};
@@ -532,17 +539,30 @@ __device__ __forceinline__ u64 finish_word(u64 v, int i, const u64* aux, const u
                                            const typename A::T& emul, const A& ar) {
   if (EPI != 0) {
     v = ar.template epilogue<EPI>(v, aux[i], emul);
-    if (EPI == 2 && add != nullptr) v = add_canon(v, add[i], ar.q);
+    if (EPI >= 2 && add != nullptr) v = add_canon(v, add[i], ar.q);
   }
   return v;
 }
 
+// place of word i of a block in its swizzled shared memory (16 lanes)
+__device__ __forceinline__ int place16(int i) { return i ^ ((i >> 4) & 15); }
+
 template <class A, int EPI>
-__device__ __forceinline__ void write_block16(u64* dst, const u64* sb, int t, const u64* aux,
-                                              const u64* add, const typename A::T& emul, const A& ar) {
+__device__ __forceinline__ void write_block16(u64* dst, u64* sb, int t, const u64* aux, const u64* add,
+                                              const typename A::T& emul, const A& ar,
+                                              const uint32_t* perm) {
 #pragma unroll
-  for (int e = 0; e < 16; e++)
-    dst[e * 16 + t] = finish_word<A, EPI>(sb[by_row(t, e)], e * 16 + t, aux, add, emul, ar);
+  for (int e = 0; e < 16; e++) {
+    const u64 v = finish_word<A, EPI>(sb[by_row(t, e)], e * 16 + t, aux, add, emul, ar);
+    if (EPI == 3) sb[by_row(t, e)] = v;
+    else dst[e * 16 + t] = v;
+  }
+  if (EPI == 3) {
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 16; e++)
+      dst[e * 16 + t] = sb[place16((int)__ldg(perm + e * 16 + t) & (kContigBlock - 1))];
+  }
 }
 
 // 32 lanes (8 values each), rounds of 2, 3 and 3 stages with the index patterns
@@ -565,7 +585,8 @@ __device__ __forceinline__ void sts64(u32 addr, u64 v) {
 template <bool INV, int EPI, class A>
 __device__ __forceinline__ void contig_int(const u64* src, u64* dst, u32 sbase, int g,
                                            const Twiddle* table, const A& ar, const u64* aux,
-                                           const u64* add, const Twiddle* emul) {
+                                           const u64* add, const Twiddle* emul,
+                                           const uint32_t* perm) {
   u64       x[8];
   const int b2 = ((g >> 3) << 6) | (g & 7);
   const u32 a1 = sbase ^ (u32)(swz(g) << 3);
@@ -595,9 +616,20 @@ __device__ __forceinline__ void contig_int(const u64* src, u64* dst, u32 sbase, 
     typename A::T w{};
     if (EPI != 0) w = ar.constant(emul);
 #pragma unroll
-    for (int e = 0; e < 8; e++)
-      dst[e * 32 + g] =
-          finish_word<A, EPI>(lds64(a1 ^ (u32)(swz(e << 5) << 3)), e * 32 + g, aux, add, w, ar);
+    for (int e = 0; e < 8; e++) {
+      const u32 at = a1 ^ (u32)(swz(e << 5) << 3);
+      const u64 v  = finish_word<A, EPI>(lds64(at), e * 32 + g, aux, add, w, ar);
+      if (EPI == 3) sts64(at, v);
+      else dst[e * 32 + g] = v;
+    }
+    if (EPI == 3) {
+      __syncwarp();
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        const int s = (int)__ldg(perm + e * 32 + g) & (kContigBlock - 1);
+        dst[e * 32 + g] = lds64(sbase ^ (u32)(swz(s) << 3));
+      }
+    }
   } else {
 #pragma unroll
     for (int e = 0; e < 8; e++) sts64(a1 ^ (u32)(swz(e << 5) << 3), src[e * 32 + g]);
@@ -628,7 +660,8 @@ __device__ __forceinline__ void contig_int(const u64* src, u64* dst, u32 sbase, 
 template <bool INV, int EPI>
 __device__ __forceinline__ void contig_float(const u64* src, u64* dst, u64* sb, int t,
                                              const double* table, const ArithFp& ar, const u64* aux,
-                                             const u64* add, const Twiddle* emul) {
+                                             const u64* add, const Twiddle* emul,
+                                             const uint32_t* perm) {
   double x[16];
   if constexpr (!INV) {
 #pragma unroll
@@ -636,7 +669,7 @@ __device__ __forceinline__ void contig_float(const u64* src, u64* dst, u64* sb, 
     contig16_fwd<ArithFp>(x, sb, t, table, ar);
     double w = 0;
     if (EPI != 0) w = ar.constant(emul);
-    write_block16<ArithFp, EPI>(dst, sb, t, aux, add, w, ar);
+    write_block16<ArithFp, EPI>(dst, sb, t, aux, add, w, ar, perm);
   } else {
 #pragma unroll
     for (int e = 0; e < 16; e++) sb[by_row(t, e)] = src[e * 16 + t];
@@ -681,10 +714,13 @@ ntt_contig_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, Ti
   const Twiddle*   tab    = tables + (size_t)lr.prime * table_entries(logn);
   const int        per    = is_int ? 32 : 16;  // lanes per block
   const int        slot = threadIdx.x / per, t = threadIdx.x & (per - 1);
-  const u32        blk    = tile * (kThreads / per) + slot;
+  const u32        to     = tile * (kThreads / per) + slot;  // block of the result
+  const uint32_t*  perm   = EPI == 3 ? epi.perm + (size_t)to * kContigBlock : nullptr;
+  const u32        blk    = EPI == 3 ? __ldg(perm) / kContigBlock : to;
   const size_t     off    = (size_t)blk * kContigBlock;
   const u64*       src    = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + off;
-  u64*             dst    = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n + off;
+  u64*             dst    = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n +
+                            (size_t)to * kContigBlock;
   const u64* aux = nullptr;
   const u64* add = nullptr;
   if (EPI != 0) {
@@ -698,12 +734,15 @@ ntt_contig_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, Ti
   if (is_int) {
     const u32 sbase = (((u32)__cvta_generic_to_shared(sm) + 2047u) & ~2047u) + (u32)slot * 2048u;
     if (dm.kind == kNttNarrow)
-      contig_int<INV, EPI>(src, dst, sbase, t, tab + entry, ArithInt<false>(dm), aux, add, emul);
+      contig_int<INV, EPI>(src, dst, sbase, t, tab + entry, ArithInt<false>(dm), aux, add, emul,
+                           perm);
     else
-      contig_int<INV, EPI>(src, dst, sbase, t, tab + entry, ArithInt<true>(dm), aux, add, emul);
+      contig_int<INV, EPI>(src, dst, sbase, t, tab + entry, ArithInt<true>(dm), aux, add, emul,
+                           perm);
   } else {
     contig_float<INV, EPI>(src, dst, sm + slot * kContigBlock, t,
-                           reinterpret_cast<const double*>(tab) + entry, ArithFp(dm), aux, add, emul);
+                           reinterpret_cast<const double*>(tab) + entry, ArithFp(dm), aux, add, emul,
+                           perm);
   }
 }
 
@@ -851,7 +890,7 @@ template <bool INV, int EPI, int S1, class A>
 __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, const Twiddle* table,
                                            const DevModulus& dm, const Twiddle* fin,
                                            const NttPro& pro, int prime, const u64* aux,
-                                           const u64* add, const Twiddle* emul) {
+                                           const u64* add, const Twiddle* emul, const uint32_t* perm) {
   constexpr int        logn = S1 + kContigLog, top = logn - 4;
   const A              ar(dm);
   const typename A::T* tree = reinterpret_cast<const typename A::T*>(table);
@@ -877,7 +916,17 @@ __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, co
     typename A::T w{};
     if (EPI != 0) w = ar.constant(emul);
     const size_t off = (size_t)half * kContigBlock;
-    write_block16<A, EPI>(dst + off, sb, t, aux + off, add != nullptr ? add + off : nullptr, w, ar);
+    if constexpr (EPI != 3) {
+      write_block16<A, EPI>(dst + off, sb, t, aux + off, add != nullptr ? add + off : nullptr, w, ar,
+                            nullptr);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; e++)
+        sb[by_row(t, e)] = finish_word<A, EPI>(sb[by_row(t, e)], (int)off + e * 16 + t, aux, add, w, ar);
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < 16; e++) dst[off + e * 16 + t] = sm[place16((int)__ldg(perm + off + e * 16 + t))];
+    }
   } else {
     const size_t off = (size_t)half * kContigBlock;
 #pragma unroll
@@ -917,11 +966,14 @@ ntt_whole_kernel(Ptr2 in, Ptr2 out, LimbBatch batch, const Twiddle* __restrict__
   }
   const Twiddle* emul = EPI != 0 ? epi.mul + lr.prime : nullptr;
   if (dm.kind == kNttFloat)
-    whole_body<INV, EPI, S1, ArithFp>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul);
+    whole_body<INV, EPI, S1, ArithFp>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
+                                       epi.perm);
   else if (dm.kind == kNttNarrow)
-    whole_body<INV, EPI, S1, ArithInt<false>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul);
+    whole_body<INV, EPI, S1, ArithInt<false>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
+                                       epi.perm);
   else
-    whole_body<INV, EPI, S1, ArithInt<true>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul);
+    whole_body<INV, EPI, S1, ArithInt<true>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
+                                       epi.perm);
 }
 
 // ---- tiny transforms (N < 512): one butterfly at a time --------------------------
@@ -1005,6 +1057,9 @@ inline void launch_contig(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, cons
   else if (epi.kind == 1)
     launch(ntt_contig_kernel<false, 1>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
            t.logn, epi);
+  else if (epi.kind == 3)
+    launch(ntt_contig_kernel<false, 3>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
+           t.logn, epi);
   else
     launch(ntt_contig_kernel<false, 2>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
            t.logn, epi);
@@ -1028,6 +1083,7 @@ inline void launch_whole(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables&
                          const NttEpi& epi = NttEpi()) {
   if (INV || epi.kind == 0) launch_whole_t<INV, 0>(in, out, b, t, stream, pro, epi);
   else if (epi.kind == 1) launch_whole_t<false, 1>(in, out, b, t, stream, pro, epi);
+  else if (epi.kind == 3) launch_whole_t<false, 3>(in, out, b, t, stream, pro, epi);
   else launch_whole_t<false, 2>(in, out, b, t, stream, pro, epi);
 }
 

@@ -475,6 +475,8 @@ void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse, const Twidd
 //             (times pro_mul[i] when given) are transformed
 //   epilogue: kind 1  out = aux[b] * epi_mul[i] + t      (rescale)
 //             kind 2  out = (aux[b] - t) * epi_mul[i] (+ add[b])   (ModDown)
+//             kind 3  kind 2, then permuted: out[i] = value[perm[i]]; `out` may not
+//                     overlap anything that is read
 //     aux / add use base p[sel bit 1]
 struct NttFuse {
   int            pro_kind = 0;
@@ -485,6 +487,7 @@ struct NttFuse {
   const Twiddle* epi_mul  = nullptr;
   Ptr2           aux{{nullptr, nullptr}};
   Ptr2           add{{nullptr, nullptr}};
+  const uint32_t* perm    = nullptr;
 };
 bool ntt_can_fuse();
 void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const NttFuse& f);
@@ -637,10 +640,12 @@ void fhert_raise_parts(fhert::Context* c, const int64_t* src, bool is_ntt, size_
                        int part_begin, int part_end, int64_t* ext_base, size_t part_stride,
                        int p_limb);
 // ModDown of one or two extended polynomials (special limbs at ext_p_limb),
-// optionally adding add[g] to the result
+// optionally adding add[g] to the result and permuting it (res[i] = value[perm[i]];
+// NTT form and ntt_can_fuse() only, res must not overlap ext or add)
 void fhert_mod_down_polys(fhert::Context* c, int npoly, int64_t* const res[2],
                           const int64_t* const ext[2], int ext_p_limb,
-                          const int64_t* const add[2], size_t level, bool is_ntt);
+                          const int64_t* const add[2], size_t level, bool is_ntt,
+                          const uint32_t* perm = nullptr);
 // Rescale of one or two NTT-form polynomials from level to level - 1
 void fhert_rescale_polys(fhert::Context* c, int npoly, int64_t* const res[2],
                          const int64_t* const poly[2], size_t level);

@@ -76,3 +76,51 @@ def test_base_conversions_match_the_oracle(degree, primes, bits, dnum):
             gpu.free(p)
     gpu.close()
     orc.close()
+
+
+def encrypted(gpu, rng, level):
+    ct = gpu.new_ciph(*(edge_limbs(rng, gpu.primes[:level], gpu.N) for _ in range(2)))
+    return ct, gpu.ciph_to_host(ct)
+
+
+# key switches of one, two and three digits, rings on both sides of the one-launch
+# transforms, in place and into a result of its own
+@pytest.mark.parametrize("degree,primes,bits,dnum", [
+    (64, 4, (33, 30), 2), (512, 7, (51, 46), 3), (4096, 5, (60, 56), 2), (16384, 9, (51, 46), 3)])
+def test_rotations_and_products_match_the_oracle(degree, primes, bits, dnum):
+    import ace_compiler_b200 as rt
+    steps = (1, -5, degree // 4)
+    gpu = rt.Runtime(degree, primes, *bits, dnum, rot_idxs=steps, keygen=True, seed=np.arange(16),
+                     fake_time_us=1_700_000_000_000_000)
+    orc = oracle_lib.Oracle(degree, primes, *bits, dnum)
+    rng, lib = np.random.default_rng(degree), gpu.lib
+    key = lambda rot, idx: [[gpu.export_switch_key(rot, idx, part, which) for which in (0, 1)] for part in range(gpu.dnum)]
+    keys, relin = {s: key(True, s) for s in steps}, key(False, 0)
+    for level in sorted({1, gpu.alpha, gpu.alpha + 1, primes}):
+        ct, host = encrypted(gpu, rng, level)
+        outs = (rt.CIPHERTEXT * 4)()
+        lib.Rotate_batch_ciph(outs, C.byref(ct), (C.c_int32 * 4)(steps[0], 0, *steps[1:]), 4)
+        for out, step in zip((outs[0], outs[2], outs[3]), steps):
+            want = orc.rotate(*host, step, keys[step])
+            single = rt.CIPHERTEXT()
+            lib.Rotate_ciph(C.byref(single), C.byref(ct), step)
+            for got in (gpu.ciph_to_host(out), gpu.ciph_to_host(single)):
+                assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (level, step)
+            gpu.free_ciph(single)
+        assert np.array_equal(gpu.ciph_to_host(outs[1])[0], host[0])
+        lib.Free_ciph_poly(outs, 4)
+        lib.Rotate_ciph(C.byref(ct), C.byref(ct), steps[1])
+        assert np.array_equal(gpu.ciph_to_host(ct)[0], orc.rotate(*host, steps[1], keys[steps[1]])[0])
+        gpu.free_ciph(ct)
+        if level < 2:
+            continue
+        (a, ha), (b, hb) = encrypted(gpu, rng, level), encrypted(gpu, rng, level)
+        prod, low = rt.CIPHERTEXT(), rt.CIPHERTEXT()
+        lib.Mul_ciph(C.byref(prod), C.byref(a), C.byref(b))
+        lib.Rescale_ciph(C.byref(low), C.byref(prod))
+        want, got = orc.mul_relin_rescale(*ha, *hb, relin), gpu.ciph_to_host(low)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), level
+        for x in (a, b, prod, low):
+            gpu.free_ciph(x)
+    gpu.close()
+    orc.close()
