@@ -851,6 +851,48 @@ void fhert_mod_down_polys(Context* c, int npoly, int64_t* const res[2],
   launch_moddown_combine(tail);
 }
 
+int fhert_mod_down_many_limit(Context* c, size_t level) {
+  if (!ntt_can_fuse()) return 0;
+  return std::min(kMaxMulti, kMaxLimbs / std::max((int)level, c->K));
+}
+
+void fhert_mod_down_many(Context* c, int polys, const int64_t* ext, size_t ext_stride, int ext_p_limb,
+                         size_t level, const NttMulti& to) {
+  const size_t n = c->N;
+  const int    K = c->K, l = (int)level;
+  int64_t*     sc   = scratch((size_t)polys * (K + level) * n);
+  int64_t*     conv = sc + (size_t)polys * K * n;  // [polys][level]
+  LimbBatch    in, out;
+  in.count  = polys * K;
+  out.count = polys * l;
+  ConvArgs args;
+  args.groups    = polys;
+  args.level     = l;
+  args.out_total = l;
+  args.p_limb    = 0;
+  args.width     = (K + 3) & ~3;
+  for (int g = 0; g < polys; g++) {
+    const size_t base = (size_t)g * ext_stride;
+    for (int k = 0; k < K; k++)
+      in.limb[g * K + k] = LimbRef{(uint16_t)(base + ext_p_limb + k), 0, (uint16_t)(g * K + k),
+                                   (uint8_t)(c->L + k), 0};
+    args.g[g] = ConvGroup{reinterpret_cast<const u64*>(sc + (size_t)g * K * n),
+                          reinterpret_cast<u64*>(conv + (size_t)g * level * n), nullptr, c->d_phat_planes,
+                          0, c->L, K, 0, 0};
+    for (int i = 0; i < l; i++)
+      out.limb[g * l + i] = LimbRef{(uint16_t)(g * l + i), (uint16_t)(base + i), (uint16_t)i, (uint8_t)i,
+                                    (uint8_t)g};
+  }
+  launch_ntt(ptr2(ext), ptr2(sc), in, true, c->d_moddown_last);
+  launch_base_conv(args);
+  NttFuse f;
+  f.epi_kind = 4;
+  f.epi_mul  = c->d_p_inv;
+  f.aux      = ptr2(ext);
+  f.multi    = &to;
+  launch_ntt_fused(ptr2(conv), conv, ptr2(nullptr), out, f);
+}
+
 POLY Mod_down(POLY res, POLY poly) {
   size_t level = poly->_num_primes;
   if (res->_data == nullptr) Alloc_poly_data(res, ctx()->N, level, 0);
@@ -1275,25 +1317,71 @@ void Rotate_batch_ciph(CIPHER res_arr, CIPHER ciph, const int32_t* rot_idx, uint
   Context* c     = ctx();
   size_t   level = Level(ciph), words = level * c->N, ext_limbs = level + c->K;
   const int parts = (int)std::min<size_t>((level + c->alpha - 1) / c->alpha, c->dnum);
-  int64_t *digits = nullptr, *t = nullptr;
+  int64_t *digits = nullptr, *acc = nullptr;
   CUDA_CHECK(dev_alloc(&digits, (size_t)parts * ext_limbs * c->N * sizeof(int64_t), c->stream));
-  CUDA_CHECK(dev_alloc(&t, 2 * words * sizeof(int64_t), c->stream));
   fhert_raise_parts(c, ciph->_c1_poly._data, true, level, 0, parts, digits, ext_limbs, (int)level);
+  std::vector<uint32_t> turns;  // the others are copies
   for (uint32_t i = 0; i < count; i++) {
-    CIPHER out = &res_arr[i];
-    FHERT_ASSERT(out != ciph, "Rotate_batch_ciph cannot work in place");
+    FHERT_ASSERT(&res_arr[i] != ciph, "Rotate_batch_ciph cannot work in place");
     if (rot_idx[i] == 0) {
-      Copy_ciph(out, ciph);
+      Copy_ciph(&res_arr[i], ciph);
       continue;
     }
-    fhert_switch_key_raised(c, t, t + words, ciph->_c1_poly._data, digits, parts, level,
-                            Swk(true, rot_idx[i]), ciph->_c0_poly._data, nullptr);
-    init_ciph(out, c->N, level, 0, ciph->_scaling_factor, ciph->_sf_degree, ciph->_slots);
-    LimbBatch one = poly_batch(c, &out->_c0_poly, &out->_c0_poly, nullptr, level, 0);
-    launch_automorphism(ptr2(out->_c0_poly._data, out->_c1_poly._data), ptr2(t, t + words),
-                        auto_table(c, auto_index_for(c, rot_idx[i])), both_polys(one));
+    init_ciph(&res_arr[i], c->N, level, 0, ciph->_scaling_factor, ciph->_sf_degree, ciph->_slots);
+    turns.push_back(i);
   }
-  CUDA_CHECK(dev_free(t, c->stream));
+  // one launch for all keys of a group, one ModDown for all its results
+  const int limit = fhert_mod_down_many_limit(c, level) / 2;
+  if (limit == 0) {  // a ring too small for the fused passes
+    int64_t* t = nullptr;
+    CUDA_CHECK(dev_alloc(&t, 2 * words * sizeof(int64_t), c->stream));
+    for (uint32_t i : turns) {
+      CIPHER out = &res_arr[i];
+      fhert_switch_key_raised(c, t, t + words, ciph->_c1_poly._data, digits, parts, level,
+                              Swk(true, rot_idx[i]), ciph->_c0_poly._data, nullptr);
+      LimbBatch one = poly_batch(c, &out->_c0_poly, &out->_c0_poly, nullptr, level, 0);
+      launch_automorphism(ptr2(out->_c0_poly._data, out->_c1_poly._data), ptr2(t, t + words),
+                          auto_table(c, auto_index_for(c, rot_idx[i])), both_polys(one));
+    }
+    CUDA_CHECK(dev_free(t, c->stream));
+    turns.clear();
+  }
+  const size_t group = std::min<size_t>(limit, turns.size());
+  if (group > 0)
+    CUDA_CHECK(dev_alloc(&acc, group * 2 * ext_limbs * c->N * sizeof(int64_t), c->stream));
+  for (size_t first = 0; first < turns.size(); first += group) {
+    KeysArgs args;
+    std::memset(&args, 0, sizeof(args));
+    args.parts        = parts;
+    args.level        = (int)level;
+    args.alpha        = c->alpha;
+    args.key_p_limb   = c->L;
+    args.count        = (int)std::min(group, turns.size() - first);
+    args.in           = reinterpret_cast<const u64*>(ciph->_c1_poly._data);
+    args.digits       = reinterpret_cast<const u64*>(digits);
+    args.digit_stride = ext_limbs * c->N;
+    args.out          = reinterpret_cast<u64*>(acc);
+    args.out_stride   = 2 * ext_limbs * c->N;
+    args.poly_stride  = ext_limbs * c->N;
+    NttMulti to;
+    std::memset(&to, 0, sizeof(to));
+    for (int r = 0; r < args.count; r++) {
+      const int32_t step = rot_idx[turns[first + r]];
+      CIPHER        out  = &res_arr[turns[first + r]];
+      SW_KEY        key  = Swk(true, step);
+      for (int j = 0; j < parts; j++) {
+        args.key0[r][j] = reinterpret_cast<const u64*>(key->_parts[j]._p0._data);
+        args.key1[r][j] = reinterpret_cast<const u64*>(key->_parts[j]._p1._data);
+      }
+      to.out[2 * r]     = reinterpret_cast<u64*>(out->_c0_poly._data);
+      to.out[2 * r + 1] = reinterpret_cast<u64*>(out->_c1_poly._data);
+      to.add[2 * r]     = reinterpret_cast<const u64*>(ciph->_c0_poly._data);
+      to.perm[2 * r] = to.perm[2 * r + 1] = auto_table(c, auto_index_for(c, step));
+    }
+    launch_keys_product(args);
+    fhert_mod_down_many(c, 2 * args.count, acc, ext_limbs, (int)level, level, to);
+  }
+  if (acc) CUDA_CHECK(dev_free(acc, c->stream));
   CUDA_CHECK(dev_free(digits, c->stream));
 }
 

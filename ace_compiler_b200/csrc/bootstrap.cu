@@ -904,34 +904,37 @@ LimbBatch q_only(Context* c, size_t level) {
   return b;
 }
 
-// key-switch inner product of raised digits with the key of automorphism k:
-// acc (two extended polynomials) = sum_j digit_j * key_j
-void digits_times_key(Context* c, const int64_t* digits, const int64_t* own, size_t level,
-                      int parts, uint32_t k, int64_t* acc) {
+// digits of a polynomial (with its own limbs at `own`) against the keys of some
+// automorphisms; the results are permuted by them (launch_keys_product)
+KeysArgs keys_args(Context* c, const int64_t* digits, const int64_t* own, size_t level, int parts) {
+  const size_t n = c->N, ext = level + c->K;
+  KeysArgs args;
+  std::memset(&args, 0, sizeof(args));
+  args.parts        = parts;
+  args.level        = (int)level;
+  args.alpha        = c->alpha;
+  args.key_p_limb   = c->L;
+  args.in           = reinterpret_cast<const u64*>(own);
+  args.digits       = reinterpret_cast<const u64*>(digits);
+  args.digit_stride = ext * n;
+  args.poly_stride  = ext * n;
+  return args;
+}
+void add_key(Context* c, KeysArgs& args, uint32_t k) {
   SWITCH_KEY* key = key_slot(c, k, false);
   FHERT_ASSERT(key != nullptr, "cannot find the rotation key of automorphism %u", k);
-  const size_t ext = level + c->K, n = c->N;
-  InnerArgs args;
-  std::memset(&args, 0, sizeof(args));
-  args.parts      = parts;
-  args.level      = (int)level;
-  args.alpha      = c->alpha;
-  args.key_p_limb = c->L;
-  args.ext_p_limb = (int)level;
-  args.acc_p_limb = (int)level;
-  args.in         = reinterpret_cast<const u64*>(own);
-  for (int j = 0; j < parts; j++) {
-    args.ext_ptr[j] = reinterpret_cast<const u64*>(digits + (size_t)j * ext * n);
-    args.key0[j]    = reinterpret_cast<const u64*>(key->_parts[j]._p0._data);
-    args.key1[j]    = reinterpret_cast<const u64*>(key->_parts[j]._p1._data);
+  const int r = args.count++;
+  // where source coefficient i goes: the table of the inverse automorphism
+  args.place[r] = auto_table(c, inverse_mod_2n(k, c->N));
+  for (int j = 0; j < args.parts; j++) {
+    args.key0[r][j] = reinterpret_cast<const u64*>(key->_parts[j]._p0._data);
+    args.key1[r][j] = reinterpret_cast<const u64*>(key->_parts[j]._p1._data);
   }
-  args.acc0 = reinterpret_cast<u64*>(acc);
-  args.acc1 = reinterpret_cast<u64*>(acc + ext * n);
-  launch_inner_product(args);
 }
 
-// one stage: rescale, hoisted giant-step rotations, fused baby-step sums,
-// outer rotations on the extended basis, one ModDown at the end
+// one stage: rescale, hoisted giant-step rotations (one launch over all their
+// keys), all baby-step sums in one launch, outer rotations on the extended basis,
+// one ModDown at the end
 void rotate_stage(Context* c, CIPHER ct, std::vector<PLAINTEXT>& plains, const FftParams& p,
                   const std::vector<int32_t>& rot_in, const std::vector<int32_t>& rot_out, int step,
                   bool encoding, bool is_rem) {
@@ -944,104 +947,113 @@ void rotate_stage(Context* c, CIPHER ct, std::vector<PLAINTEXT>& plains, const F
   const size_t pw = ext * n;  // words of one extended polynomial
   const int    parts = (int)std::min<size_t>((level + c->alpha - 1) / c->alpha, c->dnum);
   FHERT_ASSERT(giant <= kMaxParts, "giant step %d exceeds the fused limit", giant);
-  const LimbBatch eb = ext_batch(c, level), eb2 = both_polys(eb), qb = q_only(c, level);
-  // both polynomials on the extended basis; the Q limbs of the first one also
-  // pick up the lifted c0 while they are permuted
-  LimbBatch eb2_add = eb2;
-  for (int i = 0; i < eb2_add.count; i++) {
-    LimbRef& r = eb2_add.limb[i];
-    bool     q_of_c0 = i < (int)level;
-    r.b   = q_of_c0 ? (uint16_t)i : 0;
-    r.sel = (uint8_t)((r.sel & ~2) | (q_of_c0 ? 2 : 0));  // bit 1 = "add the lifted limb"
-  }
+  const LimbBatch eb2 = both_polys(ext_batch(c, level)), qb = q_only(c, level);
 
-  DevBuf digits(c, (size_t)parts * pw), rot(c, (size_t)giant * 2 * pw), lifted(c, 2 * pw);
-  DevBuf acc(c, 2 * pw), inner(c, 2 * pw), outer(c, 2 * pw), first(c, pw), turned(c, 2 * pw);
-  DevBuf low(c, level * n);
+  DevBuf digits(c, (size_t)parts * pw), rot(c, (size_t)giant * 2 * pw), sums(c, (size_t)baby * 2 * pw);
   int64_t* c0 = ct->_c0_poly._data;
   int64_t* c1 = ct->_c1_poly._data;
-
-  // lifted = (P * c0, P * c1) on the Q limbs, zero on the special limbs
-  CUDA_CHECK(zero_async(lifted.p, 2 * pw * sizeof(int64_t), c->stream));
-  launch_mul_const(ptr2(lifted.p, lifted.p + pw), ptr2(c0, c1), c->d_p_mod_q, both_polys(qb));
   fhert_raise_parts(c, c1, true, level, 0, parts, digits.p, ext, (int)level);
 
+  // rotation j at rot.p + j * 2 * pw; the first polynomials pick up P * c0
+  KeysArgs keys = keys_args(c, digits.p, c1, level, parts);
+  keys.c0         = reinterpret_cast<const u64*>(c0);
+  keys.p_mod_q    = c->d_p_mod_q;
+  keys.out_stride = 2 * pw;
+  int  run_begin  = 0;  // launches cover runs of rotations that stand side by side
+  auto flush_keys = [&]() {
+    if (keys.count == 0) return;
+    keys.out = reinterpret_cast<u64*>(rot.p + (size_t)run_begin * 2 * pw);
+    launch_keys_product(keys);
+    keys.count = 0;
+  };
   for (int j = 0; j < giant; j++) {
     int64_t* dst = rot.p + (size_t)j * 2 * pw;
-    int32_t  val = rot_in[j];
-    if (val == 0) {
-      CUDA_CHECK(counted_copy(dst, lifted.p, 2 * pw * sizeof(int64_t), cudaMemcpyDeviceToDevice,
-                                 c->stream));
+    if (rot_in[j] == 0) {  // (P * c0, P * c1), zero on the special limbs
+      flush_keys();
+      launch_mul_const(ptr2(dst, dst + pw), ptr2(c0, c1), c->d_p_mod_q, both_polys(qb));
+      for (int k = 0; k < 2; k++)
+        CUDA_CHECK(zero_async(dst + k * pw + level * n, K * n * sizeof(int64_t), c->stream));
       continue;
     }
-    uint32_t k = auto_index_for(c, val);
-    digits_times_key(c, digits.p, c1, level, parts, k, acc.p);
-    launch_automorphism_add(ptr2(dst, dst + pw), ptr2(acc.p, acc.p + pw), lifted.p,
-                            auto_table(c, k), eb2_add);
+    if (keys.count == kMaxKeys) flush_keys();
+    if (keys.count == 0) run_begin = j;
+    add_key(c, keys, auto_index_for(c, rot_in[j]));
   }
+  flush_keys();
 
+  // sum i = sum_j rot_j * plain[giant * i + j] at sums.p + i * 2 * pw
   double   plain_sf     = 0;
   uint32_t plain_degree = 0;
-  for (int i = 0; i < baby; i++) {
-    // inner = sum_j rot_j * plain[giant * i + j]
-    InnerArgs args;
+  for (int first = 0; first < baby; first += kMaxSums) {
+    SumsArgs args;
     std::memset(&args, 0, sizeof(args));
-    args.level      = (int)level;
-    args.alpha      = c->alpha;
-    args.key_p_limb = (int)level;
-    args.acc_p_limb = (int)level;
-    args.in         = nullptr;
-    int terms = 0;
-    for (int j = 0; j < giant; j++) {
-      int dim2 = giant * i + j;
-      if (dim2 == num_rot) continue;
-      PLAINTEXT& pt = plains[dim2];
-      FHERT_ASSERT(pt._poly._data != nullptr && pt._poly._num_primes >= level,
-                   "missing or too shallow transform plaintext");
-      args.ext_p_limb  = (int)(pt._poly._num_alloc_primes - pt._poly._num_primes_p);
-      args.ext_ptr[terms] = reinterpret_cast<const u64*>(pt._poly._data);
-      args.key0[terms]    = reinterpret_cast<const u64*>(rot.p + (size_t)j * 2 * pw);
-      args.key1[terms]    = reinterpret_cast<const u64*>(rot.p + (size_t)j * 2 * pw + pw);
-      plain_sf     = pt._scaling_factor;
-      plain_degree = pt._sf_degree;
-      terms++;
-    }
-    args.parts = terms;
-    args.acc0  = reinterpret_cast<u64*>(inner.p);
-    args.acc1  = reinterpret_cast<u64*>(inner.p + pw);
-    launch_inner_product(args);
-
-    if (i == 0) {
-      CUDA_CHECK(counted_copy(first.p, inner.p, pw * sizeof(int64_t), cudaMemcpyDeviceToDevice,
-                                 c->stream));
-      CUDA_CHECK(zero_async(outer.p, pw * sizeof(int64_t), c->stream));
-      CUDA_CHECK(counted_copy(outer.p + pw, inner.p + pw, pw * sizeof(int64_t),
-                                 cudaMemcpyDeviceToDevice, c->stream));
-      continue;
-    }
-    int32_t val = rot_out[i];
-    if (val == 0) {
-      launch_elementwise(EW_ADD, ptr2(first.p), ptr2(first.p), ptr2(inner.p), 0, eb);
-      launch_elementwise(EW_ADD, ptr2(outer.p + pw), ptr2(outer.p + pw), ptr2(inner.p + pw), 0, eb);
-      continue;
-    }
-    uint32_t k = auto_index_for(c, val);
-    // c0 part stays extended: first += sigma_k(inner.c0)
-    launch_automorphism(ptr2(turned.p), ptr2(inner.p), auto_table(c, k), eb);
-    launch_elementwise(EW_ADD, ptr2(first.p), ptr2(first.p), ptr2(turned.p), 0, eb);
-    // c1 part: back to Q, key switch, rotate, accumulate on the extended basis
-    int64_t*       r[2] = {low.p, nullptr};
-    const int64_t* x[2] = {inner.p + pw, nullptr};
-    fhert_mod_down_polys(c, 1, r, x, (int)level, nullptr, level, true);
-    fhert_raise_parts(c, low.p, true, level, 0, parts, digits.p, ext, (int)level);
-    digits_times_key(c, digits.p, low.p, level, parts, k, acc.p);
-    launch_automorphism(ptr2(turned.p, turned.p + pw), ptr2(acc.p, acc.p + pw), auto_table(c, k), eb2);
-    launch_elementwise(EW_ADD, ptr2(outer.p, outer.p + pw), ptr2(outer.p, outer.p + pw),
-                       ptr2(turned.p, turned.p + pw), 0, eb2);
+    args.level       = (int)level;
+    args.terms       = giant;
+    args.sums        = std::min(kMaxSums, baby - first);
+    args.rot         = reinterpret_cast<const u64*>(rot.p);
+    args.out         = reinterpret_cast<u64*>(sums.p + (size_t)first * 2 * pw);
+    args.rot_stride  = args.out_stride = 2 * pw;
+    args.poly_stride = pw;
+    for (int i = 0; i < args.sums; i++)
+      for (int j = 0; j < giant; j++) {
+        int dim2 = giant * (first + i) + j;
+        if (dim2 == num_rot) continue;
+        PLAINTEXT& pt = plains[dim2];
+        FHERT_ASSERT(pt._poly._data != nullptr && pt._poly._num_primes >= level,
+                     "missing or too shallow transform plaintext");
+        args.plain[i][j].data   = reinterpret_cast<const u64*>(pt._poly._data);
+        args.plain[i][j].p_limb = (int)(pt._poly._num_alloc_primes - pt._poly._num_primes_p);
+        plain_sf     = pt._scaling_factor;
+        plain_degree = pt._sf_degree;
+      }
+    launch_weighted_sums(args);
   }
-  launch_elementwise(EW_ADD, ptr2(outer.p), ptr2(outer.p), ptr2(first.p), 0, eb);
+
+  // The outer rotations join sum 0: both polynomials of sigma_i(sum i), the
+  // second one key-switched first (back to Q, digits, inner product).
+  int64_t* total = sums.p;
+  DevBuf   low(c, (size_t)baby * level * n);
+  std::vector<int> turned;
+  for (int i = 1; i < baby; i++) {
+    int64_t* sum = sums.p + (size_t)i * 2 * pw;
+    if (rot_out[i] != 0) {
+      turned.push_back(i);
+      continue;
+    }
+    launch_elementwise(EW_ADD, ptr2(total, total + pw), ptr2(total, total + pw), ptr2(sum, sum + pw), 0, eb2);
+  }
+  const int limit = fhert_mod_down_many_limit(c, level);
+  if (limit > 0) {
+    // turned holds consecutive sums unless one of them was not rotated
+    for (size_t k = 0; k < turned.size();) {
+      size_t run = 1;
+      while (k + run < turned.size() && (int)run < limit && turned[k + run] == turned[k] + (int)run) run++;
+      NttMulti to;
+      std::memset(&to, 0, sizeof(to));
+      for (size_t r = 0; r < run; r++)
+        to.out[r] = reinterpret_cast<u64*>(low.p + (size_t)turned[k + r] * level * n);
+      fhert_mod_down_many(c, (int)run, sums.p + (size_t)turned[k] * 2 * pw + pw, 2 * ext, (int)level, level, to);
+      k += run;
+    }
+  } else {
+    for (int i : turned) {
+      int64_t*       r[2] = {low.p + (size_t)i * level * n, nullptr};
+      const int64_t* x[2] = {sums.p + (size_t)i * 2 * pw + pw, nullptr};
+      fhert_mod_down_polys(c, 1, r, x, (int)level, nullptr, level, true);
+    }
+  }
+  for (int i : turned) {
+    const int64_t* mine = low.p + (size_t)i * level * n;
+    fhert_raise_parts(c, mine, true, level, 0, parts, digits.p, ext, (int)level);
+    KeysArgs outer   = keys_args(c, digits.p, mine, level, parts);
+    outer.c0         = reinterpret_cast<const u64*>(sums.p + (size_t)i * 2 * pw);
+    outer.out        = reinterpret_cast<u64*>(total);
+    outer.accumulate = true;
+    add_key(c, outer, auto_index_for(c, rot_out[i]));
+    launch_keys_product(outer);
+  }
   int64_t*       r[2] = {c0, c1};
-  const int64_t* x[2] = {outer.p, outer.p + pw};
+  const int64_t* x[2] = {total, total + pw};
   fhert_mod_down_polys(c, 2, r, x, (int)level, nullptr, level, true);
   ct->_scaling_factor = ct->_scaling_factor * plain_sf;
   ct->_sf_degree      = ct->_sf_degree + plain_degree;

@@ -246,6 +246,8 @@ void generate_switching_key(Context* c, SWITCH_KEY* res, POLY new_key, POLY old_
   Free_poly_data(&e);
 }
 
+}  // namespace
+
 uint32_t inverse_mod_2n(uint32_t v, uint32_t n) {
   // number_theory.c:57-80 with modulus 2N
   int64_t m = 2ll * n, a = v % m, y = 0, x = 1, mod = m;
@@ -261,7 +263,6 @@ uint32_t inverse_mod_2n(uint32_t v, uint32_t n) {
   return (uint32_t)x;
 }
 
-}  // namespace
 
 // key_gen.c:235-262 with is_fast: the key switches from the rotated secret key
 // to the secret key, so that the automorphism can be applied after the switch

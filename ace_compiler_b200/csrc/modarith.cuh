@@ -114,6 +114,19 @@ __device__ __forceinline__ u64 reduce_128(u64 hi, u64 lo, const DevModulus& m) {
   return r;
 }
 
+// Canonical reduction of a sum of at most four products of residues (value below
+// 4 q^2, q < 2^60) with the single-word constant, as in mul_mod: the quotient
+// estimate is less than 6 too small.
+__device__ __forceinline__ u64 reduce_few(u64 hi, u64 lo, const DevModulus& m) {
+  uint32_t s  = m.bits - 1;
+  u64      x1 = (hi << (64 - s)) | (lo >> s);
+  u64      r  = lo - mulhi_under(x1, m.bar) * m.q;
+  if (r >= 4 * m.q) r -= 4 * m.q;
+  if (r >= 2 * m.q) r -= 2 * m.q;
+  if (r >= m.q) r -= m.q;
+  return r;
+}
+
 // acc(hi:lo) += a*b
 __device__ __forceinline__ void mac_128(u64& hi, u64& lo, u64 a, u64 b) {
   u64 ph, pl;

@@ -87,28 +87,37 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
   LimbBatch b1 = b, b2 = b;
   for (int i = 0; i < b.count; i++) {
     b1.limb[i].dst = (uint16_t)i;
-    b1.limb[i].sel = (uint8_t)(b.limb[i].sel & 1);
+    b1.limb[i].sel = (uint8_t)(f.multi ? 0 : b.limb[i].sel & 1);
     b2.limb[i].a   = (uint16_t)i;
-    b2.limb[i].sel = (uint8_t)(b.limb[i].sel & 6);
+    b2.limb[i].sel = (uint8_t)(f.multi ? b.limb[i].sel : b.limb[i].sel & 6);
   }
   const int n_int = integers_first(c, b1);
   integers_first(c, b2);
   DagScope dag(DAG_NTT_FUSED);
   if (dag.live) {
     const size_t w = (size_t)c->N * sizeof(u64);
-    dag.batch(b, c->N, &out, &in, nullptr);
     dag.set.write(mid, (size_t)b.count * w);
-    for (int i = 0; i < b.count && f.epi_kind != 0; i++) {
+    if (f.multi == nullptr) dag.batch(b, c->N, &out, &in, nullptr);
+    for (int i = 0; i < b.count; i++) {
       const LimbRef& lr = b.limb[i];
-      dag.set.read(f.aux.p[(lr.sel >> 1) & 1] + (size_t)lr.b * c->N, w);
-      const u64* add = f.add.p[(lr.sel >> 1) & 1];
-      if (add != nullptr) dag.set.read(add + (size_t)lr.b * c->N, w);
+      const size_t   at = (size_t)lr.b * c->N;
+      if (f.multi != nullptr) {
+        const size_t to = (size_t)lr.dst * c->N;
+        dag.set.read(in.p[0] + (size_t)lr.a * c->N, w);
+        dag.set.read(f.aux.p[0] + at, w);
+        if (f.multi->add[lr.sel] != nullptr) dag.set.read(f.multi->add[lr.sel] + to, w);
+        dag.set.write(f.multi->out[lr.sel] + to, w);
+      } else if (f.epi_kind != 0) {
+        dag.set.read(f.aux.p[(lr.sel >> 1) & 1] + at, w);
+        const u64* add = f.add.p[(lr.sel >> 1) & 1];
+        if (add != nullptr) dag.set.read(add + at, w);
+      }
     }
   }
   dag.commit();
   if (t.logn <= nttk::kWholeMaxLog) {
     prof_before(KID_NTT_SMALL);
-    nttk::launch_whole<false>(in, out, b, t, c->stream, pro, epi);
+    nttk::launch_whole<false>(in, out, b, t, c->stream, pro, epi, f.multi);
     prof_after(KID_NTT_SMALL, b.count);
     c->launches++;
     CUDA_CHECK(cudaGetLastError());
@@ -118,7 +127,7 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
   nttk::launch_strided<false>(in, ptr2(mid), b1, n_int, t, c->stream, pro);
   prof_after(KID_NTT_STRIDED, b.count);
   prof_before(KID_NTT_CONTIG);
-  nttk::launch_contig<false>(ptr2(mid), out, b2, n_int, t, c->stream, epi);
+  nttk::launch_contig<false>(ptr2(mid), out, b2, n_int, t, c->stream, epi, f.multi);
   prof_after(KID_NTT_CONTIG, b.count);
   c->launches += 2;
   CUDA_CHECK(cudaGetLastError());

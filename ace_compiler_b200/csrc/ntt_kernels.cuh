@@ -166,6 +166,7 @@ __device__ __forceinline__ u64 message_residue(u64 v, const Mod m, u64 r) {
 //            23 us for 72 limbs at N = 2^16).
 // aux is limb LimbRef::b of aux.p[sel bit 1]; add uses the same limb index and
 // selector, a null base means no addend.
+//   kind 4:  kind 2 or 3, polynomial by polynomial (NttMulti)
 struct NttEpi {
   const uint32_t* perm = nullptr;
   int            kind = 0;
@@ -554,10 +555,10 @@ __device__ __forceinline__ void write_block16(u64* dst, u64* sb, int t, const u6
 #pragma unroll
   for (int e = 0; e < 16; e++) {
     const u64 v = finish_word<A, EPI>(sb[by_row(t, e)], e * 16 + t, aux, add, emul, ar);
-    if (EPI == 3) sb[by_row(t, e)] = v;
+    if (EPI >= 3 && perm != nullptr) sb[by_row(t, e)] = v;
     else dst[e * 16 + t] = v;
   }
-  if (EPI == 3) {
+  if (EPI >= 3 && perm != nullptr) {
     __syncwarp();
 #pragma unroll
     for (int e = 0; e < 16; e++)
@@ -619,10 +620,10 @@ __device__ __forceinline__ void contig_int(const u64* src, u64* dst, u32 sbase, 
     for (int e = 0; e < 8; e++) {
       const u32 at = a1 ^ (u32)(swz(e << 5) << 3);
       const u64 v  = finish_word<A, EPI>(lds64(at), e * 32 + g, aux, add, w, ar);
-      if (EPI == 3) sts64(at, v);
+      if (EPI >= 3 && perm != nullptr) sts64(at, v);
       else dst[e * 32 + g] = v;
     }
-    if (EPI == 3) {
+    if (EPI >= 3 && perm != nullptr) {
       __syncwarp();
 #pragma unroll
       for (int e = 0; e < 8; e++) {
@@ -699,11 +700,18 @@ __device__ __forceinline__ bool locate(const TileMap& map, u32& limb, u32& tile)
   return false;
 }
 
+template <int EPI>
+struct MultiArg {};
+template <>
+struct MultiArg<4> {
+  NttMulti m;
+};
+
 template <bool INV, int EPI>
 __global__ void __launch_bounds__(kThreads, 6)
 ntt_contig_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, TileMap map,
                   const Twiddle* __restrict__ tables, const DevModulus* __restrict__ mods, uint32_t n,
-                  int logn, NttEpi epi) {
+                  int logn, NttEpi epi, const __grid_constant__ MultiArg<EPI> multi) {
   // 16 KiB for the blocks and up to 2 KiB to align them
   __shared__ u64 sm[kThreads / 16 * kContigBlock + kContigBlock];
   u32              limb, tile;
@@ -715,19 +723,25 @@ ntt_contig_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, Ti
   const int        per    = is_int ? 32 : 16;  // lanes per block
   const int        slot = threadIdx.x / per, t = threadIdx.x & (per - 1);
   const u32        to     = tile * (kThreads / per) + slot;  // block of the result
-  const uint32_t*  perm   = EPI == 3 ? epi.perm + (size_t)to * kContigBlock : nullptr;
-  const u32        blk    = EPI == 3 ? __ldg(perm) / kContigBlock : to;
+  const uint32_t*  perm   = nullptr;
+  if (EPI == 3) perm = epi.perm;
+  if constexpr (EPI == 4) perm = multi.m.perm[lr.sel];
+  if (perm != nullptr) perm += (size_t)to * kContigBlock;
+  const u32        blk    = EPI >= 3 && perm != nullptr ? __ldg(perm) / kContigBlock : to;
   const size_t     off    = (size_t)blk * kContigBlock;
-  const u64*       src    = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + off;
-  u64*             dst    = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n +
-                            (size_t)to * kContigBlock;
+  const bool       two    = EPI != 4;
+  const u64*       src    = (two && (lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + off;
+  u64*             dst    = two && (lr.sel & 4) ? out.p[1] : out.p[0];
+  if constexpr (EPI == 4) dst = multi.m.out[lr.sel];
+  dst += (size_t)lr.dst * n + (size_t)to * kContigBlock;
   const u64* aux = nullptr;
   const u64* add = nullptr;
   if (EPI != 0) {
     const size_t aoff = (size_t)lr.b * n + off;
-    aux = ((lr.sel & 2) ? epi.aux.p[1] : epi.aux.p[0]) + aoff;
+    aux = (two && (lr.sel & 2) ? epi.aux.p[1] : epi.aux.p[0]) + aoff;
     add = (lr.sel & 2) ? epi.add.p[1] : epi.add.p[0];
-    if (add != nullptr) add += aoff;
+    if constexpr (EPI == 4) add = multi.m.add[lr.sel];
+    if (add != nullptr) add += two ? aoff : (size_t)lr.dst * n + off;
   }
   const Twiddle* emul  = EPI != 0 ? epi.mul + lr.prime : nullptr;
   const size_t   entry = ((size_t)1 << s1) + (size_t)blk * kContigTable;
@@ -807,14 +821,16 @@ __device__ __forceinline__ void strided_inv(typename A::V (&x)[1 << E], u64* sm,
   }
 }
 
-template <class A, int E>
+// (the prologue is a template parameter: its code in a kernel that does not use
+// it cost 2 us a launch)
+template <class A, int E, int PRO>
 __device__ __forceinline__ void load_values(typename A::V (&x)[1 << E], const u64 (&v)[1 << E],
                                             const A& ar, const NttPro& pro, int prime) {
-  if (pro.kind == 1) {
+  if constexpr (PRO == 1) {
     const typename A::Lift lift = ar.make_lift(pro, prime);
 #pragma unroll
     for (int e = 0; e < (1 << E); e++) x[e] = ar.lift(v[e], lift);
-  } else if (pro.kind == 2) {
+  } else if constexpr (PRO == 2) {
     const bool          scaled = pro.mul != nullptr;
     const typename A::T w      = scaled ? ar.constant(pro.mul + prime) : typename A::T{};
 #pragma unroll
@@ -825,7 +841,7 @@ __device__ __forceinline__ void load_values(typename A::V (&x)[1 << E], const u6
   }
 }
 
-template <bool INV, int E, int S1, int TC, class A>
+template <bool INV, int PRO, int E, int S1, int TC, class A>
 __device__ __forceinline__ void strided_body(const u64* src, u64* dst, u64* sm, const Twiddle* table,
                                              const A& ar, const Twiddle* fin, const NttPro& pro,
                                              int prime) {
@@ -841,7 +857,7 @@ __device__ __forceinline__ void strided_body(const u64* src, u64* dst, u64* sm, 
     u64 v[1 << E];
 #pragma unroll
     for (int e = 0; e < (1 << E); e++) v[e] = src[(size_t)(at_top | (e << top)) << kContigLog];
-    load_values<A, E>(x, v, ar, pro, prime);
+    load_values<A, E, PRO>(x, v, ar, pro, prime);
     strided_fwd<A, E, S1, TC, 0>(x, sm, g, c, tw, ar);
 #pragma unroll
     for (int e = 0; e < (1 << E); e++) dst[(size_t)(at_low | e) << kContigLog] = A::bits(x[e]);
@@ -857,7 +873,7 @@ __device__ __forceinline__ void strided_body(const u64* src, u64* dst, u64* sm, 
 // columns per CTA: kThreads threads at every ring degree
 __host__ __device__ constexpr int tile_columns(int s1, int e) { return kThreads >> (s1 - e); }
 
-template <bool INV, int S1>
+template <bool INV, int PRO, int S1>
 __global__ void __launch_bounds__(kThreads, 7)
 ntt_strided_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, TileMap map,
                    const Twiddle* __restrict__ tables, const DevModulus* __restrict__ mods,
@@ -874,11 +890,11 @@ ntt_strided_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, T
   const u64*       src    = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + col;
   u64*             dst    = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n + col;
   if (!is_int)
-    strided_body<INV, 4, S1, TF>(src, dst, sm, tab, ArithFp(dm), fin, pro, lr.prime);
+    strided_body<INV, PRO, 4, S1, TF>(src, dst, sm, tab, ArithFp(dm), fin, pro, lr.prime);
   else if (dm.kind == kNttNarrow)
-    strided_body<INV, 3, S1, TI>(src, dst, sm, tab, ArithInt<false>(dm), fin, pro, lr.prime);
+    strided_body<INV, PRO, 3, S1, TI>(src, dst, sm, tab, ArithInt<false>(dm), fin, pro, lr.prime);
   else
-    strided_body<INV, 3, S1, TI>(src, dst, sm, tab, ArithInt<true>(dm), fin, pro, lr.prime);
+    strided_body<INV, PRO, 3, S1, TI>(src, dst, sm, tab, ArithInt<true>(dm), fin, pro, lr.prime);
 }
 
 // ---- whole limb in one CTA (512 <= N <= 4096) ------------------------------------
@@ -886,7 +902,7 @@ ntt_strided_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, T
 // S1 = logN - 8 stages in one register round over the top bits, then the
 // contiguous rounds; N/16 threads.
 
-template <bool INV, int EPI, int S1, class A>
+template <bool INV, int PRO, int EPI, int S1, class A>
 __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, const Twiddle* table,
                                            const DevModulus& dm, const Twiddle* fin,
                                            const NttPro& pro, int prime, const u64* aux,
@@ -904,7 +920,7 @@ __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, co
     u64 v[16];
 #pragma unroll
     for (int e = 0; e < 16; e++) v[e] = src[g | (e << top)];
-    load_values<A, 4>(x, v, ar, pro, prime);
+    load_values<A, 4, PRO>(x, v, ar, pro, prime);
     fwd_stages<A, 4, S1, 0>(x, TreeTw<A>{tree, 1u}, ar);
 #pragma unroll
     for (int e = 0; e < 16; e++) sm[at(g | (e << top))] = A::bits(x[e]);
@@ -916,7 +932,7 @@ __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, co
     typename A::T w{};
     if (EPI != 0) w = ar.constant(emul);
     const size_t off = (size_t)half * kContigBlock;
-    if constexpr (EPI != 3) {
+    if (EPI < 3 || perm == nullptr) {
       write_block16<A, EPI>(dst + off, sb, t, aux + off, add != nullptr ? add + off : nullptr, w, ar,
                             nullptr);
     } else {
@@ -944,36 +960,44 @@ __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, co
   }
 }
 
-template <bool INV, int EPI, int S1>
+template <bool INV, int PRO, int EPI, int S1>
 __global__ void __launch_bounds__(16 << S1)
 ntt_whole_kernel(Ptr2 in, Ptr2 out, LimbBatch batch, const Twiddle* __restrict__ tables,
                  const DevModulus* __restrict__ mods, const Twiddle* __restrict__ inv_last,
-                 NttPro pro, NttEpi epi) {
+                 NttPro pro, NttEpi epi, const __grid_constant__ MultiArg<EPI> multi) {
   constexpr uint32_t n = (uint32_t)kContigBlock << S1;
   __shared__ u64 sm[n];
   const LimbRef    lr  = batch.limb[blockIdx.x];
   const DevModulus dm  = mods[lr.prime];
   const Twiddle*   tab = tables + (size_t)lr.prime * table_entries(S1 + kContigLog);
   const Twiddle*   fin = inv_last + (size_t)lr.prime * 2;
-  const u64*       src = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n;
-  u64*             dst = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n;
+  const bool       two = EPI != 4;
+  const u64*       src = (two && (lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n;
+  u64*             dst = two && (lr.sel & 4) ? out.p[1] : out.p[0];
+  const uint32_t*  perm = EPI == 3 ? epi.perm : nullptr;
   const u64* aux = nullptr;
   const u64* add = nullptr;
   if (EPI != 0) {
-    aux = ((lr.sel & 2) ? epi.aux.p[1] : epi.aux.p[0]) + (size_t)lr.b * n;
+    aux = (two && (lr.sel & 2) ? epi.aux.p[1] : epi.aux.p[0]) + (size_t)lr.b * n;
     add = (lr.sel & 2) ? epi.add.p[1] : epi.add.p[0];
-    if (add != nullptr) add += (size_t)lr.b * n;
+    if constexpr (EPI == 4) add = multi.m.add[lr.sel];
+    if (add != nullptr) add += (size_t)(two ? lr.b : lr.dst) * n;
   }
+  if constexpr (EPI == 4) {
+    dst  = multi.m.out[lr.sel];
+    perm = multi.m.perm[lr.sel];
+  }
+  dst += (size_t)lr.dst * n;
   const Twiddle* emul = EPI != 0 ? epi.mul + lr.prime : nullptr;
   if (dm.kind == kNttFloat)
-    whole_body<INV, EPI, S1, ArithFp>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
-                                       epi.perm);
+    whole_body<INV, PRO, EPI, S1, ArithFp>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
+                                       perm);
   else if (dm.kind == kNttNarrow)
-    whole_body<INV, EPI, S1, ArithInt<false>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
-                                       epi.perm);
+    whole_body<INV, PRO, EPI, S1, ArithInt<false>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
+                                       perm);
   else
-    whole_body<INV, EPI, S1, ArithInt<true>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
-                                       epi.perm);
+    whole_body<INV, PRO, EPI, S1, ArithInt<true>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
+                                       perm);
 }
 
 // ---- tiny transforms (N < 512): one butterfly at a time --------------------------
@@ -1021,70 +1045,92 @@ struct NttTables {
 };
 
 // n_int: how many limbs, at the front of the batch, are transformed in integers
-template <bool INV, int S1>
+template <bool INV, int PRO, int S1>
 inline void launch_strided_t(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
                              cudaStream_t stream, const NttPro& pro) {
   const TileMap map{(u32)n_int, (u32)(kContigLog - floor_log2(tile_columns(S1, 3))),
                     (u32)(kContigLog - floor_log2(tile_columns(S1, 4)))};
   const int     ctas = (n_int << map.log_int) + ((b.count - n_int) << map.log_float);
-  launch(ntt_strided_kernel<INV, S1>, ctas, kThreads, 0, stream, in, out, b, map,
+  launch(ntt_strided_kernel<INV, PRO, S1>, ctas, kThreads, 0, stream, in, out, b, map,
          INV ? t.inv : t.fwd, t.mods, t.inv_last, t.n, pro);
 }
 
-template <bool INV>
-inline void launch_strided(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
-                           cudaStream_t stream, const NttPro& pro = NttPro()) {
+template <bool INV, int PRO>
+inline void launch_strided_p(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
+                             cudaStream_t stream, const NttPro& pro) {
   switch (t.logn - kContigLog) {
-    case 5: launch_strided_t<INV, 5>(in, out, b, n_int, t, stream, pro); break;
-    case 6: launch_strided_t<INV, 6>(in, out, b, n_int, t, stream, pro); break;
-    case 7: launch_strided_t<INV, 7>(in, out, b, n_int, t, stream, pro); break;
-    case 8: launch_strided_t<INV, 8>(in, out, b, n_int, t, stream, pro); break;
-    case 9: launch_strided_t<INV, 9>(in, out, b, n_int, t, stream, pro); break;
+    case 5: launch_strided_t<INV, PRO, 5>(in, out, b, n_int, t, stream, pro); break;
+    case 6: launch_strided_t<INV, PRO, 6>(in, out, b, n_int, t, stream, pro); break;
+    case 7: launch_strided_t<INV, PRO, 7>(in, out, b, n_int, t, stream, pro); break;
+    case 8: launch_strided_t<INV, PRO, 8>(in, out, b, n_int, t, stream, pro); break;
+    case 9: launch_strided_t<INV, PRO, 9>(in, out, b, n_int, t, stream, pro); break;
     default: FHERT_ASSERT(false, "ring degree 2^%d has no transform kernel", t.logn);
   }
 }
 
 template <bool INV>
+inline void launch_strided(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
+                           cudaStream_t stream, const NttPro& pro = NttPro()) {
+  if (INV || pro.kind == 0) launch_strided_p<INV, 0>(in, out, b, n_int, t, stream, pro);
+  else if (pro.kind == 1) launch_strided_p<false, 1>(in, out, b, n_int, t, stream, pro);
+  else launch_strided_p<false, 2>(in, out, b, n_int, t, stream, pro);
+}
+
+template <bool INV>
 inline void launch_contig(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, const NttTables& t,
-                          cudaStream_t stream, const NttEpi& epi = NttEpi()) {
+                          cudaStream_t stream, const NttEpi& epi = NttEpi(),
+                          const NttMulti* multi = nullptr) {
   const u32      blocks = (u32)(t.logn - kContigLog);
   const TileMap  map{(u32)n_int, blocks - floor_log2(kThreads / 32), blocks - floor_log2(kThreads / 16)};
   const int      ctas = (n_int << map.log_int) + ((b.count - n_int) << map.log_float);
   const Twiddle* tab  = INV ? t.inv : t.fwd;
   if (INV || epi.kind == 0)
     launch(ntt_contig_kernel<INV, 0>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
-           t.logn, epi);
+           t.logn, epi, MultiArg<0>{});
   else if (epi.kind == 1)
     launch(ntt_contig_kernel<false, 1>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
-           t.logn, epi);
+           t.logn, epi, MultiArg<1>{});
+  else if (epi.kind == 4)
+    launch(ntt_contig_kernel<false, 4>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
+           t.logn, epi, MultiArg<4>{*multi});
   else if (epi.kind == 3)
     launch(ntt_contig_kernel<false, 3>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
-           t.logn, epi);
+           t.logn, epi, MultiArg<3>{});
   else
     launch(ntt_contig_kernel<false, 2>, ctas, kThreads, 0, stream, in, out, b, map, tab, t.mods, t.n,
-           t.logn, epi);
+           t.logn, epi, MultiArg<2>{});
 }
 
-template <bool INV, int EPI>
+template <bool INV, int PRO, int EPI>
 inline void launch_whole_t(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
-                           cudaStream_t stream, const NttPro& pro, const NttEpi& epi) {
+                           cudaStream_t stream, const NttPro& pro, const NttEpi& epi,
+                           const MultiArg<EPI>& multi) {
   const Twiddle* tab = INV ? t.inv : t.fwd;
+#define WHOLE_CASE(S1_)                                                                           \
+  launch(ntt_whole_kernel<INV, PRO, EPI, S1_>, b.count, 16 << S1_, 0, stream, in, out, b, tab, t.mods, \
+         t.inv_last, pro, epi, multi)
   switch (t.logn - kContigLog) {
-    case 1: launch(ntt_whole_kernel<INV, EPI, 1>, b.count, 32, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
-    case 2: launch(ntt_whole_kernel<INV, EPI, 2>, b.count, 64, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
-    case 3: launch(ntt_whole_kernel<INV, EPI, 3>, b.count, 128, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
-    default: launch(ntt_whole_kernel<INV, EPI, 4>, b.count, 256, 0, stream, in, out, b, tab, t.mods, t.inv_last, pro, epi); break;
+    case 1: WHOLE_CASE(1); break;
+    case 2: WHOLE_CASE(2); break;
+    case 3: WHOLE_CASE(3); break;
+    default: WHOLE_CASE(4); break;
   }
+#undef WHOLE_CASE
 }
 
 template <bool INV>
 inline void launch_whole(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables& t,
                          cudaStream_t stream, const NttPro& pro = NttPro(),
-                         const NttEpi& epi = NttEpi()) {
-  if (INV || epi.kind == 0) launch_whole_t<INV, 0>(in, out, b, t, stream, pro, epi);
-  else if (epi.kind == 1) launch_whole_t<false, 1>(in, out, b, t, stream, pro, epi);
-  else if (epi.kind == 3) launch_whole_t<false, 3>(in, out, b, t, stream, pro, epi);
-  else launch_whole_t<false, 2>(in, out, b, t, stream, pro, epi);
+                         const NttEpi& epi = NttEpi(), const NttMulti* multi = nullptr) {
+  // a lift comes with a rescale's last step, a message with none
+  FHERT_ASSERT(pro.kind == 0 || (pro.kind == 1 && epi.kind == 1) || (pro.kind == 2 && epi.kind == 0),
+               "no transform with prologue %d and epilogue %d", pro.kind, epi.kind);
+  if (pro.kind == 1) launch_whole_t<false, 1, 1>(in, out, b, t, stream, pro, epi, MultiArg<1>{});
+  else if (pro.kind == 2) launch_whole_t<false, 2, 0>(in, out, b, t, stream, pro, epi, MultiArg<0>{});
+  else if (INV || epi.kind == 0) launch_whole_t<INV, 0, 0>(in, out, b, t, stream, pro, epi, MultiArg<0>{});
+  else if (epi.kind == 3) launch_whole_t<false, 0, 3>(in, out, b, t, stream, pro, epi, MultiArg<3>{});
+  else if (epi.kind == 4) launch_whole_t<false, 0, 4>(in, out, b, t, stream, pro, epi, MultiArg<4>{*multi});
+  else launch_whole_t<false, 0, 2>(in, out, b, t, stream, pro, epi, MultiArg<2>{});
 }
 
 template <bool INV>

@@ -89,27 +89,6 @@ automorphism_kernel(Ptr2 res, Ptr2 val, const uint32_t* __restrict__ table, Limb
     pr[i] = pv[__ldg(table + i)];
 }
 
-// res[i] = val[table[i]] (+ add[table[i]] on limbs flagged with sel bit 1, the
-// addend limb index in lr.b): the "+ P*c0" of a hoisted rotation on the
-// extended basis, folded into the gather
-__global__ void __launch_bounds__(kThreads)
-automorphism_add_kernel(Ptr2 res, Ptr2 val, const u64* __restrict__ add,
-                        const uint32_t* __restrict__ table, LimbBatch batch,
-                        const DevModulus* __restrict__ mods, uint32_t n) {
-  const LimbRef lr  = batch.limb[blockIdx.y];
-  const u64*    pv  = sel_a(val, lr, n);
-  u64*          pr  = sel_d(res, lr, n);
-  const bool    has = (lr.sel & 2) != 0;
-  const u64*    pa  = add + (size_t)lr.b * n;
-  const u64     q   = mods[lr.prime].q;
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-    uint32_t t = __ldg(table + i);
-    u64      x = pv[t];
-    if (has) x = add_mod(x, pa[t], q);
-    pr[i] = x;
-  }
-}
-
 __global__ void __launch_bounds__(kThreads)
 mul_const_kernel(Ptr2 res, Ptr2 val, const Twiddle* __restrict__ consts, LimbBatch batch,
                  const DevModulus* __restrict__ mods, uint32_t n) {
@@ -248,92 +227,6 @@ rescale_coeff_kernel(Ptr2 res, Ptr2 x, int last, const Twiddle* __restrict__ ql_
     ri[k] = mul_shoup(sub_mod(xi[k], reduce_128(0, xl[k], md), md.q), wi.w, wi.wp, md.q);
 }
 
-// ---- key inner product (rns_poly.c:516, rns_poly_impl.c:13-160) --------------
-// One reduction per output word; two coefficients per thread (16-byte loads).
-
-// The kernel streams its operands once, so what it needs is bytes in flight:
-// the digits are taken U at a time and all operands of a group are loaded
-// before the first multiply; registers are capped for four resident CTAs per
-// SM.  EXACT: there are exactly U digits (the key switch: up to four); else
-// any number, in groups of U (a group that reaches past the last digit loads
-// nothing for the missing ones and multiplies zeros).
-template <bool TWO, bool FAST, int U, bool EXACT>
-__global__ void __launch_bounds__(kThreads, 4)
-inner_product_kernel(InnerArgs a, int num_q, const DevModulus* __restrict__ mods, uint32_t n) {
-  const int        m     = blockIdx.y;  // limb among level Q limbs then K P limbs
-  if ((a.skip_mask >> m) & 1) return;
-  const bool       is_q  = m < a.level;
-  const int        prime = is_q ? m : num_q + (m - a.level);
-  const DevModulus md    = mods[prime];
-  const size_t e_off = (size_t)(is_q ? m : a.ext_p_limb + (m - a.level)) * n;
-  const size_t k_off = (size_t)(is_q ? m : a.key_p_limb + (m - a.level)) * n;
-  const size_t d_off = (size_t)(is_q ? m : a.acc_p_limb + (m - a.level)) * n;
-  const int    own   = (a.in != nullptr && is_q) ? m / a.alpha : -1;
-  const uint32_t pairs = n >> 1;
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < pairs; i += gridDim.x * kThreads) {
-    Acc4 c00, c01, c10, c11;
-    u64  h[4] = {0, 0, 0, 0}, l[4] = {0, 0, 0, 0};
-    if (FAST) {
-      acc4_zero(c00);
-      acc4_zero(c01);
-      acc4_zero(c10);
-      acc4_zero(c11);
-    }
-#pragma unroll 1
-    for (int base = 0; base < (EXACT ? U : a.parts); base += U) {
-      ulonglong2 e[U], k0[U], k1[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int j = base + u;
-        if (!EXACT) e[u] = k0[u] = k1[u] = make_ulonglong2(0, 0);
-        if (EXACT || j < a.parts) {
-          const u64* es = (j == own) ? a.in + (size_t)m * n : a.ext_ptr[j] + e_off;
-          e[u]  = reinterpret_cast<const ulonglong2*>(es)[i];
-          // keys are read once per key switch: streamed past the L2 lines that the
-          // twiddle tables and the polynomials in flight should keep
-          k0[u] = __ldcs(reinterpret_cast<const ulonglong2*>(a.key0[j] + k_off) + i);
-          if (TWO) k1[u] = __ldcs(reinterpret_cast<const ulonglong2*>(a.key1[j] + k_off) + i);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        if (FAST) {
-          acc4_mac(c00, e[u].x, k0[u].x);
-          acc4_mac(c01, e[u].y, k0[u].y);
-          if (TWO) {
-            acc4_mac(c10, e[u].x, k1[u].x);
-            acc4_mac(c11, e[u].y, k1[u].y);
-          }
-        } else {
-          mac_128(h[0], l[0], e[u].x, k0[u].x);
-          mac_128(h[1], l[1], e[u].y, k0[u].y);
-          if (TWO) {
-            mac_128(h[2], l[2], e[u].x, k1[u].x);
-            mac_128(h[3], l[3], e[u].y, k1[u].y);
-          }
-        }
-      }
-    }
-    if (FAST) {
-      acc4_fold(c00, h[0], l[0]);
-      acc4_fold(c01, h[1], l[1]);
-      if (TWO) {
-        acc4_fold(c10, h[2], l[2]);
-        acc4_fold(c11, h[3], l[3]);
-      }
-    }
-    ulonglong2 r;
-    r.x = reduce_128(h[0], l[0], md);
-    r.y = reduce_128(h[1], l[1], md);
-    reinterpret_cast<ulonglong2*>(a.acc0 + d_off)[i] = r;
-    if (TWO) {
-      r.x = reduce_128(h[2], l[2], md);
-      r.y = reduce_128(h[3], l[3], md);
-      reinterpret_cast<ulonglong2*>(a.acc1 + d_off)[i] = r;
-    }
-  }
-}
-
 // ---- mod-raise (rns_poly.c:1101-1125) ----------------------------------------
 
 __global__ void __launch_bounds__(kThreads)
@@ -411,23 +304,6 @@ void launch_automorphism(Ptr2 res, Ptr2 val, const uint32_t* table, const LimbBa
   prof_before(KID_AUTOMORPHISM);
   launch(automorphism_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
          res, val, table, batch, c->N);
-  after_launch(c, KID_AUTOMORPHISM, batch.count);
-}
-
-void launch_automorphism_add(Ptr2 res, Ptr2 val, const int64_t* add, const uint32_t* table,
-                             const LimbBatch& batch) {
-  if (batch.count == 0) return;
-  Context* c = ctx();
-  DagScope dag(DAG_AUTOMORPHISM);
-  dag.batch(batch, c->N, &res, &val, nullptr);
-  if (dag.live)
-    for (int i = 0; i < batch.count; i++)
-      if (batch.limb[i].sel & 2)
-        dag.set.read(add + (size_t)batch.limb[i].b * c->N, (size_t)c->N * sizeof(int64_t));
-  dag.commit();
-  prof_before(KID_AUTOMORPHISM);
-  launch(automorphism_add_kernel, grid_for(c->N, 2, batch.count), kThreads, 0, c->stream,
-         res, val, reinterpret_cast<const u64*>(add), table, batch, c->d_mod, c->N);
   after_launch(c, KID_AUTOMORPHISM, batch.count);
 }
 
@@ -515,55 +391,6 @@ void launch_rescale_coeff(Ptr2 res, Ptr2 x, int polys, int level) {
   launch(rescale_coeff_kernel, grid_for(c->N, 2, polys * last), kThreads, 0, c->stream,
          res, x, last, c->d_ql_inv + (size_t)last * c->L, c->d_mod, c->N);
   after_launch(c, KID_RESCALE_COMBINE, polys * last);
-}
-
-void launch_inner_product(const InnerArgs& args) {
-  Context* c     = ctx();
-  int      limbs = args.level + c->K;
-  FHERT_ASSERT(args.parts >= 1 && args.parts <= kMaxParts, "unsupported digit count");
-  DagScope dag(DAG_INNER_PRODUCT);
-  if (dag.live) {
-    const size_t n = c->N, w = n * sizeof(u64);
-    for (int m = 0; m < limbs; m++) {
-      if ((args.skip_mask >> m) & 1) continue;
-      const bool   is_q  = m < args.level;
-      const size_t e_off = (size_t)(is_q ? m : args.ext_p_limb + (m - args.level)) * n;
-      const size_t k_off = (size_t)(is_q ? m : args.key_p_limb + (m - args.level)) * n;
-      const size_t d_off = (size_t)(is_q ? m : args.acc_p_limb + (m - args.level)) * n;
-      const int    own   = (args.in != nullptr && is_q) ? m / args.alpha : -1;
-      for (int j = 0; j < args.parts; j++) {
-        dag.set.read(j == own ? args.in + (size_t)m * n : args.ext_ptr[j] + e_off, w);
-        // the "key" operands are switching keys in a key switch, but rotated
-        // ciphertext polynomials in the baby-step sums of the bootstrap
-        dag.set.read(args.key0[j] + k_off, w);
-        if (args.acc1 != nullptr) dag.set.read(args.key1[j] + k_off, w);
-      }
-      dag.set.write(args.acc0 + d_off, w);
-      if (args.acc1 != nullptr) dag.set.write(args.acc1 + d_off, w);
-    }
-  }
-  dag.commit();
-  prof_before(KID_INNER_PRODUCT);
-  dim3 g    = grid_for(c->N, 4, limbs);
-  bool fast = c->primes_below_2_60;
-  bool two  = args.acc1 != nullptr;
-#define IP_CASE(TWO_, FAST_, U_, EXACT_)                                                       \
-  launch(inner_product_kernel<TWO_, FAST_, U_, EXACT_>, g, kThreads, 0, c->stream, args, c->L, c->d_mod, c->N)
-#define IP_GROUPS(TWO_, FAST_)                                 \
-  do {                                                         \
-    if (args.parts == 1) IP_CASE(TWO_, FAST_, 1, true);        \
-    else if (args.parts == 2) IP_CASE(TWO_, FAST_, 2, true);   \
-    else if (args.parts == 3) IP_CASE(TWO_, FAST_, 3, true);   \
-    else if (args.parts == 4) IP_CASE(TWO_, FAST_, 4, true);   \
-    else IP_CASE(TWO_, FAST_, 2, false);                       \
-  } while (0)
-  if (two && fast) IP_GROUPS(true, true);
-  else if (two) IP_GROUPS(true, false);
-  else if (fast) IP_GROUPS(false, true);
-  else IP_GROUPS(false, false);
-#undef IP_GROUPS
-#undef IP_CASE
-  after_launch(c, KID_INNER_PRODUCT, limbs);
 }
 
 void launch_mod_raise(int64_t* res, const int64_t* src, const LimbBatch& batch) {

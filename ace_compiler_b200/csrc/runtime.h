@@ -237,6 +237,7 @@ u64  shoup(u64 w, u64 q);
 const Context::ModUpTable& modup_table(Context* c, int level, int digit);
 const Twiddle* modup_last(Context* c, int level);
 uint32_t* auto_table(Context* c, uint32_t k);
+uint32_t  inverse_mod_2n(uint32_t v, uint32_t n);
 
 // ---- sampling.cu (host randomness, same generators as the CPU runtime) ----
 void seed_prng(const uint32_t seed[16], u64 counter, int64_t fake_time_us);
@@ -478,6 +479,14 @@ void launch_ntt(Ptr2 in, Ptr2 out, const LimbBatch& b, bool inverse, const Twidd
 //             kind 3  kind 2, then permuted: out[i] = value[perm[i]]; `out` may not
 //                     overlap anything that is read
 //     aux / add use base p[sel bit 1]
+// kind 4: kind 2 or 3 on many polynomials at once; sel is the polynomial, whose
+// result, addend and permutation (null: none) stand here
+constexpr int kMaxMulti = 16;
+struct NttMulti {
+  u64*            out[kMaxMulti];
+  const u64*      add[kMaxMulti];
+  const uint32_t* perm[kMaxMulti];
+};
 struct NttFuse {
   int            pro_kind = 0;
   const Twiddle* pro_mul = nullptr;
@@ -488,6 +497,7 @@ struct NttFuse {
   Ptr2           aux{{nullptr, nullptr}};
   Ptr2           add{{nullptr, nullptr}};
   const uint32_t* perm    = nullptr;
+  const NttMulti* multi   = nullptr;
 };
 bool ntt_can_fuse();
 void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const NttFuse& f);
@@ -502,10 +512,6 @@ void launch_elementwise(EwOp op, Ptr2 res, Ptr2 a, Ptr2 b, int64_t scalar,
 void launch_scalars(bool mul, Ptr2 res, Ptr2 a, const u64* per_limb, const LimbBatch& batch);
 // res[dst][i] = val[a][table[i]]
 void launch_automorphism(Ptr2 res, Ptr2 val, const uint32_t* table, const LimbBatch& batch);
-// res[dst][i] = val[a][table[i]] + add[b][table[i]] on limbs whose sel has bit 1
-// set (b indexes limbs of `add`), plain gather on the others
-void launch_automorphism_add(Ptr2 res, Ptr2 val, const int64_t* add, const uint32_t* table,
-                             const LimbBatch& batch);
 // res[dst] = val[a] * consts[prime]
 void launch_mul_const(Ptr2 res, Ptr2 val, const Twiddle* consts, const LimbBatch& batch);
 // tensor product of two ciphertexts (evaluator.c:137-173), one launch:
@@ -597,6 +603,44 @@ struct InnerArgs {
   int        ext_p_limb;  // limb index of the first P limb in ext
 };
 void launch_inner_product(const InnerArgs& args);
+// The digits of one polynomial (digit j at digits + j * digit_stride, level Q
+// limbs then K special limbs; a digit's own limbs come from `in`) against the
+// keys of up to kMaxKeys rotations, for every limb m:
+//   (v0, v1) = sum_j e_j * (key0[r][j], key1[r][j])
+//   v0 += c0[m], times P mod q_m when p_mod_q is given (then only on Q limbs)
+//   out_r[place_r[i]] = v[i]     (place null: out_r[i]; accumulate: added there)
+// with out_r = out + r * out_stride, its second polynomial poly_stride behind.
+constexpr int kMaxKeys = 16;
+struct KeysArgs {
+  int             parts, level, alpha, key_p_limb, count;
+  bool            accumulate;
+  const u64*      in;
+  const u64*      digits;
+  size_t          digit_stride;
+  const u64*      c0;
+  const Twiddle*  p_mod_q;
+  u64*            out;
+  size_t          out_stride, poly_stride;
+  const uint32_t* place[kMaxKeys];
+  const u64*      key0[kMaxKeys][kMaxParts];
+  const u64*      key1[kMaxKeys][kMaxParts];
+};
+void launch_keys_product(const KeysArgs& args);
+// Up to kMaxSums sums out_i = sum_j rot_j * plain[i][j] (null plaintexts left out)
+// of both polynomials of `terms` extended ciphertexts; strides as above.
+constexpr int kMaxSums = 4;
+struct SumsArgs {
+  struct Plain {
+    const u64* data;
+    int        p_limb;  // its first special limb
+  };
+  int        level, terms, sums;
+  const u64* rot;
+  u64*       out;
+  size_t     rot_stride, out_stride, poly_stride;
+  Plain      plain[kMaxSums][kMaxParts];
+};
+void launch_weighted_sums(const SumsArgs& args);
 // Mod-raise (rns_poly.c:1101-1125): res[dst] = switch_modulus(src, q_0 -> q_i)
 void launch_mod_raise(int64_t* res, const int64_t* src, const LimbBatch& batch);
 
@@ -646,6 +690,12 @@ void fhert_mod_down_polys(fhert::Context* c, int npoly, int64_t* const res[2],
                           const int64_t* const ext[2], int ext_p_limb,
                           const int64_t* const add[2], size_t level, bool is_ntt,
                           const uint32_t* perm = nullptr);
+// ModDown of `polys` extended polynomials in NTT form that stand ext_stride limbs
+// apart (special limbs at ext_p_limb of each), with results, addends and
+// permutations of their own; polys <= fhert_mod_down_many_limit(level)
+void fhert_mod_down_many(fhert::Context* c, int polys, const int64_t* ext, size_t ext_stride,
+                         int ext_p_limb, size_t level, const fhert::NttMulti& to);
+int  fhert_mod_down_many_limit(fhert::Context* c, size_t level);  // 0: not for this ring
 // Rescale of one or two NTT-form polynomials from level to level - 1
 void fhert_rescale_polys(fhert::Context* c, int npoly, int64_t* const res[2],
                          const int64_t* const poly[2], size_t level);
