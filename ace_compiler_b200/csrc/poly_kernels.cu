@@ -5,6 +5,7 @@
 // walks the N coefficients of a limb, the y dimension the limbs.
 #include <algorithm>
 
+#include "ntt_kernels.cuh"
 #include "runtime.h"
 
 namespace fhert {
@@ -30,32 +31,78 @@ __device__ __forceinline__ u64* sel_d(const Ptr2& p, const LimbRef& lr, uint32_t
 
 // ---- element-wise (hal/src/hal.c:15-121, poly/src/rns_poly.c:852-1054) ------
 
+// What bounds these kernels is bytes in flight: every thread issues the loads of
+// two 16-byte words per operand before the first result.  With one 8-byte word at
+// a time and integer products throughout, the 9 products and 8 sums of a
+// convolution row at N = 65536 took 185 us, this way 140.  A limb has at least
+// four coefficients, so whole words always fit.
+constexpr int kWords = 2;  // 16-byte words per thread
+
+inline dim3 grid_words(uint32_t n, int limbs) {
+  const uint32_t per_block = kThreads * kWords * 2;
+  return dim3((n + per_block - 1) / per_block, limbs);
+}
+struct WordLoop {  // the words of this thread
+  uint32_t at[kWords];
+  bool     in[kWords];
+  __device__ __forceinline__ explicit WordLoop(uint32_t n) {
+#pragma unroll
+    for (int k = 0; k < kWords; k++) {
+      at[k] = (blockIdx.x * kWords + k) * kThreads + threadIdx.x;
+      in[k] = at[k] < n / 2;
+    }
+  }
+  __device__ __forceinline__ void load(ulonglong2 (&v)[kWords], const u64* p) const {
+#pragma unroll
+    for (int k = 0; k < kWords; k++)
+      v[k] = in[k] ? reinterpret_cast<const ulonglong2*>(p)[at[k]] : make_ulonglong2(0, 0);
+  }
+};
+
+// a * b mod q on the pipe the prime allows
+struct Product {
+  const DevModulus& m;
+  nttk::ArithFp     fp;
+  __device__ __forceinline__ explicit Product(const DevModulus& md) : m(md), fp(md) {}
+  __device__ __forceinline__ u64 operator()(u64 a, u64 b) const {
+    return m.kind == kNttFloat ? fp.word(fp.mul(nttk::ArithFp::load(a), nttk::ArithFp::load(b)))
+                               : mul_mod(a, b, m);
+  }
+};
+
 template <int OP>
 __global__ void __launch_bounds__(kThreads)
-ew_kernel(Ptr2 res, Ptr2 a, Ptr2 b, u64 scalar, LimbBatch batch,
+ew_kernel(Ptr2 res, Ptr2 a, Ptr2 b, u64 scalar, const __grid_constant__ LimbBatch batch,
           const DevModulus* __restrict__ mods, uint32_t n) {
+  constexpr bool   two  = OP == EW_ADD || OP == EW_SUB || OP == EW_MUL || OP == EW_MULADD;
+  constexpr bool   accu = OP == EW_MULADD || OP == EW_MULADD_SCALAR;
   const LimbRef    lr = batch.limb[blockIdx.y];
   const DevModulus m  = mods[lr.prime];
-  const u64*       pa = sel_a(a, lr, n);
-  const u64*       pb = sel_b(b, lr, n);
   u64*             pr = sel_d(res, lr, n);
   u64              sc = 0;
-  if (OP == EW_ADD_SCALAR || OP == EW_MUL_SCALAR || OP == EW_MULADD_SCALAR) {
+  if (!two) {
     // scalars arrive as signed 64-bit values; bring into [0, q)
     int64_t s = (int64_t)scalar % (int64_t)m.q;
     sc        = s < 0 ? (u64)(s + (int64_t)m.q) : (u64)s;
   }
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-    u64 x = pa[i], r;
-    if (OP == EW_ADD) r = add_mod(x, pb[i], m.q);
-    else if (OP == EW_SUB) r = sub_mod(x, pb[i], m.q);
-    else if (OP == EW_MUL) r = mul_mod(x, pb[i], m);
-    else if (OP == EW_MULADD) r = add_mod(pr[i], mul_mod(x, pb[i], m), m.q);
-    else if (OP == EW_ADD_SCALAR) r = add_mod(x, sc, m.q);
-    else if (OP == EW_MULADD_SCALAR) r = add_mod(pr[i], mul_mod(x, sc, m), m.q);
-    else r = mul_mod(x, sc, m);
-    pr[i] = r;
-  }
+  const WordLoop words(n);
+  ulonglong2     x[kWords], y[kWords], r[kWords];
+  words.load(x, sel_a(a, lr, n));
+  if (two) words.load(y, sel_b(b, lr, n));
+  if (accu) words.load(r, pr);
+  const Product mul(m);
+  auto one = [&](u64 x, u64 y, u64 r) {
+    if (!two) y = sc;
+    if (OP == EW_ADD || OP == EW_ADD_SCALAR) return add_mod(x, y, m.q);
+    if (OP == EW_SUB) return sub_mod(x, y, m.q);
+    const u64 p = mul(x, y);
+    return accu ? add_mod(r, p, m.q) : p;
+  };
+#pragma unroll
+  for (int k = 0; k < kWords; k++)
+    if (words.in[k])
+      reinterpret_cast<ulonglong2*>(pr)[words.at[k]] =
+          make_ulonglong2(one(x[k].x, y[k].x, r[k].x), one(x[k].y, y[k].y, r[k].y));
 }
 
 // one reduced scalar per limb of the batch, passed by value
@@ -66,15 +113,22 @@ struct ScalarList {
 
 template <bool MUL>
 __global__ void __launch_bounds__(kThreads)
-ew_scalars_kernel(Ptr2 res, Ptr2 a, ScalarList sc, LimbBatch batch,
-                  const DevModulus* __restrict__ mods, uint32_t n) {
+ew_scalars_kernel(Ptr2 res, Ptr2 a, const __grid_constant__ ScalarList sc,
+                  const __grid_constant__ LimbBatch batch, const DevModulus* __restrict__ mods,
+                  uint32_t n) {
   const LimbRef    lr = batch.limb[blockIdx.y];
   const DevModulus m  = mods[lr.prime];
   const u64        s  = sc.v[blockIdx.y];
-  const u64*       pa = sel_a(a, lr, n);
   u64*             pr = sel_d(res, lr, n);
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
-    pr[i] = MUL ? mul_mod(pa[i], s, m) : add_mod(pa[i], s, m.q);
+  const WordLoop   words(n);
+  ulonglong2       x[kWords];
+  words.load(x, sel_a(a, lr, n));
+  const Product mul(m);
+  auto one = [&](u64 v) { return MUL ? mul(v, s) : add_mod(v, s, m.q); };
+#pragma unroll
+  for (int k = 0; k < kWords; k++)
+    if (words.in[k])
+      reinterpret_cast<ulonglong2*>(pr)[words.at[k]] = make_ulonglong2(one(x[k].x), one(x[k].y));
 }
 
 // ---- automorphism in NTT form: a pure gather (hal.c:123-138) ----------------
@@ -102,25 +156,46 @@ mul_const_kernel(Ptr2 res, Ptr2 val, const Twiddle* __restrict__ consts, LimbBat
 }
 
 // ---- tensor product (ckks/src/evaluator.c:137-173) ---------------------------
-// limb index = prime index = blockIdx.y; the middle term is summed in 128 bits
-// and reduced once.
+// limb index = prime index = blockIdx.y; the middle term is summed before its one
+// reduction.  Seven words move per coefficient; two coefficients per thread and
+// double-precision products where the prime allows.
 
 __global__ void __launch_bounds__(kThreads)
-tensor_kernel(u64* __restrict__ d0, u64* __restrict__ d1, u64* __restrict__ d2,
-              const u64* __restrict__ a0, const u64* __restrict__ a1,
-              const u64* __restrict__ b0, const u64* __restrict__ b1,
+tensor_kernel(u64* d0, u64* d1, u64* d2, const u64* a0, const u64* a1, const u64* b0, const u64* b1,
               const DevModulus* __restrict__ mods, uint32_t n, int first_prime) {
   const DevModulus m   = mods[first_prime + blockIdx.y];
-  const size_t     off = (size_t)blockIdx.y * n;
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-    u64 x0 = a0[off + i], x1 = a1[off + i], y0 = b0[off + i], y1 = b1[off + i];
-    d0[off + i] = mul_mod(x0, y0, m);
-    d2[off + i] = mul_mod(x1, y1, m);
-    u64 hi = 0, lo = 0;
-    mac_128(hi, lo, x0, y1);
-    mac_128(hi, lo, x1, y0);
-    d1[off + i] = reduce_128(hi, lo, m);
+  const size_t     off = (size_t)blockIdx.y * (n / 2);
+  const uint32_t   i   = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= n / 2) return;
+  typedef ulonglong2 w2;
+  const w2 x0 = reinterpret_cast<const w2*>(a0)[off + i], x1 = reinterpret_cast<const w2*>(a1)[off + i];
+  const w2 y0 = reinterpret_cast<const w2*>(b0)[off + i], y1 = reinterpret_cast<const w2*>(b1)[off + i];
+  w2 r0, r1, r2;
+  if (m.kind == kNttFloat) {
+    const nttk::ArithFp f(m);
+    auto                one = [&](u64 p0, u64 p1, u64 q0, u64 q1, u64& o0, u64& o1, u64& o2) {
+      const double u0 = f.load(p0), u1 = f.load(p1), v0 = f.load(q0), v1 = f.load(q1);
+      o0 = f.word(f.mul(u0, v0));
+      o2 = f.word(f.mul(u1, v1));
+      o1 = f.canon(__dadd_rn(f.mul(u0, v1), f.mul(u1, v0)));
+    };
+    one(x0.x, x1.x, y0.x, y1.x, r0.x, r1.x, r2.x);
+    one(x0.y, x1.y, y0.y, y1.y, r0.y, r1.y, r2.y);
+  } else {
+    auto one = [&](u64 p0, u64 p1, u64 q0, u64 q1, u64& o0, u64& o1, u64& o2) {
+      o0 = mul_mod(p0, q0, m);
+      o2 = mul_mod(p1, q1, m);
+      u64 hi = 0, lo = 0;
+      mac_128(hi, lo, p0, q1);
+      mac_128(hi, lo, p1, q0);
+      o1 = reduce_128(hi, lo, m);
+    };
+    one(x0.x, x1.x, y0.x, y1.x, r0.x, r1.x, r2.x);
+    one(x0.y, x1.y, y0.y, y1.y, r0.y, r1.y, r2.y);
   }
+  reinterpret_cast<w2*>(d0)[off + i] = r0;
+  reinterpret_cast<w2*>(d1)[off + i] = r1;
+  reinterpret_cast<w2*>(d2)[off + i] = r2;
 }
 
 // ---- rescale (rns_poly.c:351-383) -------------------------------------------
@@ -260,7 +335,7 @@ void launch_elementwise(EwOp op, Ptr2 res, Ptr2 a, Ptr2 b, int64_t scalar,
   }
   dag.commit();
   prof_before(KID_ELEMENTWISE);
-  dim3 g = grid_for(c->N, 2, batch.count);
+  dim3 g = grid_words(c->N, batch.count);
 #define EW_CASE(OP)                                                                        \
   case OP:                                                                                 \
     launch(ew_kernel<OP>, g, kThreads, 0, c->stream, res, a, b, (u64)scalar, batch, c->d_mod, c->N);                                    \
@@ -287,7 +362,7 @@ void launch_scalars(bool mul, Ptr2 res, Ptr2 a, const u64* per_limb, const LimbB
   dag.batch(batch, c->N, &res, &a, nullptr);
   dag.commit();
   prof_before(KID_ELEMENTWISE);
-  dim3 g = grid_for(c->N, 2, batch.count);
+  dim3 g = grid_words(c->N, batch.count);
   if (mul) launch(ew_scalars_kernel<true>, g, kThreads, 0, c->stream,
                   res, a, sc, batch, c->d_mod, c->N);
   else launch(ew_scalars_kernel<false>, g, kThreads, 0, c->stream,

@@ -124,3 +124,26 @@ def test_rotations_and_products_match_the_oracle(degree, primes, bits, dnum):
             gpu.free_ciph(x)
     gpu.close()
     orc.close()
+
+
+# limbs shorter and longer than what one CTA covers, products in double precision
+# and in integers
+@pytest.mark.parametrize("degree", [4, 8, 1024, 4096])
+@pytest.mark.parametrize("bits", [(51, 46), (60, 56)])
+def test_elementwise_operations(degree, bits):
+    import ace_compiler_b200 as rt
+    gpu = rt.Runtime(degree, 3, *bits, 2)
+    rng, lib = np.random.default_rng(degree), gpu.lib
+    a, b = (edge_limbs(rng, gpu.primes[:3], degree) for _ in range(2))
+    q = np.array(gpu.primes[:3], dtype=object)[:, None]
+    x, y = a.astype(object), b.astype(object)
+    pa, pb, out = gpu.new_poly(3, data=a), gpu.new_poly(3, data=b), gpu.new_poly(3)
+    for call, want in ((lib.Add_poly, x + y), (lib.Sub_poly, x - y), (lib.Mul_poly, x * y)):
+        call(out, pa, pb)
+        assert np.array_equal(gpu.download(out), want % q)
+    acc = gpu.download(out)
+    lib.Hw_modmuladd_scalar(gpu.limb_ptr(out, 0), gpu.limb_ptr(pa, 0), -12345, gpu.modulus(0), degree)
+    assert np.array_equal(gpu.download(out)[0], (acc[0].astype(object) - 12345 * x[0]) % q[0])
+    for p in (pa, pb, out):
+        gpu.free(p)
+    gpu.close()
