@@ -684,23 +684,65 @@ struct Cheb {  // state of one Paterson-Stockmeyer evaluation
   std::vector<Ct*>  t2;  // T_k, T_2k, ..., T_{2^(m-1) k}
 };
 
+// out = sum_j x_j * scalar_j (+ constant), one residue per limb, over `level`
+// limbs; out, which may be among the x_j, has its storage already
+struct Term {
+  CIPHER               x;
+  std::vector<int64_t> scalar;
+};
+void linear_sum(CIPHER out, const std::vector<Term>& terms, size_t level,
+                const std::vector<int64_t>& constant = {}) {
+  LinearArgs args;
+  std::memset(&args, 0, sizeof(args));
+  args.level  = (int)level;
+  args.out[0] = reinterpret_cast<u64*>(out->_c0_poly._data);
+  args.out[1] = reinterpret_cast<u64*>(out->_c1_poly._data);
+  auto add = [&](CIPHER x) {
+    args.x[args.terms][0] = reinterpret_cast<const u64*>(x->_c0_poly._data);
+    args.x[args.terms][1] = reinterpret_cast<const u64*>(x->_c1_poly._data);
+    return args.scalar[args.terms++];
+  };
+  for (const Term& t : terms) {
+    if (args.terms == kMaxLinear) {  // goes on from what there is
+      launch_linear(args);
+      args.terms = 0;
+      u64* one   = add(out);
+      for (size_t i = 0; i < level; i++) one[i] = 1;
+    }
+    u64* s = add(t.x);
+    for (size_t i = 0; i < level; i++) s[i] = (u64)t.scalar[i];
+  }
+  for (size_t i = 0; i < constant.size(); i++) args.constant[i] = (u64)constant[i];
+  launch_linear(args);
+}
+
+// out += tk * factor + value, out at tk's level or below
+void add_multiple(Context* c, CIPHER out, CIPHER tk, uint64_t factor, double value) {
+  const size_t level = out->_c0_poly._num_primes;
+  FHERT_ASSERT(level <= tk->_c0_poly._num_primes, "unmatched levels");
+  Term t{tk, std::vector<int64_t>(level)};
+  for (size_t i = 0; i < level; i++) t.scalar[i] = (int64_t)(factor % c->primes[i]);
+  linear_sum(out, {Term{out, std::vector<int64_t>(level, 1)}, t}, level,
+             encode_value(c, value, (uint32_t)level, out->_scaling_factor, 0));
+}
+
 // chebyshev_impl.c:286-325: out = rescale(sum_i w_i * T_{i+1}) over the first
 // `count` base polynomials, skipping zero weights
 void weighted_sum(Cheb& st, CIPHER out, uint32_t count, const double* w) {
-  Context* c = st.c;
-  Ct       tmp;
-  bool     first = true;
+  Context*          c     = st.c;
+  const double      delta = std::pow(2.0, (double)c->sf_bits);
+  std::vector<Term> terms;
   for (uint32_t i = 0; i < count; i++) {
     if (w[i] == 0.) continue;
-    mul_const(c, tmp.p(), st.t[i]->p(), w[i]);
-    if (first) {
-      Copy_ciph(out, tmp.p());
-      first = false;
-    } else {
-      Add_ciph(out, out, tmp.p());
-    }
+    CIPHER x = st.t[i]->p();
+    terms.push_back(Term{x, encode_value(c, w[i], (uint32_t)x->_c0_poly._num_primes, delta, 0)});
   }
-  FHERT_ASSERT(!first, "polynomial has no non_zero coefficient");
+  FHERT_ASSERT(!terms.empty(), "polynomial has no non_zero coefficient");
+  CIPHER first = terms[0].x;
+  size_t level = first->_c0_poly._num_primes;
+  for (const Term& t : terms) FHERT_ASSERT(t.x->_c0_poly._num_primes == level, "unmatched levels");
+  shape_like(c, out, first, first->_scaling_factor * delta, first->_sf_degree + 1);
+  linear_sum(out, terms, level);
   Rescale_ciph(out, out);
 }
 
@@ -713,29 +755,22 @@ void eval_quot_or_rem(Cheb& st, CIPHER out, const Coeffs& qr, uint32_t k, bool i
   CIPHER   tk = st.t[k - 1]->p();
   uint32_t dg = degree_of(cut);
   if (dg > 0) {
+    uint64_t factor = 1;
+    if (is_quotient && in_recursion) {
+      // the leading coefficient is a power of two
+      for (uint32_t i = 0; i < std::log2(qr.back()); i++) factor *= 2;
+    } else if (is_quotient) {
+      factor = 2;
+    }
     weighted_sum(st, out, dg, cut.data() + 1);
-    if (is_quotient) {
-      if (in_recursion) {
-        // the leading coefficient is a power of two: add instead of multiplying
-        double quot_last = qr.back();
-        Ct     sum;
-        Copy_ciph(sum.p(), tk);
-        for (uint32_t i = 0; i < std::log2(quot_last); i++) Add_ciph(sum.p(), sum.p(), sum.p());
-        Add_ciph(out, out, sum.p());
-      } else {
-        Add_ciph(out, out, tk);
-        Add_ciph(out, out, tk);
-      }
-    } else {
-      Add_ciph(out, out, tk);
-    }
-  } else {
-    Copy_ciph(out, tk);
-    if (is_quotient) {
-      double   quot_last = qr.back();
-      uint32_t end       = in_recursion ? (uint32_t)std::log2(quot_last) : (uint32_t)quot_last;
-      for (uint32_t i = 0; i < end; i++) Add_ciph(out, out, tk);
-    }
+    add_multiple(c, out, tk, factor, qr[0] / 2);
+    return;
+  }
+  Copy_ciph(out, tk);
+  if (is_quotient) {
+    double   quot_last = qr.back();
+    uint32_t end       = in_recursion ? (uint32_t)std::log2(quot_last) : (uint32_t)quot_last;
+    for (uint32_t i = 0; i < end; i++) Add_ciph(out, out, tk);
   }
   add_const(c, out, out, qr[0] / 2);
 }

@@ -641,6 +641,17 @@ struct SumsArgs {
   Plain      plain[kMaxSums][kMaxParts];
 };
 void launch_weighted_sums(const SumsArgs& args);
+// out = sum_j x_j * scalar[j][limb] (+ constant[limb], first polynomial) over the
+// first `level` Q limbs of both polynomials; out may be one of the x_j
+constexpr int kMaxLinear = 12;
+struct LinearArgs {
+  int        terms, level;
+  const u64* x[kMaxLinear][2];
+  u64*       out[2];
+  u64        scalar[kMaxLinear][kMaxLimbs / 2];
+  u64        constant[kMaxLimbs / 2];
+};
+void launch_linear(const LinearArgs& args);
 // Mod-raise (rns_poly.c:1101-1125): res[dst] = switch_modulus(src, q_0 -> q_i)
 void launch_mod_raise(int64_t* res, const int64_t* src, const LimbBatch& batch);
 
