@@ -828,8 +828,7 @@ void ps_inner(Cheb& st, CIPHER out, const Coeffs& f, uint32_t k, uint32_t m, boo
   } else {
     add_const(c, out, t2, cq[0] / 2);
   }
-  Mul_ciph(out, out, qu.p());
-  Rescale_ciph(out, out);
+  fhert_mul_rescale(c, out, out, qu.p(), false, nullptr);
   Add_ciph(out, out, su.p());
 }
 
@@ -853,32 +852,27 @@ void eval_chebyshev(Context* c, CIPHER out, CIPHER in, const Coeffs& coeffs) {
   Ct y;
   Copy_ciph(y.p(), t0);
 
-  Ct prod;
   std::vector<int64_t> minus_one =
       encode_value(c, -1.0, (uint32_t)t0->_c0_poly._num_primes, t0->_scaling_factor,
                    (uint32_t)t0->_c0_poly._num_primes_p);
-  auto double_and_shift = [&](CIPHER tj) {  // tj = 2 * prod, rescaled
-    Add_ciph(tj, prod.p(), prod.p());
-    Rescale_ciph(tj, tj);
+  auto twice_product = [&](CIPHER tj, CIPHER x, CIPHER y) {  // tj = rescale(2 * x * y)
+    fhert_mul_rescale(c, tj, x, y, true, nullptr);
   };
   for (uint32_t i = 2; i <= k; i++) {
     CIPHER tj = st.t[i - 1]->p();
     if (!(i & (i - 1))) {
       CIPHER h = st.t[i / 2 - 1]->p();
-      Mul_ciph(prod.p(), h, h);
-      double_and_shift(tj);
+      twice_product(tj, h, h);
       add_scalars(c, tj, tj, minus_one);
     } else if (i % 2 == 1) {
       if (even) continue;
-      Mul_ciph(prod.p(), st.t[i / 2 - 1]->p(), st.t[i / 2]->p());
-      double_and_shift(tj);
+      twice_product(tj, st.t[i / 2 - 1]->p(), st.t[i / 2]->p());
       Sub_ciph(tj, tj, y.p());
     } else {
       uint32_t h1 = i / 2;
       if (even && (h1 % 2 == 1)) h1 += 1;
       uint32_t h2 = i - h1;
-      Mul_ciph(prod.p(), st.t[h1 - 1]->p(), st.t[h2 - 1]->p());
-      double_and_shift(tj);
+      twice_product(tj, st.t[h1 - 1]->p(), st.t[h2 - 1]->p());
       if (h1 == h2) add_scalars(c, tj, tj, minus_one);
       else Sub_ciph(tj, tj, st.t[1]->p());
     }
@@ -893,15 +887,13 @@ void eval_chebyshev(Context* c, CIPHER out, CIPHER in, const Coeffs& coeffs) {
   Copy_ciph(st.t2[0]->p(), st.t[k - 1]->p());
   for (uint32_t i = 1; i < m; i++) {
     CIPHER prev = st.t2[i - 1]->p(), cur = st.t2[i]->p();
-    Mul_ciph(prod.p(), prev, prev);
-    double_and_shift(cur);
+    twice_product(cur, prev, prev);
     add_scalars(c, cur, cur, minus_one);
   }
   Ct t2km1;
   Copy_ciph(t2km1.p(), st.t2[0]->p());
   for (uint32_t i = 1; i < m; i++) {
-    Mul_ciph(prod.p(), t2km1.p(), st.t2[i]->p());
-    double_and_shift(t2km1.p());
+    twice_product(t2km1.p(), t2km1.p(), st.t2[i]->p());
     Sub_ciph(t2km1.p(), t2km1.p(), st.t2[0]->p());
   }
 
@@ -967,17 +959,14 @@ void add_key(Context* c, KeysArgs& args, uint32_t k) {
   }
 }
 
-// one stage: rescale, hoisted giant-step rotations (one launch over all their
+// one stage on a rescaled ciphertext: hoisted giant-step rotations (one launch over all their
 // keys), all baby-step sums in one launch, outer rotations on the extended basis,
-// one ModDown at the end
+// one ModDown at the end, with the rescale before the stage that follows
 void rotate_stage(Context* c, CIPHER ct, std::vector<PLAINTEXT>& plains, const FftParams& p,
-                  const std::vector<int32_t>& rot_in, const std::vector<int32_t>& rot_out, int step,
-                  bool encoding, bool is_rem) {
+                  const std::vector<int32_t>& rot_in, const std::vector<int32_t>& rot_out,
+                  bool is_rem, bool rescale) {
   const int giant = is_rem ? p.g_rem : p.g, baby = is_rem ? p.b_rem : p.b;
   const int num_rot = is_rem ? p.num_rot_rem : p.num_rot;
-  const int level_idx = encoding ? p.level_budget - 1 : 0;
-  if (is_rem || step != level_idx) Rescale_ciph(ct, ct);
-
   const size_t n = c->N, K = c->K, level = ct->_c0_poly._num_primes, ext = level + K;
   const size_t pw = ext * n;  // words of one extended polynomial
   const int    parts = (int)std::min<size_t>((level + c->alpha - 1) / c->alpha, c->dnum);
@@ -1089,9 +1078,17 @@ void rotate_stage(Context* c, CIPHER ct, std::vector<PLAINTEXT>& plains, const F
   }
   int64_t*       r[2] = {c0, c1};
   const int64_t* x[2] = {total, total + pw};
-  fhert_mod_down_polys(c, 2, r, x, (int)level, nullptr, level, true);
   ct->_scaling_factor = ct->_scaling_factor * plain_sf;
   ct->_sf_degree      = ct->_sf_degree + plain_degree;
+  if (rescale && ntt_can_fuse()) {
+    fhert_mod_down_rescale(c, r, x, level, false);
+    ct->_scaling_factor /= Get_default_sc();
+    ct->_sf_degree -= 1;
+    set_level(ct, level - 1);
+    return;
+  }
+  fhert_mod_down_polys(c, 2, r, x, (int)level, nullptr, level, true);
+  if (rescale) Rescale_ciph(ct, ct);
 }
 
 // bootstrap.c:1375-1484
@@ -1124,20 +1121,22 @@ void linear_transform(Context* c, CIPHER result, CIPHER in, Precom* pre, bool en
     for (int i = 0; i < p.b_rem; i++)
       rot_out[s][i] = (int32_t)reduce_rotation((p.g_rem * i) * shift, order / 4);
   }
-  Copy_ciph(result, in);
+  // the stages in order, the remainder's last; every stage but the first works on
+  // rescaled input, except that a remainder is always rescaled
+  std::vector<int> order_of;
   if (encoding)
-    for (int s = end - 1; s > start - 1; s--) {
-      rotate_stage(c, result, plain[s], p, rot_in[s], rot_out[s], s, true, false);
-      trace_sum("c2s stage", result);
-    }
+    for (int s = end - 1; s > start - 1; s--) order_of.push_back(s);
   else
-    for (int s = start; s < end; s++) {
-      rotate_stage(c, result, plain[s], p, rot_in[s], rot_out[s], s, false, false);
-      trace_sum("s2c stage", result);
-    }
-  if (flag_rem) {
-    int s = encoding ? stop : p.level_budget - flag_rem;
-    rotate_stage(c, result, plain[s], p, rot_in[s], rot_out[s], s, encoding, true);
+    for (int s = start; s < end; s++) order_of.push_back(s);
+  const int full = (int)order_of.size();
+  if (flag_rem) order_of.push_back(encoding ? stop : p.level_budget - flag_rem);
+  Copy_ciph(result, in);
+  if (full == 0) Rescale_ciph(result, result);
+  for (int i = 0; i < (int)order_of.size(); i++) {
+    const int  s    = order_of[i];
+    const bool last = i + 1 == (int)order_of.size();
+    rotate_stage(c, result, plain[s], p, rot_in[s], rot_out[s], i >= full, !last);
+    if (i < full) trace_sum(encoding ? "c2s stage" : "s2c stage", result);
   }
 }
 
@@ -1157,10 +1156,15 @@ void approx_mod(Context* c, CIPHER ct) {
   // double-angle iterations: cos(2x) = 2 cos^2(x) - 1, scaled
   int r = tab.double_angle;
   for (int j = 1; j < r + 1; j++) {
-    Mul_ciph(ct, ct, ct);
-    Add_ciph(ct, ct, ct);
-    add_const(c, ct, ct, -1.0 / std::pow(2.0 * M_PI, std::pow(2.0, j - r)));
-    Rescale_ciph(ct, ct);
+    // half the constant joins the product before it is doubled
+    const double         shift = -1.0 / std::pow(2.0 * M_PI, std::pow(2.0, j - r));
+    std::vector<int64_t> sc = encode_value(c, shift, (uint32_t)ct->_c0_poly._num_primes,
+                                           ct->_scaling_factor * ct->_scaling_factor, 0);
+    std::vector<u64>     half(sc.begin(), sc.end());
+    for (size_t i = 0; i < half.size(); i++)
+      if (half[i] & 1) half[i] += c->primes[i];
+    for (u64& h : half) h /= 2;
+    fhert_mul_rescale(c, ct, ct, ct, true, half.data());
   }
 }
 

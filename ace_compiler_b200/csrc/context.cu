@@ -634,7 +634,7 @@ Context* create_context(const CKKS_PARAMS* p) {
 
   // ModDown / Extend constants (crt.c:357-414)
   std::vector<Twiddle> phat_inv(K), p_inv(L), p_mod_q(L);
-  std::vector<u64>     phat_mod_q((size_t)L * K);
+  std::vector<u64>     phat_mod_q((size_t)L * K), phat_p_inv((size_t)L * K);
   std::vector<Twiddle> moddown_last(2 * (size_t)total);
   for (int k = 0; k < K; k++) {
     u64 pk = pp[k], hat = 1;
@@ -648,13 +648,25 @@ Context* create_context(const CKKS_PARAMS* p) {
     for (int k = 0; k < K; k++) P = mulmod(P, pp[k] % qi, qi);
     p_mod_q[i] = tw_of(P, qi);
     p_inv[i]   = tw_of(invmod(P, qi), qi);
+    last_stage(&moddown_last[2 * i], dm[i].n_inv, c->h_inv[i][1].w, p_inv[i].w, qi);
     for (int k = 0; k < K; k++) {
       u64 hat = 1;
       for (int j = 0; j < K; j++)
         if (j != k) hat = mulmod(hat, pp[j] % qi, qi);
       phat_mod_q[(size_t)i * K + k] = hat;
+      phat_p_inv[(size_t)i * K + k] = mulmod(hat, p_inv[i].w, qi);
     }
   }
+  // ModDown and rescale in one step: row l of table t holds 2^t / (P q_l)
+  std::vector<Twiddle> pql_inv(2 * (size_t)L * L);
+  for (int l = 1; l < L; l++)
+    for (int i = 0; i < l; i++) {
+      const u64 v = mulmod(p_inv[i].w, ql_inv[(size_t)l * L + i].w, q[i]);
+      pql_inv[(size_t)l * L + i]       = tw_of(v, q[i]);
+      pql_inv[(size_t)(L + l) * L + i] = tw_of(mulmod(v, 2, q[i]), q[i]);
+    }
+  c->d_pql_inv     = upload(pql_inv);
+  c->d_down_planes = upload(conv_planes(K, (K + 3) & ~3, L, phat_p_inv.data(), c->primes.data()));
   c->d_phat_inv   = upload(phat_inv);
   c->d_phat_planes = upload(conv_planes(K, (K + 3) & ~3, L, phat_mod_q.data(), c->primes.data()));
   c->d_moddown_last = upload(moddown_last);
@@ -695,6 +707,8 @@ void destroy_context() {
   cudaFree(c->d_phat_inv);
   cudaFree(c->d_phat_planes);
   cudaFree(c->d_moddown_last);
+  cudaFree(c->d_pql_inv);
+  cudaFree(c->d_down_planes);
   for (auto& kv : c->modup_last) cudaFree(kv.second);
   cudaFreeHost(c->h_error);
   cudaFree(c->d_p_inv);

@@ -155,11 +155,19 @@ inner_product_kernel(const __grid_constant__ InnerArgs a, const __grid_constant_
         }
       }
     }
-    reinterpret_cast<ulonglong2*>(a.acc0 + d_off)[i] =
-        make_ulonglong2(s[0].template value<EXACT>(sm, md), s[1].template value<EXACT>(sm, md));
-    if (TWO)
-      reinterpret_cast<ulonglong2*>(a.acc1 + d_off)[i] =
-          make_ulonglong2(s[2].template value<EXACT>(sm, md), s[3].template value<EXACT>(sm, md));
+    ulonglong2 v0 = make_ulonglong2(s[0].template value<EXACT>(sm, md), s[1].template value<EXACT>(sm, md));
+    ulonglong2 v1{};
+    if (TWO) v1 = make_ulonglong2(s[2].template value<EXACT>(sm, md), s[3].template value<EXACT>(sm, md));
+    if (TWO && a.add[0] != nullptr && is_q) {
+      const Twiddle    p  = a.p_mod_q[m];
+      const ulonglong2 x0 = load2(a.add[0] + d_off, i), x1 = load2(a.add[1] + d_off, i);
+      v0.x = add_mod(v0.x, mul_shoup(x0.x, p.w, p.wp, md.q), md.q);
+      v0.y = add_mod(v0.y, mul_shoup(x0.y, p.w, p.wp, md.q), md.q);
+      v1.x = add_mod(v1.x, mul_shoup(x1.x, p.w, p.wp, md.q), md.q);
+      v1.y = add_mod(v1.y, mul_shoup(x1.y, p.w, p.wp, md.q), md.q);
+    }
+    reinterpret_cast<ulonglong2*>(a.acc0 + d_off)[i] = v0;
+    if (TWO) reinterpret_cast<ulonglong2*>(a.acc1 + d_off)[i] = v1;
   }
 }
 
@@ -414,6 +422,8 @@ void launch_inner_product(const InnerArgs& args) {
       }
       dag.set.write(args.acc0 + d_off, w);
       if (args.acc1 != nullptr) dag.set.write(args.acc1 + d_off, w);
+      if (args.add[0] != nullptr && is_q)
+        for (const u64* add : args.add) dag.set.read(add + d_off, w);
     }
   }
   dag.commit();

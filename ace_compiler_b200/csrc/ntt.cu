@@ -77,18 +77,23 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
   pro.mul    = f.pro_mul;
   pro.mod    = f.pro_mod;
   pro.q_last = f.q_last;
+  pro.last_x    = f.last_x;
+  pro.last_conv = f.last_conv;
+  pro.twice     = f.twice;
   nttk::NttEpi epi;
   epi.kind = f.epi_kind;
   epi.mul  = f.epi_mul;
   epi.aux  = f.aux;
   epi.add  = f.add;
   epi.perm = f.perm;
-  // strided pass: in[a] -> mid[k]; contiguous pass: mid[k] -> out[dst] with the epilogue
+  // strided pass: in[a] -> mid[k] (mid[a] with prologue 3); contiguous pass: from there
+  // to out[dst] with the epilogue
   LimbBatch b1 = b, b2 = b;
   for (int i = 0; i < b.count; i++) {
-    b1.limb[i].dst = (uint16_t)i;
+    const uint16_t mid_limb = (uint16_t)(f.pro_kind == 3 ? b.limb[i].a : i);
+    b1.limb[i].dst = mid_limb;
     b1.limb[i].sel = (uint8_t)(f.multi ? 0 : b.limb[i].sel & 1);
-    b2.limb[i].a   = (uint16_t)i;
+    b2.limb[i].a   = mid_limb;
     b2.limb[i].sel = (uint8_t)(f.multi ? b.limb[i].sel : b.limb[i].sel & 6);
   }
   const int n_int = integers_first(c, b1);
@@ -96,7 +101,11 @@ void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const
   DagScope dag(DAG_NTT_FUSED);
   if (dag.live) {
     const size_t w = (size_t)c->N * sizeof(u64);
-    dag.set.write(mid, (size_t)b.count * w);
+    for (int i = 0; i < b.count; i++) dag.set.write(mid + (size_t)b1.limb[i].dst * c->N, w);
+    for (int g = 0; g < 2 && f.pro_kind == 3; g++) {
+      dag.set.read(f.last_x.p[g], w);
+      dag.set.read(f.last_conv.p[g], w);
+    }
     if (f.multi == nullptr) dag.batch(b, c->N, &out, &in, nullptr);
     for (int i = 0; i < b.count; i++) {
       const LimbRef& lr = b.limb[i];

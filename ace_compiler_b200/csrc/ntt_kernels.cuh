@@ -139,6 +139,12 @@ __device__ __forceinline__ Twiddle ld_tw(const Twiddle* p) {
 //   kind 1, the lift of a rescale (rns_poly.c:351-366): the source limb holds
 //     residues modulo q_last in coefficient form; the value that enters the
 //     transform under prime i is switch_modulus(v, q_last -> q_i) * mul[i]
+//   kind 3, the lift of a rescale that follows a ModDown at once: the dropped limb
+//     is y = last_x - last_conv (both multiples of P^-1 already), the source limb
+//     the converted special limbs under prime i, also times P^-1; enters
+//     (switch_modulus(y) + source) * mul[i], with y and source doubled for the
+//     rescale of twice the polynomial.  One forward transform per limb then
+//     serves both steps.
 //   kind 2, a message polynomial (crt.c:1153-1221): signed 64-bit integers,
 //     negatives also as kMax64 + v; their residues, times mul[i] when given
 struct NttPro {
@@ -146,6 +152,9 @@ struct NttPro {
   const Twiddle* mul  = nullptr;  // [prime]
   const u64*     mod  = nullptr;  // [prime] q_last mod q_i
   u64            q_last = 0;
+  Ptr2           last_x{{nullptr, nullptr}};
+  Ptr2           last_conv{{nullptr, nullptr}};
+  bool           twice = false;
 };
 // a message coefficient modulo q; r = floor(2^64 / q)   (modular.h:278-280)
 __device__ __forceinline__ u64 message_residue(u64 v, const Mod m, u64 r) {
@@ -300,16 +309,21 @@ struct ArithFp {
     const V x = load(message_residue(v, make_mod(q), rq));
     return scaled ? mul(x, w) : x;
   }
-  __device__ __forceinline__ V lift(u64 v, const Lift& l) const {
+  __device__ __forceinline__ V centred(u64 v, const Lift& l) const {
     if (l.narrow) {
       V x = load(v);
       if (v > l.half) x = __dadd_rn(x, -l.dq_last);
-      return mul(x, l.w);
+      return x;
     }
     const Mod m = make_mod(q);
     u64       r = canon_any(v, m, rq);
     if (v > l.half) r = r >= l.last_mod_q ? r - l.last_mod_q : r + q - l.last_mod_q;
-    return mul(load(r), l.w);
+    return load(r);
+  }
+  __device__ __forceinline__ V lift(u64 v, const Lift& l) const { return mul(centred(v, l), l.w); }
+  __device__ __forceinline__ V lift_sum(u64 v, u64 more, bool twice, const Lift& l) const {
+    const V a = load(more);
+    return mul(__dadd_rn(centred(v, l), twice ? __dadd_rn(a, a) : a), l.w);
   }
   template <int EPI>
   __device__ __forceinline__ u64 epilogue(u64 t, u64 aux, T w) const {
@@ -391,10 +405,11 @@ struct ArithInt {
     const u64 r = message_residue(v, m, rq);
     return scaled ? canon_4q(shoup4(r, w, m), m) : r;
   }
-  __device__ __forceinline__ V lift(u64 v, const Lift& l) const {
+  __device__ __forceinline__ V lift(u64 v, const Lift& l) const { return lift_sum(v, 0, false, l); }
+  __device__ __forceinline__ V lift_sum(u64 v, u64 more, bool twice, const Lift& l) const {
     u64 r = canon_any(v, m, rq);
     if (v > l.half) r = r >= l.last_mod_q ? r - l.last_mod_q : r + q - l.last_mod_q;
-    return canon_4q(shoup4(r, l.w, m), m);
+    return canon_4q(shoup4(r + (twice ? 2 * more : more), l.w, m), m);
   }
   template <int EPI>
   __device__ __forceinline__ u64 epilogue(u64 t, u64 aux, const T w) const {
@@ -823,10 +838,26 @@ __device__ __forceinline__ void strided_inv(typename A::V (&x)[1 << E], u64* sm,
 
 // (the prologue is a template parameter: its code in a kernel that does not use
 // it cost 2 us a launch)
-template <class A, int E, int PRO>
+// at(e): where in the limb value e stands; last: the dropped limb's pair (kind 3)
+struct LastLimb {
+  const u64* x    = nullptr;
+  const u64* conv = nullptr;
+};
+template <class A, int E, int PRO, class At>
 __device__ __forceinline__ void load_values(typename A::V (&x)[1 << E], const u64 (&v)[1 << E],
-                                            const A& ar, const NttPro& pro, int prime) {
-  if constexpr (PRO == 1) {
+                                            const A& ar, const NttPro& pro, int prime,
+                                            const LastLimb& last, At at) {
+  if constexpr (PRO == 3) {
+    const typename A::Lift lift = ar.make_lift(pro, prime);
+    const u64              ql   = pro.q_last;
+#pragma unroll
+    for (int e = 0; e < (1 << E); e++) {
+      u64 y = last.x[at(e)], s = last.conv[at(e)];
+      y = y >= s ? y - s : y + ql - s;
+      if (pro.twice) y = csub(2 * y, ql);
+      x[e] = ar.lift_sum(y, v[e], pro.twice, lift);
+    }
+  } else if constexpr (PRO == 1) {
     const typename A::Lift lift = ar.make_lift(pro, prime);
 #pragma unroll
     for (int e = 0; e < (1 << E); e++) x[e] = ar.lift(v[e], lift);
@@ -844,7 +875,7 @@ __device__ __forceinline__ void load_values(typename A::V (&x)[1 << E], const u6
 template <bool INV, int PRO, int E, int S1, int TC, class A>
 __device__ __forceinline__ void strided_body(const u64* src, u64* dst, u64* sm, const Twiddle* table,
                                              const A& ar, const Twiddle* fin, const NttPro& pro,
-                                             int prime) {
+                                             int prime, LastLimb last) {
   const typename A::T* tw = reinterpret_cast<const typename A::T*>(table);
   const int            c = threadIdx.x % TC, g = threadIdx.x / TC;
   typename A::V        x[1 << E];
@@ -854,10 +885,13 @@ __device__ __forceinline__ void strided_body(const u64* src, u64* dst, u64* sm, 
   src += c;
   dst += c;
   if constexpr (!INV) {
-    u64 v[1 << E];
+    auto at = [&](int e) { return (size_t)(at_top | (e << top)) << kContigLog; };
+    u64  v[1 << E];
 #pragma unroll
-    for (int e = 0; e < (1 << E); e++) v[e] = src[(size_t)(at_top | (e << top)) << kContigLog];
-    load_values<A, E, PRO>(x, v, ar, pro, prime);
+    for (int e = 0; e < (1 << E); e++) v[e] = src[at(e)];
+    last.x += c;
+    last.conv += c;
+    load_values<A, E, PRO>(x, v, ar, pro, prime, last, at);
     strided_fwd<A, E, S1, TC, 0>(x, sm, g, c, tw, ar);
 #pragma unroll
     for (int e = 0; e < (1 << E); e++) dst[(size_t)(at_low | e) << kContigLog] = A::bits(x[e]);
@@ -877,7 +911,8 @@ template <bool INV, int PRO, int S1>
 __global__ void __launch_bounds__(kThreads, 7)
 ntt_strided_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, TileMap map,
                    const Twiddle* __restrict__ tables, const DevModulus* __restrict__ mods,
-                   const Twiddle* __restrict__ inv_last, uint32_t n, NttPro pro) {
+                   const Twiddle* __restrict__ inv_last, uint32_t n,
+                   const __grid_constant__ NttPro pro) {
   constexpr int TI = tile_columns(S1, 3), TF = tile_columns(S1, 4);
   __shared__ u64   sm[TF << S1];
   u32              limb, tile;
@@ -889,12 +924,14 @@ ntt_strided_kernel(Ptr2 in, Ptr2 out, const __grid_constant__ LimbBatch batch, T
   const size_t     col    = (size_t)tile * (is_int ? TI : TF);
   const u64*       src    = ((lr.sel & 1) ? in.p[1] : in.p[0]) + (size_t)lr.a * n + col;
   u64*             dst    = ((lr.sel & 4) ? out.p[1] : out.p[0]) + (size_t)lr.dst * n + col;
+  LastLimb last;
+  if (PRO == 3) last = LastLimb{pro.last_x.p[lr.sel & 1] + col, pro.last_conv.p[lr.sel & 1] + col};
   if (!is_int)
-    strided_body<INV, PRO, 4, S1, TF>(src, dst, sm, tab, ArithFp(dm), fin, pro, lr.prime);
+    strided_body<INV, PRO, 4, S1, TF>(src, dst, sm, tab, ArithFp(dm), fin, pro, lr.prime, last);
   else if (dm.kind == kNttNarrow)
-    strided_body<INV, PRO, 3, S1, TI>(src, dst, sm, tab, ArithInt<false>(dm), fin, pro, lr.prime);
+    strided_body<INV, PRO, 3, S1, TI>(src, dst, sm, tab, ArithInt<false>(dm), fin, pro, lr.prime, last);
   else
-    strided_body<INV, PRO, 3, S1, TI>(src, dst, sm, tab, ArithInt<true>(dm), fin, pro, lr.prime);
+    strided_body<INV, PRO, 3, S1, TI>(src, dst, sm, tab, ArithInt<true>(dm), fin, pro, lr.prime, last);
 }
 
 // ---- whole limb in one CTA (512 <= N <= 4096) ------------------------------------
@@ -906,7 +943,8 @@ template <bool INV, int PRO, int EPI, int S1, class A>
 __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, const Twiddle* table,
                                            const DevModulus& dm, const Twiddle* fin,
                                            const NttPro& pro, int prime, const u64* aux,
-                                           const u64* add, const Twiddle* emul, const uint32_t* perm) {
+                                           const u64* add, const Twiddle* emul, const uint32_t* perm,
+                                           const LastLimb& last) {
   constexpr int        logn = S1 + kContigLog, top = logn - 4;
   const A              ar(dm);
   const typename A::T* tree = reinterpret_cast<const typename A::T*>(table);
@@ -920,7 +958,7 @@ __device__ __forceinline__ void whole_body(const u64* src, u64* dst, u64* sm, co
     u64 v[16];
 #pragma unroll
     for (int e = 0; e < 16; e++) v[e] = src[g | (e << top)];
-    load_values<A, 4, PRO>(x, v, ar, pro, prime);
+    load_values<A, 4, PRO>(x, v, ar, pro, prime, last, [&](int e) { return g | (e << top); });
     fwd_stages<A, 4, S1, 0>(x, TreeTw<A>{tree, 1u}, ar);
 #pragma unroll
     for (int e = 0; e < 16; e++) sm[at(g | (e << top))] = A::bits(x[e]);
@@ -964,7 +1002,7 @@ template <bool INV, int PRO, int EPI, int S1>
 __global__ void __launch_bounds__(16 << S1)
 ntt_whole_kernel(Ptr2 in, Ptr2 out, LimbBatch batch, const Twiddle* __restrict__ tables,
                  const DevModulus* __restrict__ mods, const Twiddle* __restrict__ inv_last,
-                 NttPro pro, NttEpi epi, const __grid_constant__ MultiArg<EPI> multi) {
+                 const __grid_constant__ NttPro pro, NttEpi epi, const __grid_constant__ MultiArg<EPI> multi) {
   constexpr uint32_t n = (uint32_t)kContigBlock << S1;
   __shared__ u64 sm[n];
   const LimbRef    lr  = batch.limb[blockIdx.x];
@@ -989,15 +1027,17 @@ ntt_whole_kernel(Ptr2 in, Ptr2 out, LimbBatch batch, const Twiddle* __restrict__
   }
   dst += (size_t)lr.dst * n;
   const Twiddle* emul = EPI != 0 ? epi.mul + lr.prime : nullptr;
+  LastLimb       last;
+  if (PRO == 3) last = LastLimb{pro.last_x.p[lr.sel & 1], pro.last_conv.p[lr.sel & 1]};
   if (dm.kind == kNttFloat)
     whole_body<INV, PRO, EPI, S1, ArithFp>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
-                                       perm);
+                                       perm, last);
   else if (dm.kind == kNttNarrow)
     whole_body<INV, PRO, EPI, S1, ArithInt<false>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
-                                       perm);
+                                       perm, last);
   else
     whole_body<INV, PRO, EPI, S1, ArithInt<true>>(src, dst, sm, tab, dm, fin, pro, lr.prime, aux, add, emul,
-                                       perm);
+                                       perm, last);
 }
 
 // ---- tiny transforms (N < 512): one butterfly at a time --------------------------
@@ -1073,6 +1113,7 @@ inline void launch_strided(Ptr2 in, Ptr2 out, const LimbBatch& b, int n_int, con
                            cudaStream_t stream, const NttPro& pro = NttPro()) {
   if (INV || pro.kind == 0) launch_strided_p<INV, 0>(in, out, b, n_int, t, stream, pro);
   else if (pro.kind == 1) launch_strided_p<false, 1>(in, out, b, n_int, t, stream, pro);
+  else if (pro.kind == 3) launch_strided_p<false, 3>(in, out, b, n_int, t, stream, pro);
   else launch_strided_p<false, 2>(in, out, b, n_int, t, stream, pro);
 }
 
@@ -1123,9 +1164,10 @@ inline void launch_whole(Ptr2 in, Ptr2 out, const LimbBatch& b, const NttTables&
                          cudaStream_t stream, const NttPro& pro = NttPro(),
                          const NttEpi& epi = NttEpi(), const NttMulti* multi = nullptr) {
   // a lift comes with a rescale's last step, a message with none
-  FHERT_ASSERT(pro.kind == 0 || (pro.kind == 1 && epi.kind == 1) || (pro.kind == 2 && epi.kind == 0),
+  FHERT_ASSERT(pro.kind == 0 || ((pro.kind & 1) && epi.kind == 1) || (pro.kind == 2 && epi.kind == 0),
                "no transform with prologue %d and epilogue %d", pro.kind, epi.kind);
   if (pro.kind == 1) launch_whole_t<false, 1, 1>(in, out, b, t, stream, pro, epi, MultiArg<1>{});
+  else if (pro.kind == 3) launch_whole_t<false, 3, 1>(in, out, b, t, stream, pro, epi, MultiArg<1>{});
   else if (pro.kind == 2) launch_whole_t<false, 2, 0>(in, out, b, t, stream, pro, epi, MultiArg<0>{});
   else if (INV || epi.kind == 0) launch_whole_t<INV, 0, 0>(in, out, b, t, stream, pro, epi, MultiArg<0>{});
   else if (epi.kind == 3) launch_whole_t<false, 0, 3>(in, out, b, t, stream, pro, epi, MultiArg<3>{});

@@ -117,6 +117,10 @@ struct Context {
   // planes of (P/p_k) mod q_i for all Q primes i (conv_planes), p_inv[i] = P^-1 mod q_i
   Twiddle* d_phat_inv    = nullptr;
   uint8_t* d_phat_planes = nullptr;
+  // ModDown and rescale in one step: the conversion with P^-1 mod q_i in row i,
+  // and [t][l][i] = 2^t / (P q_l) mod q_i
+  uint8_t* d_down_planes = nullptr;
+  Twiddle* d_pql_inv = nullptr;
   Twiddle* d_p_inv      = nullptr;
   // Extend: P mod q_i
   Twiddle* d_p_mod_q = nullptr;
@@ -498,6 +502,11 @@ struct NttFuse {
   Ptr2           add{{nullptr, nullptr}};
   const uint32_t* perm    = nullptr;
   const NttMulti* multi   = nullptr;
+  // prologue 3: the dropped limb is last_x - last_conv (polynomial by selector bit
+  // 0), everything doubled when twice; source and middle limbs have the same index
+  Ptr2           last_x{{nullptr, nullptr}};
+  Ptr2           last_conv{{nullptr, nullptr}};
+  bool           twice = false;
 };
 bool ntt_can_fuse();
 void launch_ntt_fused(Ptr2 in, int64_t* mid, Ptr2 out, const LimbBatch& b, const NttFuse& f);
@@ -601,6 +610,9 @@ struct InnerArgs {
   u64*       acc1;
   int        acc_p_limb;  // limb index of the first P limb in acc
   int        ext_p_limb;  // limb index of the first P limb in ext
+  // sums start from P * add on the Q limbs (null: from zero)
+  const u64*     add[2];
+  const Twiddle* p_mod_q;
 };
 void launch_inner_product(const InnerArgs& args);
 // The digits of one polynomial (digit j at digits + j * digit_stride, level Q
@@ -694,6 +706,11 @@ extern "C" {
 void fhert_raise_parts(fhert::Context* c, const int64_t* src, bool is_ntt, size_t level,
                        int part_begin, int part_end, int64_t* ext_base, size_t part_stride,
                        int p_limb);
+void fhert_mul_rescale(fhert::Context* c, CIPHER res, CIPHER a, CIPHER b, bool twice,
+                       const fhert::u64* constant);
+// ModDown and rescale in one (level + K limbs in, level - 1 out; ntt_can_fuse() only)
+void fhert_mod_down_rescale(fhert::Context* c, int64_t* const res[2], const int64_t* const ext[2],
+                            size_t level, bool twice);
 // ModDown of one or two extended polynomials (special limbs at ext_p_limb),
 // optionally adding add[g] to the result and permuting it (res[i] = value[perm[i]];
 // NTT form and ntt_can_fuse() only, res must not overlap ext or add)

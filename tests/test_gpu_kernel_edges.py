@@ -1,6 +1,7 @@
 """Kernels against the plain-C oracle at the sizes where a tile, a variant or a
 range of primes ends."""
 import ctypes as C
+import hashlib
 
 import numpy as np
 import pytest
@@ -146,4 +147,34 @@ def test_elementwise_operations(degree, bits):
     assert np.array_equal(gpu.download(out)[0], (acc[0].astype(object) - 12345 * x[0]) % q[0])
     for p in (pa, pb, out):
         gpu.free(p)
+    gpu.close()
+
+
+# digests of refreshed ciphertexts, taken when every step of a bootstrap (product,
+# doubling, ModDown, rescale, sums term by term) was an operation of its own; those
+# equalled the CPU runtime's residue for residue.  Rings without and with fused
+# transforms, a remainder stage, sparse packing, both arithmetics, the even series.
+@pytest.mark.parametrize("degree,primes,bits,slots,even,digest", [
+    (256, 18, (60, 56), 128, 0, "691c6348ad06ad75"), (512, 18, (60, 56), 256, 0, "f3e246895a7dfdeb"),
+    (2048, 19, (60, 56), 1024, 0, "7b8af421ee5a0168"), (2048, 19, (60, 56), 256, 0, "d3fde1baac59e419"),
+    (1024, 20, (60, 45), 512, 0, "e9032d2f86761a55"), (8192, 18, (60, 56), 4096, 0, "05a2e7cd3e6bb17f"),
+    (8192, 18, (55, 45), 4096, 0, "758cb09ff025fc0b"), (1024, 20, (60, 45), 512, 1, "1b814ce8f3a0a33a")])
+def test_bootstrap_digests(degree, primes, bits, slots, even, digest, monkeypatch):
+    import ace_compiler_b200 as rt
+    monkeypatch.setenv("RTLIB_DISABLE_BOOTSTRAP_PRECOM", "0")
+    monkeypatch.setenv("RTLIB_BTS_EVEN_POLY", str(even))
+    gpu = rt.Runtime(degree, primes, *bits, 3, keygen=True, seed=np.arange(16),
+                     fake_time_us=1_700_000_000_000_000)
+    if slots != degree // 2:
+        gpu.lib.Bootstrap_precom(slots)
+    rng = np.random.default_rng(degree)
+    ct = gpu.new_ciph(*(np.stack([rng.integers(0, p, degree, dtype=np.int64) for p in gpu.primes[:2]])
+                        for _ in range(2)))
+    ct._slots = slots
+    res = rt.CIPHERTEXT()
+    gpu.lib.Bootstrap(C.byref(res), C.byref(ct), 0)
+    got = hashlib.sha256(b"".join(np.ascontiguousarray(g).tobytes() for g in gpu.ciph_to_host(res)))
+    assert got.hexdigest()[:16] == digest
+    for c in (ct, res):
+        gpu.free_ciph(c)
     gpu.close()
