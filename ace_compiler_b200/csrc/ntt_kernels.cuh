@@ -418,6 +418,16 @@ struct ArithInt {
   }
 };
 
+// a * b mod q on the pipe the prime allows, canonical
+struct Product {
+  const DevModulus& m;
+  ArithFp           fp;
+  __device__ __forceinline__ explicit Product(const DevModulus& md) : m(md), fp(md) {}
+  __device__ __forceinline__ u64 operator()(u64 a, u64 b) const {
+    return m.kind == kNttFloat ? fp.word(fp.mul(ArithFp::load(a), ArithFp::load(b))) : mul_mod(a, b, m);
+  }
+};
+
 // ---- register rounds --------------------------------------------------------------
 //
 // A thread holds the 2^E values of an E-bit field of the index; a round does the

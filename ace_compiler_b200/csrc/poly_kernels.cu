@@ -32,11 +32,11 @@ __device__ __forceinline__ u64* sel_d(const Ptr2& p, const LimbRef& lr, uint32_t
 // ---- element-wise (hal/src/hal.c:15-121, poly/src/rns_poly.c:852-1054) ------
 
 // What bounds these kernels is bytes in flight: every thread issues the loads of
-// two 16-byte words per operand before the first result.  With one 8-byte word at
+// four 16-byte words per operand before the first result.  With one 8-byte word at
 // a time and integer products throughout, the 9 products and 8 sums of a
-// convolution row at N = 65536 took 185 us, this way 140.  A limb has at least
-// four coefficients, so whole words always fit.
-constexpr int kWords = 2;  // 16-byte words per thread
+// convolution row at N = 65536 took 185 us, with two words 140, with four 131.  A
+// limb has at least four coefficients, so whole words always fit.
+constexpr int kWords = 4;  // 16-byte words per thread
 
 inline dim3 grid_words(uint32_t n, int limbs) {
   const uint32_t per_block = kThreads * kWords * 2;
@@ -56,17 +56,6 @@ struct WordLoop {  // the words of this thread
 #pragma unroll
     for (int k = 0; k < kWords; k++)
       v[k] = in[k] ? reinterpret_cast<const ulonglong2*>(p)[at[k]] : make_ulonglong2(0, 0);
-  }
-};
-
-// a * b mod q on the pipe the prime allows
-struct Product {
-  const DevModulus& m;
-  nttk::ArithFp     fp;
-  __device__ __forceinline__ explicit Product(const DevModulus& md) : m(md), fp(md) {}
-  __device__ __forceinline__ u64 operator()(u64 a, u64 b) const {
-    return m.kind == kNttFloat ? fp.word(fp.mul(nttk::ArithFp::load(a), nttk::ArithFp::load(b)))
-                               : mul_mod(a, b, m);
   }
 };
 
@@ -90,7 +79,7 @@ ew_kernel(Ptr2 res, Ptr2 a, Ptr2 b, u64 scalar, const __grid_constant__ LimbBatc
   words.load(x, sel_a(a, lr, n));
   if (two) words.load(y, sel_b(b, lr, n));
   if (accu) words.load(r, pr);
-  const Product mul(m);
+  const nttk::Product mul(m);
   auto one = [&](u64 x, u64 y, u64 r) {
     if (!two) y = sc;
     if (OP == EW_ADD || OP == EW_ADD_SCALAR) return add_mod(x, y, m.q);
@@ -123,7 +112,7 @@ ew_scalars_kernel(Ptr2 res, Ptr2 a, const __grid_constant__ ScalarList sc,
   const WordLoop   words(n);
   ulonglong2       x[kWords];
   words.load(x, sel_a(a, lr, n));
-  const Product mul(m);
+  const nttk::Product mul(m);
   auto one = [&](u64 v) { return MUL ? mul(v, s) : add_mod(v, s, m.q); };
 #pragma unroll
   for (int k = 0; k < kWords; k++)
