@@ -19,11 +19,13 @@
 // 128-bit reduction (about 130 at 12 inputs, bound by the integer multiplier:
 // 63 % of the launch).
 //
-// A CTA takes 256 coefficients (two row tiles) and all outputs of one group,
-// 16 outputs (128 columns) at a time: 256 columns of tensor memory, two CTAs
-// per SM, so that one CTA's products run under the other's reductions.
-// What bounds it now is the issue rate of those reductions and the traffic of
-// inputs and outputs with L2.
+// A CTA takes 256 coefficients (two row tiles) and all outputs of one group, 8
+// outputs (64 columns) at a time: 128 columns of tensor memory, four CTAs per SM,
+// so that one CTA's products run under the others' reductions.  What bounds it
+// is the issue rate of those reductions (59 instructions per output word, 57 % of
+// the issue slots; ModUp and ModDown of a rotation at 36 limbs of N = 65536 took
+// 164 us with multiply-adds, 46 here).  Four outputs per product with two products
+// in turn (29 us), and the outputs split over two to four CTAs (30 to 32), lost.
 #include <algorithm>
 #include <vector>
 
